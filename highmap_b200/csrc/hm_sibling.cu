@@ -27,6 +27,7 @@
 
 #include "hm_internal.h"
 #include "hm_thermal.h"
+#include "hm_thermal_block.cuh"
 #include "hm_thermal_math.cuh"
 #include "hm_thermal_sweep.cuh"
 
@@ -120,6 +121,13 @@ struct SiblingRule
     if (RULE == HM_SCREE) amp = __fmul_rn(amp, almost_unit_identity(clamp01(__fsub_rn(1.f, __fdiv_rn(c, zmax)))));
     return __fadd_rn(c, __fmul_rn(__fmul_rn(0.25f, __fsub_rn(t, __fmul_rn(0.5f, sum))), amp));
   }
+  __device__ static __forceinline__ F2 pair(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw, F2 sw, F2 ne, F2 se, F2 t, F2 x,
+                                            bool first, float p)
+  {
+    return pk(cell(lo(c), lo(w), lo(s), lo(n), lo(e), lo(nw), lo(sw), lo(ne), lo(se), lo(t), lo(x), first, p),
+              cell(hi(c), hi(w), hi(s), hi(n), hi(e), hi(nw), hi(sw), hi(ne), hi(se), hi(t), hi(x), first, p));
+  }
+  __device__ static __forceinline__ F2 talus_pair(F2 t) { return t; }
 };
 
 constexpr int SS_NT = 256, SS2_NT = 128, SS_H = 16; /* as the thermal sweeps */
@@ -146,6 +154,25 @@ __global__ void __launch_bounds__(SS2_NT)
   const int y0 = blockIdx.y * SS_H;
   thermal_sweep2_warp<RULE != HM_RIB, SiblingRule<RULE>>(a, b, nx, ny, talus, 0.f, zmax, 0, wx, y0,
                                                           min(ny, y0 + SS_H), intensity);
+}
+
+/* T steps of a 3 x 3 rule per launch (hm_thermal_block.cuh) */
+template <int RULE, int ROWS, bool VEC>
+__global__ void __launch_bounds__(TBK_NT)
+    k_sibling_block(const float *__restrict__ a, float *__restrict__ b, int nx, int ny, const float *__restrict__ talus,
+                    const float *__restrict__ zmax, float intensity, int T)
+{
+  thermal_block<RULE != HM_RIB, SiblingRule<RULE>, ROWS, VEC>(a, b, nx, ny, talus, 0.f, zmax, T, blockIdx.x,
+                                                              blockIdx.y, false, intensity);
+}
+
+template <int RULE>
+void launch_sibling_block(const float *a, float *b, int nx, int ny, const float *talus, const float *zmax,
+                          float intensity, int T, int rows, bool vec, cudaStream_t s)
+{
+  auto k = rows == 1 ? (vec ? k_sibling_block<RULE, 1, true> : k_sibling_block<RULE, 1, false>)
+                     : (vec ? k_sibling_block<RULE, 2, true> : k_sibling_block<RULE, 2, false>);
+  k<<<tbk_grid(nx, ny, BlockPlan{T, rows, 1}), TBK_NT, 0, s>>>(a, b, nx, ny, talus, zmax, intensity, T);
 }
 
 /* thermal_olsen and thermal_flatten: radius-2 reads, a shared-memory tile
@@ -359,22 +386,26 @@ int sibling_core(int device, int rule, float *z, int nx, int ny, const float *ta
                  float intensity, int iterations, float *depo, const float *mask, float *scratch_buf,
                  cudaStream_t s, float p1)
 {
-  const size_t n = (size_t)nx * ny;
-  float       *tmp = scratch_buf;
-  float       *z0 = scratch_buf + align_up(n, 64);
+  const size_t na = align_up((size_t)nx * ny, 64);
   const bool   want_depo = depo && rule <= HM_SCHOTT;
-  if (want_depo || mask) HM_CUDA_TRY(cudaMemcpyAsync(z0, z, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
+  const bool   keep_z = want_depo || mask; /* z holds the input heights to the end */
+  float       *buf[2] = {scratch_buf, keep_z ? scratch_buf + na : z}; /* the grids the launches write in turn */
   const dim3   grid((nx + SB_TX - 1) / SB_TX, (ny + SB_TY - 1) / SB_TY), block(SB_TX, SB_TY);
-  const float *src = z;
-  float       *dst = tmp;
   auto al8 = [](const void *p) { return ((uintptr_t)p & 7u) == 0; };
-  const bool pairs = nx % 2 == 0 && al8(z) && al8(tmp) && al8(talus) && (rule != HM_SCREE || al8(zmax));
+  const bool pairs = nx % 2 == 0 && al8(z) && al8(scratch_buf) && al8(talus) && (rule != HM_SCREE || al8(zmax));
   const dim3 g2((nx + 2 * SS2_NT - 1) / (2 * SS2_NT), (ny + SS_H - 1) / SS_H);
   const dim3 g1((nx + SS_NT - 1) / SS_NT, (ny + SS_H - 1) / SS_H);
-  for (int it = 0; it < iterations; it++)
+  /* several steps per launch for the 3 x 3 rules, as thermal chooses them */
+  const BlockPlan plan = rule == HM_OLSEN || rule == HM_FLATTEN ? BlockPlan{1, 0, iterations}
+                                                                : block_pick(nx, ny, iterations, !keep_z);
+  const float *src = z;
+  for (int l = 0; l < plan.launches; l++)
   {
+    float    *dst = buf[l & 1];
+    const int T = plan.T == 1 ? 1 : block_steps(plan, iterations, l);
 #define HM_SIB_SWEEP(R)                                                                                                \
-  if (pairs) k_sibling_sweep2<R><<<g2, SS2_NT, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity);                       \
+  if (plan.T > 1) launch_sibling_block<R>(src, dst, nx, ny, talus, zmax, intensity, T, plan.rows, pairs, s);            \
+  else if (pairs) k_sibling_sweep2<R><<<g2, SS2_NT, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity);                  \
   else k_sibling_sweep<R><<<g1, SS_NT, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity);
     switch (rule)
     {
@@ -388,13 +419,21 @@ int sibling_core(int device, int rule, float *z, int nx, int ny, const float *ta
     }
 #undef HM_SIB_SWEEP
     HM_LAUNCH_CHECK("k_sibling_step");
-    const float *t = src;
     src = dst;
-    dst = const_cast<float *>(t);
   }
-  if (src != z) HM_CUDA_TRY(cudaMemcpyAsync(z, src, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  return thermal_finish(device, z, nx, ny, z0, want_depo ? depo : nullptr, mask, s, rule != HM_SCREE,
-                        rule == HM_RIB ? 3 : 1);
+  float *dep = want_depo ? depo : nullptr;
+  if (rule != HM_RIB && nx >= 4 && ny >= 4 && (src != z || !keep_z))
+    return thermal_out(src, z, nx, ny, dep, mask, s, rule != HM_SCREE);
+  /* in place: a deeper border, a grid narrower than 4, or no steps */
+  const size_t bytes = (size_t)nx * ny * sizeof(float);
+  float       *z0 = nullptr;
+  if (keep_z)
+  {
+    z0 = src == buf[0] ? buf[1] : buf[0];
+    HM_CUDA_TRY(cudaMemcpyAsync(z0, z, bytes, cudaMemcpyDeviceToDevice, s));
+  }
+  if (src != z) HM_CUDA_TRY(cudaMemcpyAsync(z, src, bytes, cudaMemcpyDeviceToDevice, s));
+  return thermal_finish(device, z, nx, ny, z0, dep, mask, s, rule != HM_SCREE, rule == HM_RIB ? 3 : 1);
 }
 
 } // namespace hm

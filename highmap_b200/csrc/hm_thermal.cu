@@ -6,11 +6,14 @@
  * (HighMap/src/gpu_opencl/kernels/thermal.cl:26-100).
  *
  * Device data: z, talus and bedrock stay in HBM for the whole call; steps
- * ping-pong between z and one workspace grid (Jacobi).  After the steps:
- * extrapolate_borders (HighMap/src/boundary/boundary.cpp:19-41) on the
- * outer ring, then, when asked, the deposition map max(z - z0, 0)
+ * ping-pong between z and one workspace grid (Jacobi), or, where the input
+ * heights are needed to the end (deposition map, mask, auto-bedrock),
+ * between two workspace grids, so that no copy of them is made.  After the
+ * steps: extrapolate_borders (HighMap/src/boundary/boundary.cpp:19-41) on
+ * the outer ring, then, when asked, the deposition map max(z - z0, 0)
  * (HighMap/src/range/range.cpp:253-262) and the mask blend
- * lerp(z0, z, mask) (HighMap/include/highmap/operator.hpp:405-418).
+ * lerp(z0, z, mask) (HighMap/include/highmap/operator.hpp:405-418), all in
+ * one kernel that also brings the result to z.
  *
  * Kernels
  *   k_thermal_sweep2  one step per launch: a warp walks down rows of 64
@@ -18,12 +21,14 @@
  *                     reads z, talus and bedrock once, writes z: 12 B/cell
  *                     (16 B with bedrock).  Even nx, 8-byte aligned grids.
  *   k_thermal_sweep   the same with one column per lane (any grid).
- *   k_thermal_tb      up to 8 steps per launch (temporal blocking): a
- *                     strip of columns streams down the grid; each time
- *                     level keeps a 4-row ring in shared memory, so HBM
- *                     sees the 12/16 B of one step per T steps.
- *   k_extrapolate     the outer ring, one block.
- *   k_thermal_final   deposition map and mask blend, elementwise.
+ *   k_thermal_block   up to 8 steps per launch (temporal blocking,
+ *                     hm_thermal_block.cuh): the choice up to 1.5 M cells.
+ *   k_thermal_out     border, deposition map and mask blend from the last
+ *                     step's grid into z.
+ *   k_border          the border alone, in place.
+ *   k_extrapolate(_n), k_thermal_final   the same in place, border first
+ *                     (grids under 4 cells a side, deeper borders, the
+ *                     batched form).
  */
 #include <cuda_runtime.h>
 
@@ -32,14 +37,13 @@
 
 #include "hm_internal.h"
 #include "hm_thermal.h"
+#include "hm_thermal_block.cuh"
 #include "hm_thermal_math.cuh"
 #include "hm_thermal_sweep.cuh"
 #include "hm_tune.h"
 
 namespace hm
 {
-
-__device__ __forceinline__ int clamp_col(int g, int n) { return g < 0 ? 0 : (g > n - 1 ? n - 1 : g); }
 
 /* ------------------------------------------------------------------ */
 /* one step per launch, column sweep                                  */
@@ -92,109 +96,20 @@ __global__ void __launch_bounds__(S2_NT)
 /* several steps per launch (temporal blocking)                       */
 /* ------------------------------------------------------------------ */
 
-constexpr int TB_TPB = 256; /* strip width in columns, one thread each      */
-constexpr int TB_TMAX = 8;  /* most steps one launch advances                */
-
-__device__ __forceinline__ void tb_cp_async4(float *smem, const float *gmem)
+template <bool TMAP, int BED, int ROWS, bool VEC>
+__global__ void __launch_bounds__(TBK_NT)
+    k_thermal_block(const float *__restrict__ a,
+                    float *__restrict__ b,
+                    int nx,
+                    int ny,
+                    const float *__restrict__ talus,
+                    float talus_value,
+                    const float *__restrict__ bedrock,
+                    int T,
+                    int first)
 {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
-/* T Jacobi steps of a column strip in one pass down the rows.
- *
- * Thread t owns global column gi = x0 - T + t of a strip of TPB columns
- * (W = TPB - 2T output columns), and the CTA owns output rows [y0, y1).
- * Level 0 is the input z, staged row by row into an 8-row ring with
- * cp.async; level k (1 <= k < T) keeps a 4-row ring.  Iteration r loads
- * row r and computes, for every level k, row r - 1 - 2k from rows
- * r - 2 - 2k .. r - 2k of level k - 1, all finished in earlier iterations;
- * one __syncthreads per iteration publishes them.  Level T goes straight
- * to the output grid.  Level k is needed on rows [y0 - (T-k), y1 + T-k)
- * and is correct on columns [k, TPB - k) of the strip, so the T halo
- * columns each side cover the shrinking valid region.
- *
- * Each cell follows the rule of the one-step kernel (border copy, then
- * the talus exchange with bedrock), so T steps here are bit-identical to
- * T one-step launches. */
-template <bool TMAP, int BED>
-__global__ void __launch_bounds__(TB_TPB)
-    k_thermal_tb(const float *__restrict__ a,
-                 float *__restrict__ b,
-                 int nx,
-                 int ny,
-                 const float *__restrict__ talus,
-                 float talus_value,
-                 const float *__restrict__ bedrock,
-                 int T,
-                 int H,
-                 int it0)
-{
-  __shared__ float lv0[8][TB_TPB];
-  __shared__ float lvk[TB_TMAX - 1][4][TB_TPB];
-
-  const int  tid = threadIdx.x;
-  const int  W = TB_TPB - 2 * T;
-  const int  x0 = blockIdx.x * W;
-  const int  gi = x0 - T + tid;
-  const bool in_grid = gi >= 0 && gi < nx;
-  const int  gic = clamp_col(gi, nx);
-  const int  y0 = blockIdx.y * H;
-  const int  y1 = min(ny, y0 + H);
-  const int  lw = max(tid - 1, 0), le = min(tid + 1, TB_TPB - 1);
-  const bool out_col = tid >= T && tid < T + W && gi < nx;
-  const int  load_lo = max(0, y0 - T), load_hi = min(ny - 1, y1 - 1 + T);
-
-  for (int r = y0 - T; r <= y1 + 2 * T; ++r)
-  {
-    if (r >= load_lo && r <= load_hi && in_grid) tb_cp_async4(&lv0[r & 7][tid], a + (size_t)r * nx + gi);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-
-#pragma unroll
-    for (int k = 1; k <= TB_TMAX; k++)
-    {
-      if (k > T) break;
-      const int j = r - 1 - 2 * k;
-      if (j < max(0, y0 - (T - k)) || j > min(ny - 1, y1 - 1 + (T - k))) continue;
-      /* rows j-1, j, j+1 of level k-1 */
-      const float *pn, *pc, *ps;
-      if (k == 1)
-      {
-        pn = lv0[(j - 1) & 7];
-        pc = lv0[j & 7];
-        ps = lv0[(j + 1) & 7];
-      }
-      else
-      {
-        pn = lvk[k - 2][(j - 1) & 3];
-        pc = lvk[k - 2][j & 3];
-        ps = lvk[k - 2][(j + 1) & 3];
-      }
-      float out;
-      /* apply_boundaries, _common_index.cl:106-132 */
-      if (gi == 0) out = pc[le];
-      else if (gi == nx - 1) out = pc[lw];
-      else if (j == 0) out = ps[tid];
-      else if (j == ny - 1) out = pn[tid];
-      else
-      {
-        const size_t q = (size_t)j * nx + gic;
-        const float  t = TMAP ? __ldg(talus + q) : talus_value;
-        const float  zb = BED != BED_NONE ? __ldg(bedrock + q) : 0.f;
-        out = thermal_cell<BED>(pc[tid], pc[lw], ps[tid], pn[tid], pc[le], pn[lw], ps[lw], pn[le], ps[le], t, zb,
-                                it0 + k == 1);
-      }
-      if (k == T)
-      {
-        if (out_col && j >= y0 && j < y1) b[(size_t)j * nx + gi] = out;
-      }
-      else
-        lvk[k - 1][j & 3][tid] = out;
-    }
-    __syncthreads();
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  thermal_block<TMAP, TalusExchange<BED>, ROWS, VEC>(a, b, nx, ny, talus, talus_value, bedrock, T, blockIdx.x,
+                                                     blockIdx.y, first != 0);
 }
 
 /* ------------------------------------------------------------------ */
@@ -268,6 +183,83 @@ __global__ void k_thermal_final(float *__restrict__ z,
       float m = mask[k];
       z[k] = __fadd_rn(__fmul_rn(o, __fsub_rn(1.f, m)), __fmul_rn(r, m));
     }
+  }
+}
+
+/* Cell (i, j) of extrapolate_borders(s, 1, 0) for grids of at least 4 x 4,
+ * where every border cell is a function of interior cells alone: columns
+ * from the two inward ones of their row, then rows from the two inward
+ * rows (whose end cells are the column pass's). */
+__device__ __forceinline__ float bordered_row(const float *__restrict__ r, int i, int nx)
+{
+  if (i == 0) return __fsub_rn(__fmul_rn(2.f, r[1]), r[2]);
+  if (i == nx - 1) return __fsub_rn(__fmul_rn(2.f, r[nx - 2]), r[nx - 3]);
+  return r[i];
+}
+__device__ __forceinline__ float bordered(const float *__restrict__ s, int i, int j, int nx, int ny)
+{
+  if (j == 0 || j == ny - 1)
+  {
+    const float *r1 = s + (size_t)(j == 0 ? 1 : ny - 2) * nx, *r2 = s + (size_t)(j == 0 ? 2 : ny - 3) * nx;
+    return __fsub_rn(__fmul_rn(2.f, bordered_row(r1, i, nx)), bordered_row(r2, i, nx));
+  }
+  return bordered_row(s + (size_t)j * nx, i, nx);
+}
+
+/* the outer ring in place: one thread per border cell; only interior cells
+ * are read and only border cells written */
+__global__ void __launch_bounds__(256) k_border(float *z, int nx, int ny)
+{
+  const long long n = 2ll * nx + 2ll * (ny - 2);
+  for (long long k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
+  {
+    int i, j;
+    if (k < 2ll * nx)
+    {
+      j = k < nx ? 0 : ny - 1;
+      i = (int)(k < nx ? k : k - nx);
+    }
+    else
+    {
+      const long long m = k - 2ll * nx;
+      j = 1 + (int)(m >> 1);
+      i = (m & 1) ? nx - 1 : 0;
+    }
+    z[(size_t)j * nx + i] = bordered(z, i, j, nx, ny);
+  }
+}
+
+/* The result of a solve from its last grid s (not z): border, deposition
+ * map against the input heights z still holds, mask blend; 256 cells of a
+ * row per CTA and turn. */
+__global__ void __launch_bounds__(256)
+    k_thermal_out(const float *__restrict__ s, float *__restrict__ z, float *__restrict__ depo,
+                  const float *__restrict__ mask, int nx, int ny, int depo_abs)
+{
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= nx) return;
+  for (int j = blockIdx.y; j < ny; j += gridDim.y)
+  {
+    const size_t k = (size_t)j * nx + i;
+    const float  r = bordered(s, i, j, nx, ny);
+    if (!depo && !mask)
+    {
+      z[k] = r;
+      continue;
+    }
+    const float o = z[k];
+    if (depo)
+    {
+      const float dz = __fsub_rn(r, o);
+      depo[k] = depo_abs ? fabsf(dz) : (dz > 0.f ? dz : 0.f);
+    }
+    if (mask)
+    {
+      const float m = mask[k];
+      z[k] = __fadd_rn(__fmul_rn(o, __fsub_rn(1.f, m)), __fmul_rn(r, m));
+    }
+    else
+      z[k] = r;
   }
 }
 
@@ -355,40 +347,55 @@ int thermal_finish(int device, float *z, int nx, int ny, const float *z0, float 
   return HM_OK;
 }
 
-template <bool TMAP, int BED>
-static void launch_tb(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
-                      int T, int H, int it0, cudaStream_t s)
+int thermal_out(const float *src, float *z, int nx, int ny, float *depo, const float *mask, cudaStream_t s,
+                bool depo_abs)
 {
-  const int W = TB_TPB - 2 * T;
-  dim3      grid((nx + W - 1) / W, (ny + H - 1) / H);
-  k_thermal_tb<TMAP, BED><<<grid, TB_TPB, 0, s>>>(a, b, nx, ny, talus, tv, bed, T, H, it0);
+  if (src == z && !depo && !mask && nx >= 4 && ny >= 4)
+  {
+    const long long n = 2ll * nx + 2ll * (ny - 2);
+    k_border<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(z, nx, ny);
+    HM_LAUNCH_CHECK("k_border");
+    return HM_OK;
+  }
+  const int gx = (nx + 255) / 256;
+  k_thermal_out<<<dim3(gx, ny < 32768 ? ny : 32768), 256, 0, s>>>(src, z, depo, mask, nx, ny, depo_abs ? 1 : 0);
+  HM_LAUNCH_CHECK("k_thermal_out");
+  return HM_OK;
+}
+
+template <bool TMAP, int BED>
+static void launch_block(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
+                         int T, int rows, int first, cudaStream_t s)
+{
+  auto       al8 = [](const void *p) { return ((uintptr_t)p & 7u) == 0; };
+  const bool vec = nx % 2 == 0 && al8(a) && al8(b) && (!TMAP || al8(talus)) && (BED == BED_NONE || al8(bed));
+  const dim3 g = tbk_grid(nx, ny, BlockPlan{T, rows, 1});
+  auto       k = rows == 1 ? (vec ? k_thermal_block<TMAP, BED, 1, true> : k_thermal_block<TMAP, BED, 1, false>)
+                           : (vec ? k_thermal_block<TMAP, BED, 2, true> : k_thermal_block<TMAP, BED, 2, false>);
+  k<<<g, TBK_NT, 0, s>>>(a, b, nx, ny, talus, tv, bed, T, first);
 }
 
 template <bool TMAP>
-static void tb_dispatch_t(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
-                          int mode, int T, int H, int it0, cudaStream_t s)
+static void block_dispatch_t(const float *a, float *b, int nx, int ny, const float *talus, float tv,
+                             const float *bed, int mode, int T, int rows, int first, cudaStream_t s)
 {
   switch (mode)
   {
-  case BED_NONE: launch_tb<TMAP, BED_NONE>(a, b, nx, ny, talus, tv, bed, T, H, it0, s); break;
-  case BED_INTENDED: launch_tb<TMAP, BED_INTENDED>(a, b, nx, ny, talus, tv, bed, T, H, it0, s); break;
-  case BED_LITERAL: launch_tb<TMAP, BED_LITERAL>(a, b, nx, ny, talus, tv, bed, T, H, it0, s); break;
-  default: launch_tb<TMAP, BED_AUTO>(a, b, nx, ny, talus, tv, bed, T, H, it0, s); break;
+  case BED_NONE: launch_block<TMAP, BED_NONE>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
+  case BED_INTENDED: launch_block<TMAP, BED_INTENDED>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
+  case BED_LITERAL: launch_block<TMAP, BED_LITERAL>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
+  default: launch_block<TMAP, BED_AUTO>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
   }
 }
 
-static void tb_dispatch(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
-                        int mode, int T, int H, int it0, cudaStream_t s)
+static void block_dispatch(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
+                           int mode, int T, int rows, int first, cudaStream_t s)
 {
-  if (talus) tb_dispatch_t<true>(a, b, nx, ny, talus, tv, bed, mode, T, H, it0, s);
-  else tb_dispatch_t<false>(a, b, nx, ny, talus, tv, bed, mode, T, H, it0, s);
+  if (talus) block_dispatch_t<true>(a, b, nx, ny, talus, tv, bed, mode, T, rows, first, s);
+  else block_dispatch_t<false>(a, b, nx, ny, talus, tv, bed, mode, T, rows, first, s);
 }
 
-static int g_tb_rows = 0; /* output rows per CTA of the blocked kernel; 0 = built-in */
-
-/* steps per launch when the caller leaves the choice to the library and
- * the grid's size class is not tuned */
-static int g_tb_default = 1;
+static int g_tb_rows = 0; /* tile rows of the blocked kernel (hm_thermal_set_launch); 0 = built-in */
 
 int thermal_check_args(const float *z, int nx, int ny, int iterations, const hm_thermal_options *o)
 {
@@ -427,59 +434,61 @@ int thermal_core(int device,
   hm_thermal_options o;
   hm_thermal_default_options(&o);
   if (opts) o = *opts;
-  const size_t n = (size_t)nx * ny;
-  const bool   need_z0 = depo || mask || auto_bed;
-  float       *tmp = scratch_buf;
-  float       *z0 = need_z0 ? scratch_buf + align_up(n, 64) : nullptr;
+  const bool   keep_z = depo || mask || auto_bed; /* z holds the input heights to the end */
+  const size_t na = align_up((size_t)nx * ny, 64);
+  /* the grids the launches write in turn */
+  float       *buf[2] = {scratch_buf, keep_z ? scratch_buf + na : z};
   (void)device;
 
-  if (need_z0) HM_CUDA_TRY(cudaMemcpyAsync(z0, z, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-
-  /* steps per launch: 1 runs the one-step kernel, 2..8 the blocked kernel.
-   * 0 takes the tuned choice for this grid (thermal_pick_block), else one
-   * step per launch, the faster of the two on B200 at 4096^2 when untuned
-   * (both are bound by the issue rate of the exact arithmetic, not by
-   * HBM). */
-  int tb = o.time_block;
-  int rows = g_tb_rows;
-  if (tb == 0)
+  /* steps per launch: 1 runs the one-step kernel, 2..8 the blocked kernel;
+   * 0 takes the tuned choice for this grid, else block_pick's.  Without
+   * the input heights to keep, an even number of launches ends in z. */
+  BlockPlan plan;
+  int       tb = o.time_block, rows = g_tb_rows;
+  TuneEntry e;
+  if (tb == 0 && tuned_thermal(nx, ny, &e))
   {
-    TuneEntry e;
-    if (tuned_thermal(nx, ny, &e))
-    {
-      tb = e.block;
-      if (rows == 0) rows = e.rows;
-    }
-    else
-      tb = g_tb_default;
+    tb = e.block;
+    if (rows == 0) rows = e.rows;
   }
-  if (tb > TB_TMAX) tb = TB_TMAX;
-  if (rows <= 0) rows = 128;
+  if (tb == 0) plan = block_pick(nx, ny, iterations, !keep_z);
+  else if (tb == 1 || iterations < 2) plan = BlockPlan{1, 0, iterations};
+  else plan = block_fixed(tb > TBK_TMAX ? TBK_TMAX : tb, rows, iterations, !keep_z);
   /* auto-bedrock reads the input heights as its bedrock */
   const int    mode = kernel_bed_mode(bedrock, o.bedrock_mode, auto_bed);
-  const float *bed = auto_bed ? z0 : bedrock;
+  const float *bed = auto_bed ? z : bedrock;
   const float *src = z;
-  float       *dst = tmp;
-  for (int done = 0; done < iterations;)
+  for (int l = 0; l < plan.launches; l++)
   {
-    const int T = (iterations - done < tb) ? iterations - done : tb;
-    if (tb == 1)
+    float *dst = buf[l & 1];
+    if (plan.T == 1)
     {
-      step_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, done == 0, s);
+      step_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, l == 0, s);
       HM_LAUNCH_CHECK("k_thermal_sweep");
     }
     else
     {
-      tb_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, T, rows, done, s);
-      HM_LAUNCH_CHECK("k_thermal_tb");
+      block_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, block_steps(plan, iterations, l), plan.rows,
+                     l == 0, s);
+      HM_LAUNCH_CHECK("k_thermal_block");
     }
-    done += T;
-    const float *t = src;
     src = dst;
-    dst = const_cast<float *>(t);
   }
-  if (src != z) HM_CUDA_TRY(cudaMemcpyAsync(z, src, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  return thermal_finish(device, z, nx, ny, z0, depo, mask, s);
+  /* in place, or on a grid too narrow for k_thermal_out: border first,
+   * then the rest against a copy of the input heights */
+  if (nx < 4 || ny < 4 || (src == z && (depo || mask)))
+  {
+    const size_t bytes = (size_t)nx * ny * sizeof(float);
+    float       *z0 = nullptr;
+    if (depo || mask)
+    {
+      z0 = src == buf[0] ? buf[1] : buf[0];
+      HM_CUDA_TRY(cudaMemcpyAsync(z0, z, bytes, cudaMemcpyDeviceToDevice, s));
+    }
+    if (src != z) HM_CUDA_TRY(cudaMemcpyAsync(z, src, bytes, cudaMemcpyDeviceToDevice, s));
+    return thermal_finish(device, z, nx, ny, z0, depo, mask, s);
+  }
+  return thermal_out(src, z, nx, ny, depo, mask, s, false);
 }
 
 } // namespace hm

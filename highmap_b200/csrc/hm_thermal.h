@@ -9,16 +9,22 @@
 namespace hm
 {
 int    thermal_check_args(const float *z, int nx, int ny, int iterations, const hm_thermal_options *o);
-/* floats of workspace thermal_core needs (one grid, two with a z0 copy) */
+/* floats of workspace thermal_core needs: one grid, two where z has to hold
+ * the input heights to the end (deposition map, mask, auto-bedrock) */
 size_t thermal_scratch_floats(int nx, int ny, bool need_z0);
 /* Device pointers; ordered on s.  talus NULL selects talus_value.
- * auto_bed: thermal_auto_bedrock (bedrock must be NULL; needs the z0 copy). */
+ * auto_bed: thermal_auto_bedrock (bedrock must be NULL; two grids). */
 int    thermal_core(int device, float *z, int nx, int ny, const float *talus, float talus_value, int iterations,
                     const float *bedrock, float *depo, const float *mask, const hm_thermal_options *opts,
                     float *scratch_buf, cudaStream_t s, bool auto_bed = false);
 /* border extrapolation, deposition map and mask blend after the steps */
 int    thermal_finish(int device, float *z, int nx, int ny, const float *z0, float *depo, const float *mask,
                       cudaStream_t s, bool depo_abs = false, int nbuffer = 1);
+/* the same out of the last step's grid src into z, which holds the input
+ * heights (src == z: the border alone, in place); grids of at least 4 x 4,
+ * one border cell deep */
+int    thermal_out(const float *src, float *z, int nx, int ny, float *depo, const float *mask, cudaStream_t s,
+                   bool depo_abs);
 /* sediment_deposition (hm_deposition.cu): device pointers, ordered on s */
 size_t deposition_scratch_floats(int nx, int ny);
 int    deposition_core(int device, float *z, int nx, int ny, const float *talus, float max_deposition,

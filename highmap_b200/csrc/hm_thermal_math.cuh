@@ -29,6 +29,8 @@
 
 #include <cfloat>
 
+#include "hm_pack.cuh"
+
 namespace hm
 {
 
@@ -134,6 +136,90 @@ __device__ __forceinline__ float thermal_cell(float c,
     out = __fadd_rn(c, thermal_amount(c, w, s, n, e, nw, sw, ne, se, talus));
   if (BED == BED_INTENDED) out = out > bedrock ? out : bedrock;
   return out;
+}
+
+/* The same for two adjacent cells at once, in packed arithmetic
+ * (hm_pack.cuh): 42 instead of 62 issue slots per cell, the same bits.
+ * Each exchange is the scalar one, operation by operation: the
+ * subtractions, the products and the sums are packed; the max and the sign
+ * go per half (packed instructions take no absolute value).
+ * No product feeds a packed add directly (a copysign or the last fma of
+ * the division lies between), so nothing is contracted. */
+__device__ __forceinline__ F2 copysign2(F2 mag, F2 sgn)
+{
+  /* mag is not negative */
+  F2 r;
+  asm("{\n.reg .b32 a, b, c, d;\nmov.b64 {a, b}, %1;\nmov.b64 {c, d}, %2;\n"
+      "lop3.b32 a, a, c, 0x80000000, 0xf8;\nlop3.b32 b, b, d, 0x80000000, 0xf8;\nmov.b64 %0, {a, b};\n}"
+      : "=l"(r.v)
+      : "l"(mag.v), "l"(sgn.v));
+  return r;
+}
+
+/* 0.2 * max(|n| - t, 0) for both halves as 0.2 * (max(|n|, t) - t), which
+ * leaves only the max per half: the same value for every n (NaN gives 0 in
+ * both) and every t that talus2 lets through */
+__device__ __forceinline__ F2 exch2(F2 n, F2 t)
+{
+  const float2 a = up(n), b = up(t);
+  return mul2(sub2(pk(fmaxf(fabsf(a.x), b.x), fmaxf(fabsf(a.y), b.y)), t), pk1(0.2f));
+}
+
+/* A talus pair for the packed exchanges: NaN and +inf, which stop every
+ * exchange, become the largest talus whose product with 1.414 is finite */
+__device__ __forceinline__ F2 talus2(F2 t)
+{
+  const float2 v = up(t);
+  return pk(fminf(v.x, 2.4e38f), fminf(v.y, 2.4e38f));
+}
+
+__device__ __forceinline__ F2 exch_axial2(F2 self, F2 other, F2 t)
+{
+  const F2 n = sub2(other, self);
+  return copysign2(exch2(n, t), n);
+}
+
+__device__ __forceinline__ F2 exch_diag2(F2 self, F2 other, F2 md)
+{
+  const F2 n = sub2(other, self);
+  const F2 x = exch2(n, md);
+  const F2 y = pk1(0x1.6a17e6p-1f); /* div_by_diag */
+  const F2 q = mul2(x, y);
+  const F2 r = fma2(q, pk1(-1.414f), x);
+  return copysign2(fma2(r, y, q), n);
+}
+
+__device__ __forceinline__ F2 thermal_amount2(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw, F2 sw, F2 ne, F2 se, F2 t)
+{
+  const F2 md = mul2(pk1(1.414f), t);
+  F2       a = exch_axial2(c, w, t);
+  a = add2(a, exch_axial2(c, s, t));
+  a = add2(a, exch_axial2(c, n, t));
+  a = add2(a, exch_axial2(c, e, t));
+  a = add2(a, exch_diag2(c, nw, md));
+  a = add2(a, exch_diag2(c, sw, md));
+  a = add2(a, exch_diag2(c, ne, md));
+  a = add2(a, exch_diag2(c, se, md));
+  return a;
+}
+
+/* thermal_cell for two adjacent cells */
+template <int BED>
+__device__ __forceinline__ F2 thermal_cell2(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw, F2 sw, F2 ne, F2 se, F2 t, F2 bed,
+                                            bool first)
+{
+  const float2 v = up(c), b = up(bed);
+  if (BED == BED_LITERAL) return pk(v.x > b.x ? v.x : b.x, v.y > b.y ? v.y : b.y);
+  const F2     x2 = add2(c, thermal_amount2(c, w, s, n, e, nw, sw, ne, se, t));
+  if (BED == BED_NONE) return x2;
+  const float2 x = up(x2);
+  /* val < bedrock leaves the bedrock, so both tests of thermal_cell end in
+   * one select */
+  if (BED == BED_INTENDED)
+    return pk(v.x >= b.x && x.x > b.x ? x.x : b.x, v.y >= b.y && x.y > b.y ? x.y : b.y);
+  const float zx = x.x > b.x ? x.x : b.x, zy = x.y > b.y ? x.y : b.y;
+  const float fx = first ? -FLT_MAX : v.x, fy = first ? -FLT_MAX : v.y;
+  return pk(b.x >= -FLT_MAX ? (zx > fx ? zx : fx) : v.x, b.y >= -FLT_MAX ? (zy > fy ? zy : fy) : v.y);
 }
 
 } // namespace hm

@@ -29,7 +29,8 @@ constexpr int SW_P = 8; /* rows whose loads are issued together */
  * extra, first, param) is the new value of an interior cell from its 3 x 3
  * neighbourhood (named by position: w = (i-1, j), s = (i, j+1), n =
  * (i, j-1), ...), its talus, the value of the optional per-cell grid
- * `extra` (R::EXTRA), the first-step flag and a scalar parameter. */
+ * `extra` (R::EXTRA), the first-step flag and a scalar parameter;
+ * R::pair is the same for two adjacent cells at once (hm_pack.cuh). */
 template <int BED>
 struct TalusExchange
 {
@@ -39,6 +40,13 @@ struct TalusExchange
   {
     return thermal_cell<BED>(c, w, s, n, e, nw, sw, ne, se, t, x, first);
   }
+  __device__ static __forceinline__ F2 pair(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw, F2 sw, F2 ne, F2 se, F2 t, F2 x,
+                                            bool first, float)
+  {
+    return thermal_cell2<BED>(c, w, s, n, e, nw, sw, ne, se, t, x, first);
+  }
+  /* the talus of a pair as R::pair takes it */
+  __device__ static __forceinline__ F2 talus_pair(F2 t) { return talus2(t); }
 };
 
 /* Columns wx .. wx+31 (lane = column; columns past nx only feed the
@@ -127,11 +135,36 @@ __device__ __forceinline__ void thermal_sweep_warp(const float *__restrict__ a,
 
 
 /* The same sweep with two adjacent columns per lane (a warp owns the 64
- * columns wx .. wx+63): z, talus and bedrock move as 8-byte pairs, and one
- * pair of shuffles per row serves both cells, which halves the per-cell
- * load, shuffle and address work.  Needs an even nx and 8-byte aligned
+ * columns wx .. wx+63): z, talus and bedrock move as 8-byte pairs, one
+ * pair of shuffles per row serves both cells, and the cell rule runs on
+ * both in packed arithmetic (R::pair).  Needs an even nx and 8-byte aligned
  * grids; identical bits to thermal_sweep_warp. */
 constexpr int S2_P = 4; /* rows whose loads are issued together */
+
+__device__ __forceinline__ F2 ldg2(const float *p)
+{
+  F2 r;
+  r.v = __ldg(reinterpret_cast<const unsigned long long *>(p));
+  return r;
+}
+__device__ __forceinline__ void st2(float *p, F2 v) { *reinterpret_cast<unsigned long long *>(p) = v.v; }
+
+/* One row of a lane's column pair: the pair (x, y), the pair one column to
+ * the west (w, x) and the pair one column to the east (y, e). */
+struct PairRow
+{
+  F2 c, w, e;
+};
+
+/* the shifted pairs of a row from the neighbouring lanes' pairs; halo is
+ * the column just outside the warp on lanes 0 and 31 */
+__device__ __forceinline__ void pair_exchange(PairRow &r, int lane, float halo)
+{
+  const float2 c = up(r.c);
+  const float  wv = __shfl_up_sync(0xffffffffu, c.y, 1), ev = __shfl_down_sync(0xffffffffu, c.x, 1);
+  r.w = pk(lane == 0 ? halo : wv, c.x);
+  r.e = pk(c.y, lane == 31 ? halo : ev);
+}
 
 template <bool TMAP, class R, int P = S2_P>
 __device__ __forceinline__ void thermal_sweep2_warp(const float *__restrict__ a,
@@ -154,53 +187,41 @@ __device__ __forceinline__ void thermal_sweep2_warp(const float *__restrict__ a,
   /* lanes 0 and 31 also load the column west / east of the warp */
   const int  hx = lane == 0 ? max(wx - 1, 0) : (lane == 31 ? min(wx + 64, nx - 1) : gxc);
 
-  /* per row: the pair (x, y), the west neighbour of x and the east one of y */
-  float vx[P + 2], vy[P + 2], vw[P + 2], ve[P + 2];
+  PairRow    v[P + 2];
+  float      halo[P + 2];
   const bool halo_lane = lane == 0 || lane == 31;
   auto load = [&](int r, int q) {
     const float *row = a + (size_t)r * nx;
-    const float2 t = __ldg(reinterpret_cast<const float2 *>(row + gxc));
-    vx[q] = t.x;
-    vy[q] = t.y;
-    /* the halo value until the shuffles; only the edge lanes keep theirs */
-    vw[q] = halo_lane ? __ldg(row + hx) : 0.f;
-  };
-  auto exchange = [&](int q) {
-    const float up = __shfl_up_sync(0xffffffffu, vy[q], 1), dn = __shfl_down_sync(0xffffffffu, vx[q], 1);
-    ve[q] = lane == 31 ? vw[q] : dn;
-    vw[q] = lane == 0 ? vw[q] : up;
+    v[q].c = ldg2(row + gxc);
+    halo[q] = halo_lane ? __ldg(row + hx) : 0.f;
   };
   load(max(y0 - 1, 0), 0);
   load(y0, 1);
-  exchange(0);
-  exchange(1);
+  pair_exchange(v[0], lane, halo[0]);
+  pair_exchange(v[1], lane, halo[1]);
   for (int j0 = y0; j0 < y1; j0 += P)
   {
-    float2 tl[P], bd[P];
+    F2 tl[P], bd[P];
 #pragma unroll
     for (int q = 0; q < P; q++)
     {
       load(min(j0 + 1 + q, ny - 1), q + 2);
       const size_t o = (size_t)min(j0 + q, ny - 1) * nx + gxc;
-      tl[q] = TMAP ? __ldg(reinterpret_cast<const float2 *>(talus + o)) : make_float2(talus_value, talus_value);
-      bd[q] = R::EXTRA ? __ldg(reinterpret_cast<const float2 *>(bedrock + o)) : make_float2(0.f, 0.f);
+      tl[q] = R::talus_pair(TMAP ? ldg2(talus + o) : pk1(talus_value));
+      bd[q] = R::EXTRA ? ldg2(bedrock + o) : pk1(0.f);
     }
 #pragma unroll
-    for (int q = 2; q < P + 2; q++) exchange(q);
+    for (int q = 2; q < P + 2; q++) pair_exchange(v[q], lane, halo[q]);
+    auto cell2 = [&](int q) {
+      return R::pair(v[q + 1].c, v[q + 1].w, v[q + 2].c, v[q].c, v[q + 1].e, v[q].w, v[q + 2].w, v[q].e, v[q + 2].e,
+                     tl[q], bd[q], first != 0, param);
+    };
     /* a warp whose columns and rows are all interior: no border tests
      * (10 % of the step at 4096^2) */
     if (wx > 0 && wx + 64 < nx && j0 > 0 && j0 + P < ny - 1 && j0 + P <= y1)
     {
 #pragma unroll
-      for (int q = 0; q < P; q++)
-      {
-        float2 out;
-        out.x = R::cell(vx[q + 1], vw[q + 1], vx[q + 2], vx[q], vy[q + 1], vw[q], vw[q + 2], vy[q], vy[q + 2],
-                        tl[q].x, bd[q].x, first != 0, param);
-        out.y = R::cell(vy[q + 1], vx[q + 1], vy[q + 2], vy[q], ve[q + 1], vx[q], vx[q + 2], ve[q], ve[q + 2],
-                        tl[q].y, bd[q].y, first != 0, param);
-        *reinterpret_cast<float2 *>(b + (size_t)(j0 + q) * nx + gx) = out;
-      }
+      for (int q = 0; q < P; q++) st2(b + (size_t)(j0 + q) * nx + gx, cell2(q));
     }
     else
     {
@@ -209,31 +230,17 @@ __device__ __forceinline__ void thermal_sweep2_warp(const float *__restrict__ a,
       {
         const int j = j0 + q;
         if (!live || j >= y1) continue;
-        float2 out;
-        /* apply_boundaries, _common_index.cl:106-132, for each of the two cells */
-        if (gx == 0) out.x = vy[q + 1];
-        else if (j == 0) out.x = vx[q + 2];
-        else if (j == ny - 1) out.x = vx[q];
-        else
-          out.x = R::cell(vx[q + 1], vw[q + 1], vx[q + 2], vx[q], vy[q + 1], vw[q], vw[q + 2], vy[q], vy[q + 2],
-                          tl[q].x, bd[q].x, first != 0, param);
-        if (gx + 1 == nx - 1) out.y = vx[q + 1];
-        else if (j == 0) out.y = vy[q + 2];
-        else if (j == ny - 1) out.y = vy[q];
-        else
-          out.y = R::cell(vy[q + 1], vx[q + 1], vy[q + 2], vy[q], ve[q + 1], vx[q], vx[q + 2], ve[q], ve[q + 2],
-                          tl[q].y, bd[q].y, first != 0, param);
-        *reinterpret_cast<float2 *>(b + (size_t)j * nx + gx) = out;
+        /* apply_boundaries, _common_index.cl:106-132: rows 0 and ny - 1
+         * copy their inward row, then columns 0 and nx - 1 their inward
+         * column */
+        F2 out = j == 0 ? v[q + 2].c : (j == ny - 1 ? v[q].c : cell2(q));
+        if (gx == 0) out = pk(hi(v[q + 1].c), hi(out));
+        if (gx + 1 == nx - 1) out = pk(lo(out), lo(v[q + 1].c));
+        st2(b + (size_t)j * nx + gx, out);
       }
     }
-    vx[0] = vx[P];
-    vy[0] = vy[P];
-    vw[0] = vw[P];
-    ve[0] = ve[P];
-    vx[1] = vx[P + 1];
-    vy[1] = vy[P + 1];
-    vw[1] = vw[P + 1];
-    ve[1] = ve[P + 1];
+    v[0] = v[P];
+    v[1] = v[P + 1];
   }
 }
 

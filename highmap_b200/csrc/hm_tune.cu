@@ -9,8 +9,8 @@
  *             (temporal-block depth 1, 2), and the streaming kernel's
  *             threads per CTA (strip width) x staged advection radius x
  *             output rows per CTA (the occupancy / halo / warm-up trade);
- *   thermal : steps per launch (temporal-block depth 1, 2, 4, 8) x rows
- *             per CTA of the blocked kernel;
+ *   thermal : steps per launch (temporal-block depth 1, 2, 4, 8) x tile
+ *             rows of the blocked kernel;
  *   batch   : persistent CTAs per SM (occupancy; 0 = one CTA per tile of
  *             the round) x rows of a thermal tile
  *             of the batched form's round kernel, on a synthetic mixed
@@ -254,7 +254,8 @@ int hm_autotune(hm_context *ctx, int kind, int nx, int ny, int steps, hm_tune_re
   }
   else
   {
-    const int shapes[][2] = {{1, 0}, {2, 64}, {4, 64}, {4, 128}, {8, 64}, {8, 128}};
+    /* steps per launch, tile rows of the blocked kernel */
+    const int shapes[][2] = {{1, 0}, {2, 32}, {4, 16}, {4, 32}, {8, 32}};
     for (auto &c : shapes) cands.push_back(hm::TuneEntry{0, 0, c[1], c[0], 0.f});
   }
 

@@ -643,9 +643,10 @@ int hm_vpipes_set_algorithm(int algo);
  * of 16 and at most 4096; 0 (the default) turns it off. */
 int hm_debug_tma_expect_extra(unsigned bytes);
 
-/* Output rows per CTA of the temporally blocked thermal kernel,
- * process-wide (8..4096; 0 restores the built-in choice).  Results do not
- * depend on it. */
+/* Tile rows per CTA of the temporally blocked thermal kernel when the steps
+ * per launch are given or tuned, process-wide (8..4096; up to 16 asks for
+ * tiles of 16 rows where the depth allows it, more for 32; 0 restores the
+ * built-in choice).  Results do not depend on it. */
 int hm_thermal_set_launch(int rows);
 
 /* ---- batched and served forms ------------------------------------------ */
