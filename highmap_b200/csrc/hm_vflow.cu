@@ -15,13 +15,32 @@
  *
  * The reference round-trips the depth to the host around every step and
  * takes hmax on the host; here the depth stays in HBM and dt is formed on
- * the device: a max reduction over order-preserving integer keys of the
- * depth (exact for negative values too), then one thread computes dt into
- * a device slot that the step kernels read.  pow is evaluated in fp64 and
- * rounded once to fp32, which equals the host's powf except where the
- * exact power lies within about 2^-52 of a float rounding boundary.
+ * the device: the launch that ends a group of 10 steps also takes the max
+ * over order-preserving integer keys of the depth (exact for negative
+ * values too), and its last CTA turns it into the next group's dt.  pow is
+ * evaluated in fp64 and rounded once to fp32, which equals the host's powf
+ * except where the exact power lies within about 2^-52 of a float rounding
+ * boundary.
+ *
+ * Powers that are multiples of 1/2 from 1 to 4 (the default is 2.5) are
+ * x^floor times sqrt(x) in fp64, at most five roundings of 2^-53: the same
+ * accuracy at a fifth of pow's instructions.
+ *
+ * Kernels
+ *   k_vflow_block  up to VB_TMAX steps per launch on a 64 x 32 tile in
+ *                  registers (the layout of hm_thermal_block.cuh: a warp
+ *                  owns two rows, two columns per lane), up to 1.5 M
+ *                  cells, where a step's launch (4.1 us of host time) is
+ *                  longer than its arithmetic: 512^2, power 2.5, 200
+ *                  steps 2.51 ms with one step per launch and pow, 0.94 ms
+ *                  here (23 us a launch, bound by the fp64 pipe and its
+ *                  conversions).
+ *   k_vflow_step   one step, a 32 x 8 tile in shared memory (larger grids).
  */
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
 
 #include "hm_internal.h"
 #include "hm_vpipes.h"
@@ -48,50 +67,72 @@ __device__ __forceinline__ float funkey(unsigned k)
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+/* device scalars of a solve: the running max key, the CTAs done, the key
+ * of the last finished max and the time step */
+struct VfScalars
+{
+  unsigned slot, ticket, hmax;
+  float    dt;
+};
+
+/* power 0: the general pow; else twice the power, an integer in 2 .. 8 */
+struct VfConst
+{
+  float viscosity, power;
+  int   half;
+};
+
+/* x^power in fp64, rounded once (header) */
+__device__ __forceinline__ float vf_pow(float xf, const VfConst &c)
+{
+  if (c.half == 0) return powr(xf, c.power);
+  const double x = (double)xf, x2 = __dmul_rn(x, x); /* the square is exact */
+  double       r = c.half & 4 ? x2 : 1.0;            /* x^2 of 4 .. 7 halves */
+  if (c.half == 8) r = __dmul_rn(x2, x2);
+  else if (c.half & 2) r = c.half & 4 ? __dmul_rn(x2, x) : x;
+  if (c.half & 1) r = __dmul_rn(r, __dsqrt_rn(x));
+  return __double2float_rn(r);
+}
+
+__device__ __forceinline__ float face_mobility(float h, float hn, const VfConst &c)
+{
+  const float p = vf_pow(fmul(0.5f, fadd(h, hn)), c);
+  return c.viscosity == 1.f ? p : fdiv(p, c.viscosity); /* p / 1 is p */
+}
+
+/* The CTA's part of the max of h, m = the thread's greatest key; the last
+ * CTA stores the key, forms dt = 0.2 / fmax(hmax^power / viscosity, 1e-6)
+ * and re-arms the slot for the next max. */
+__device__ __forceinline__ void vf_max_commit(unsigned m, VfScalars *sc, unsigned nblocks, const VfConst &c)
+{
+  m = __reduce_max_sync(0xffffffffu, m);
+  const unsigned tid = threadIdx.y * blockDim.x + threadIdx.x;
+  if ((tid & 31u) == 0) atomicMax(&sc->slot, m);
+  __threadfence();
+  __syncthreads();
+  if (tid != 0) return;
+  if (atomicAdd(&sc->ticket, 1u) != nblocks - 1u) return;
+  __threadfence();
+  const unsigned key = atomicExch(&sc->slot, 0u);
+  sc->hmax = key;
+  const float p = vf_pow(funkey(key), c);
+  sc->dt = fdiv(0.2f, fmaxf(fdiv(p, c.viscosity), 1e-6f));
+  sc->ticket = 0u;
+}
+
+/* h = water_height * depth_map, its max and the first time step */
 __global__ void __launch_bounds__(VF_NT) k_vflow_init(float *__restrict__ h, const float *__restrict__ depth_map,
-                                                      float water_height, size_t n)
-{
-  for (size_t k = blockIdx.x * (size_t)VF_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * VF_NT)
-    h[k] = __fmul_rn(water_height, depth_map[k]);
-}
-
-/* clear the key slot; dt = the caller's (replaced before the first step) */
-__global__ void k_vflow_reset(unsigned *slot, float *dtp, float dt)
-{
-  *slot = 0u;
-  *dtp = dt;
-}
-
-/* slot = key of max(h); the slot must hold 0 (the least key) before */
-__global__ void __launch_bounds__(VF_NT) k_vflow_max(const float *__restrict__ h, size_t n, unsigned *slot)
+                                                      float water_height, size_t n, VfScalars *sc, VfConst c)
 {
   unsigned m = 0u;
   for (size_t k = blockIdx.x * (size_t)VF_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * VF_NT)
   {
-    const unsigned c = fkey(h[k]);
-    m = c > m ? c : m;
+    const float    v = __fmul_rn(water_height, depth_map[k]);
+    const unsigned key = fkey(v);
+    h[k] = v;
+    m = key > m ? key : m;
   }
-  for (int o = 16; o > 0; o >>= 1)
-  {
-    const unsigned t = __shfl_xor_sync(0xffffffffu, m, o);
-    m = t > m ? t : m;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMax(slot, m);
-}
-
-/* dt = 0.2 / fmax(hmax^power / viscosity, 1e-6); the key slot is cleared
- * for the next reduction */
-__global__ void k_vflow_dt(unsigned *slot, float viscosity, float power, float *dt)
-{
-  const float hmax = funkey(*slot);
-  const float mobility = fdiv(powr(hmax, power), viscosity);
-  *dt = fdiv(0.2f, fmaxf(mobility, 1e-6f));
-  *slot = 0u;
-}
-
-__device__ __forceinline__ float face_mobility(float h, float hn, float viscosity, float power)
-{
-  return fdiv(powr(fmul(0.5f, fadd(h, hn)), power), viscosity);
+  vf_max_commit(m, sc, gridDim.x, c);
 }
 
 /* One step over a 32 x 8 tile.  Each face mobility is evaluated once, by
@@ -103,8 +144,8 @@ __device__ __forceinline__ float face_mobility(float h, float hn, float viscosit
 constexpr int VT_X = 32, VT_Y = 8;
 
 __global__ void __launch_bounds__(VT_X *VT_Y) k_vflow_step(const float *__restrict__ z, const float *__restrict__ hin,
-                                                          float *__restrict__ hout, int nx, int ny,
-                                                          const float *__restrict__ dtp, float viscosity, float power)
+                                                          float *__restrict__ hout, int nx, int ny, VfScalars *sc,
+                                                          VfConst c, int want_max)
 {
   __shared__ float me[VT_Y][VT_X + 1]; /* me[ty][tx + 1]: east face of (tx, ty); [ty][0]: west edge  */
   __shared__ float mn[VT_Y + 1][VT_X]; /* mn[ty + 1][tx]: north face of (tx, ty); [0][tx]: south edge */
@@ -119,31 +160,149 @@ __global__ void __launch_bounds__(VT_X *VT_Y) k_vflow_step(const float *__restri
   const float  hxp = hin[ke], hxm = hin[kw], hyp = hin[kn], hym = hin[ks];
   if (in)
   {
-    me[ty][tx + 1] = face_mobility(h, hxp, viscosity, power);
-    mn[ty + 1][tx] = face_mobility(h, hyp, viscosity, power);
-    if (tx == 0) me[ty][0] = face_mobility(h, hxm, viscosity, power);
-    if (ty == 0) mn[0][tx] = face_mobility(h, hym, viscosity, power);
+    me[ty][tx + 1] = face_mobility(h, hxp, c);
+    mn[ty + 1][tx] = face_mobility(h, hyp, c);
+    if (tx == 0) me[ty][0] = face_mobility(h, hxm, c);
+    if (ty == 0) mn[0][tx] = face_mobility(h, hym, c);
   }
   __syncthreads();
-  if (!in) return;
-  const float dt = *dtp;
-  const float zc = z[k];
-  const float Hc = fadd(h, zc);
-  const float Hxp = fadd(hxp, z[ke]), Hxm = fadd(hxm, z[kw]), Hyp = fadd(hyp, z[kn]), Hym = fadd(hym, z[ks]);
-  const float Mp = me[ty][tx + 1], Mm = me[ty][tx], Myp = mn[ty + 1][tx], Mym = mn[ty][tx];
-  const float qxp = fmul(-Mp, fsub(Hxp, Hc));
-  const float qxm = fmul(-Mm, fsub(Hc, Hxm));
-  const float qyp = fmul(-Myp, fsub(Hyp, Hc));
-  const float qym = fmul(-Mym, fsub(Hc, Hym));
-  const float dhdt = -fsub(fadd(fsub(qxp, qxm), qyp), qym);
-  hout[k] = fmaxf(0.f, fadd(h, fmul(dt, dhdt)));
+  unsigned key = 0u;
+  if (in)
+  {
+    const float dt = sc->dt;
+    const float zc = z[k];
+    const float Hc = fadd(h, zc);
+    const float Hxp = fadd(hxp, z[ke]), Hxm = fadd(hxm, z[kw]), Hyp = fadd(hyp, z[kn]), Hym = fadd(hym, z[ks]);
+    const float Mp = me[ty][tx + 1], Mm = me[ty][tx], Myp = mn[ty + 1][tx], Mym = mn[ty][tx];
+    const float qxp = fmul(-Mp, fsub(Hxp, Hc));
+    const float qxm = fmul(-Mm, fsub(Hc, Hxm));
+    const float qyp = fmul(-Myp, fsub(Hyp, Hc));
+    const float qym = fmul(-Mym, fsub(Hc, Hym));
+    const float dhdt = -fsub(fadd(fsub(qxp, qxm), qyp), qym);
+    const float o = fmaxf(0.f, fadd(h, fmul(dt, dhdt)));
+    hout[k] = o;
+    key = fkey(o);
+  }
+  if (want_max) vf_max_commit(key, sc, gridDim.x * gridDim.y, c);
+}
+
+/* T steps on a tile of 64 columns x 32 rows.  Warp w holds rows 2 w and
+ * 2 w + 1 and reads the rows above and below them from shared memory; the
+ * terrain around the cells is loaded once for all steps.  Vertical faces
+ * are evaluated by the row below them (three per column and step for two
+ * rows), horizontal ones by the cell west of them, the value shuffled
+ * east.  The halo is that of hm_thermal_block.cuh, one cell per step. */
+constexpr int VB_NW = 16, VB_NT = 32 * VB_NW, VB_TY = 2 * VB_NW, VB_TMAX = 5;
+
+template <bool VEC>
+__device__ __forceinline__ float2 vb_load(const float *__restrict__ row, int x0, int x1)
+{
+  return VEC ? __ldg(reinterpret_cast<const float2 *>(row + x0)) : make_float2(__ldg(row + x0), __ldg(row + x1));
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(VB_NT)
+    k_vflow_block(const float *__restrict__ z, const float *__restrict__ hin, float *__restrict__ hout, int nx, int ny,
+                  VfScalars *sc, VfConst c, int T, int want_max)
+{
+  __shared__ float2 rows[2][VB_NW][2][32];
+  const int  HL = (T + 1) >> 1, W = 64 - 4 * HL;
+  const int  lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int  gx = blockIdx.x * W - 2 * HL + 2 * lane;
+  const int  j0 = blockIdx.y * (VB_TY - 2 * T) - T + 2 * wp; /* first of the warp's two rows */
+  const int  x0 = min(max(gx, 0), VEC ? nx - 2 : nx - 1), x1 = min(max(gx + 1, 0), nx - 1);
+  /* the warp's rows are 1, 2 of these; 0 and 3 are their neighbours */
+  float2     h[4], zr[4];
+  float      zw[2], ze[2]; /* terrain west of the pair and east of it */
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+  {
+    const size_t o = (size_t)min(max(j0 + q - 1, 0), ny - 1) * nx;
+    zr[q] = vb_load<VEC>(z + o, x0, x1);
+    if (q == 1 || q == 2)
+    {
+      h[q] = vb_load<VEC>(hin + o, x0, x1);
+      zw[q - 1] = __ldg(z + o + min(max(gx - 1, 0), nx - 1));
+      ze[q - 1] = __ldg(z + o + min(max(gx + 2, 0), nx - 1));
+    }
+  }
+  const float dt = sc->dt;
+  const bool  wedge = gx == 0, e0 = gx == nx - 1, e1 = gx + 1 == nx - 1;
+  for (int t = 0; t < T; t++)
+  {
+    const int par = t & 1;
+    rows[par][wp][0][lane] = h[1];
+    rows[par][wp][1][lane] = h[2];
+    __syncthreads();
+    if (2 * wp + 1 <= t || 2 * wp >= VB_TY - 1 - t) continue; /* halo rows that are done */
+    h[0] = rows[par][max(wp - 1, 0)][1][lane];
+    h[3] = rows[par][min(wp + 1, VB_NW - 1)][0][lane];
+    /* clamped reads: the row outside the grid is the edge row */
+    if (j0 == 0) h[0] = h[1];
+    if (j0 == -1) h[1] = h[2];
+    if (j0 == ny - 1) h[2] = h[1];
+    if (j0 + 1 == ny - 1) h[3] = h[2];
+    /* vertical faces below row 1, between rows 1 and 2, above row 2 */
+    float2 my[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      my[q] = make_float2(face_mobility(h[q].x, h[q + 1].x, c), face_mobility(h[q].y, h[q + 1].y, c));
+    float2 o[2];
+#pragma unroll
+    for (int q = 1; q < 3; q++)
+    {
+      const float2 hc = h[q];
+      float        hw = __shfl_up_sync(0xffffffffu, hc.y, 1), he = __shfl_down_sync(0xffffffffu, hc.x, 1);
+      if (wedge) hw = hc.x;
+      if (e1) he = hc.y;
+      const float hm = e0 ? hc.x : hc.y; /* east of the first column */
+      const float mx = face_mobility(hc.x, hm, c), mxe = face_mobility(hc.y, he, c);
+      float       mxw = __shfl_up_sync(0xffffffffu, mxe, 1);
+      if (wedge) mxw = face_mobility(hw, hc.x, c);
+      const float Hc0 = fadd(hc.x, zr[q].x), Hc1 = fadd(hc.y, zr[q].y);
+      const float Hw = fadd(hw, zw[q - 1]), He = fadd(he, ze[q - 1]), Hm = fadd(hm, zr[q].y);
+      const float Hn0 = fadd(h[q + 1].x, zr[q + 1].x), Hn1 = fadd(h[q + 1].y, zr[q + 1].y);
+      const float Hs0 = fadd(h[q - 1].x, zr[q - 1].x), Hs1 = fadd(h[q - 1].y, zr[q - 1].y);
+      auto cell = [&](float hh, float Hc, float He_, float Hw_, float Hn, float Hs, float Me, float Mw, float Mn,
+                      float Ms) {
+        const float qxp = fmul(-Me, fsub(He_, Hc)), qxm = fmul(-Mw, fsub(Hc, Hw_));
+        const float qyp = fmul(-Mn, fsub(Hn, Hc)), qym = fmul(-Ms, fsub(Hc, Hs));
+        return fmaxf(0.f, fadd(hh, fmul(dt, -fsub(fadd(fsub(qxp, qxm), qyp), qym))));
+      };
+      o[q - 1].x = cell(hc.x, Hc0, Hm, Hw, Hn0, Hs0, mx, mxw, my[q].x, my[q - 1].x);
+      o[q - 1].y = cell(hc.y, Hc1, He, Hc0, Hn1, Hs1, mxe, mx, my[q].y, my[q - 1].y);
+    }
+    h[1] = o[0];
+    h[2] = o[1];
+  }
+  unsigned key = 0u;
+  if (lane >= HL && lane < 32 - HL && gx < nx)
+  {
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+    {
+      const int tr = 2 * wp + q, j = j0 + q;
+      if (tr < T || tr >= VB_TY - T || j >= ny) continue;
+      float       *p = hout + (size_t)j * nx + gx;
+      const float2 v = h[q + 1];
+      if (VEC) *reinterpret_cast<float2 *>(p) = v;
+      else
+      {
+        p[0] = v.x;
+        if (gx + 1 < nx) p[1] = v.y;
+      }
+      const unsigned k0 = fkey(v.x), k1 = gx + 1 < nx ? fkey(v.y) : 0u;
+      key = max(key, max(k0, k1));
+    }
+  }
+  if (want_max) vf_max_commit(key, sc, gridDim.x * gridDim.y, c);
 }
 
 /* water_depth_dry_out: h -= ratio * hmax, then max(0, h) */
-__global__ void __launch_bounds__(VF_NT) k_vflow_dry_out(const float *__restrict__ h, const unsigned *slot,
+__global__ void __launch_bounds__(VF_NT) k_vflow_dry_out(const float *__restrict__ h, const VfScalars *sc,
                                                          float ratio, float *__restrict__ out, size_t n)
 {
-  const float drop = fmul(ratio, funkey(*slot));
+  const float drop = fmul(ratio, funkey(sc->hmax));
   for (size_t k = blockIdx.x * (size_t)VF_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * VF_NT)
   {
     const float w = fsub(h[k], drop);
@@ -155,7 +314,7 @@ __global__ void __launch_bounds__(VF_NT) k_vflow_dry_out(const float *__restrict
 
 size_t vflow_scratch_bytes(int nx, int ny)
 {
-  /* two depth grids, then the key slot and dt */
+  /* two depth grids, then the scalars */
   return 2 * align_up((size_t)nx * ny, 64) * sizeof(float) + 256;
 }
 
@@ -178,37 +337,53 @@ int vflow_core(const float *z, int nx, int ny, float water_height, const float *
   const size_t n = (size_t)nx * ny;
   const size_t na = align_up(n, 64);
   float       *hA = (float *)scratch, *hB = hA + na;
-  unsigned    *slot = (unsigned *)(hB + na);
-  float       *dtp = (float *)(slot + 1);
-  k_vflow_reset<<<1, 1, 0, s>>>(slot, dtp, dt);
-  HM_LAUNCH_CHECK("k_vflow_reset");
-  k_vflow_init<<<VF_GRID, VF_NT, 0, s>>>(hA, depth_map, water_height, n);
+  VfScalars   *sc = (VfScalars *)(hB + na);
+  VfConst      c{viscosity, power, 0};
+  for (int half = 2; half <= 8; half++)
+    if (power == 0.5f * (float)half) c.half = half;
+  (void)dt; /* replaced before the first step */
+  HM_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(VfScalars), s));
+  k_vflow_init<<<VF_GRID, VF_NT, 0, s>>>(hA, depth_map, water_height, n, sc, c);
   HM_LAUNCH_CHECK("k_vflow_init");
-  const dim3 tiles((nx + VT_X - 1) / VT_X, (ny + VT_Y - 1) / VT_Y);
+  /* Steps per launch: 5 up to 1.5 M cells (two launches per time step
+   * update), one above, where the recomputed halo (1.6 x at 5) costs more
+   * than the launches. */
+  const int  per = n <= 1500000 ? VB_TMAX : 1;
+  auto       al8 = [](const void *p) { return ((uintptr_t)p & 7u) == 0; };
   float     *cur = hA, *nxt = hB;
-  for (int it = 0; it < iterations; ++it)
+  for (int it = 0; it < iterations;)
   {
-    if (it % 10 == 0)
+    const int  T = std::min(per, std::min(10 - it % 10, iterations - it));
+    const bool last = it + T == iterations;
+    /* the depth's max is needed before every tenth step and by the dry-out */
+    const int  want_max = ((it + T) % 10 == 0 && !last) || (last && dry_out_ratio != 0.f);
+    if (last && dry_out_ratio == 0.f && water_depth != z) nxt = water_depth;
+    if (per == 1)
     {
-      k_vflow_max<<<VF_GRID, VF_NT, 0, s>>>(cur, n, slot);
-      HM_LAUNCH_CHECK("k_vflow_max");
-      k_vflow_dt<<<1, 1, 0, s>>>(slot, viscosity, power, dtp);
-      HM_LAUNCH_CHECK("k_vflow_dt");
+      const dim3 tiles((nx + VT_X - 1) / VT_X, (ny + VT_Y - 1) / VT_Y);
+      k_vflow_step<<<tiles, dim3(VT_X, VT_Y), 0, s>>>(z, cur, nxt, nx, ny, sc, c, want_max);
+      HM_LAUNCH_CHECK("k_vflow_step");
     }
-    k_vflow_step<<<tiles, dim3(VT_X, VT_Y), 0, s>>>(z, cur, nxt, nx, ny, dtp, viscosity, power);
-    HM_LAUNCH_CHECK("k_vflow_step");
+    else
+    {
+      const int  w = 64 - 4 * ((T + 1) / 2), hgt = VB_TY - 2 * T;
+      const dim3 tiles((nx + w - 1) / w, (ny + hgt - 1) / hgt);
+      const bool vec = nx % 2 == 0 && al8(z) && al8(cur) && al8(nxt);
+      if (vec) k_vflow_block<true><<<tiles, VB_NT, 0, s>>>(z, cur, nxt, nx, ny, sc, c, T, want_max);
+      else k_vflow_block<false><<<tiles, VB_NT, 0, s>>>(z, cur, nxt, nx, ny, sc, c, T, want_max);
+      HM_LAUNCH_CHECK("k_vflow_block");
+    }
     float *t = cur;
     cur = nxt;
     nxt = t;
+    it += T;
   }
   if (dry_out_ratio != 0.f)
   {
-    k_vflow_max<<<VF_GRID, VF_NT, 0, s>>>(cur, n, slot);
-    HM_LAUNCH_CHECK("k_vflow_max");
-    k_vflow_dry_out<<<VF_GRID, VF_NT, 0, s>>>(cur, slot, dry_out_ratio, water_depth, n);
+    k_vflow_dry_out<<<VF_GRID, VF_NT, 0, s>>>(cur, sc, dry_out_ratio, water_depth, n);
     HM_LAUNCH_CHECK("k_vflow_dry_out");
   }
-  else
+  else if (cur != water_depth)
     HM_CUDA_TRY(cudaMemcpyAsync(water_depth, cur, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
   return HM_OK;
 }
