@@ -419,19 +419,20 @@ int hm_flow_simulation(hm_context *ctx, const float *z, int nx, int ny, float wa
   if ((st = hm::use_device(ctx->device))) return st;
   const size_t n = (size_t)nx * ny;
   const size_t nbytes = n * sizeof(float);
-  const size_t total = 3 * align_up(nbytes, 256) + align_up(hm::flow_scratch_bytes(nx, ny), 256);
+  const bool   padded = hm::flow_wants_padding(nullptr, nx, ny, iterations); /* z goes to an aligned grid */
+  const size_t total = 3 * align_up(nbytes, 256) + align_up(hm::flow_scratch_bytes(nx, ny, padded), 256);
   void        *ws = nullptr;
   if ((st = hm::workspace(ctx, total, &ws))) return st;
   Slab         sl{(char *)ws};
   float       *dz = sl.take(n);
   float       *dm = sl.take(n);
   float       *dd = sl.take(n);
-  void        *scr = sl.take_bytes(hm::flow_scratch_bytes(nx, ny));
+  void        *scr = sl.take_bytes(hm::flow_scratch_bytes(nx, ny, padded));
   cudaStream_t s = ctx->stream;
   HM_CUDA_TRY(cudaMemcpyAsync(dz, z, nbytes, cudaMemcpyHostToDevice, s));
   HM_CUDA_TRY(cudaMemcpyAsync(dm, depth_map, nbytes, cudaMemcpyHostToDevice, s));
   st = hm::flow_simulation_core(dz, nx, ny, water_height, dm, iterations, dt, flux_diffusion, flux_diffusion_strength,
-                                dry_out_ratio, dd, scr, s);
+                                dry_out_ratio, dd, scr, s, padded);
   if (st)
   {
     cudaStreamSynchronize(s);
@@ -440,7 +441,8 @@ int hm_flow_simulation(hm_context *ctx, const float *z, int nx, int ny, float wa
   HM_CUDA_TRY(cudaMemcpyAsync(water_depth, dd, nbytes, cudaMemcpyDeviceToHost, s));
   unsigned dev_error = 0;
   HM_CUDA_TRY(
-      cudaMemcpyAsync(&dev_error, hm::flow_error_word(scr, nx, ny), sizeof dev_error, cudaMemcpyDeviceToHost, s));
+      cudaMemcpyAsync(&dev_error, hm::flow_error_word(scr, nx, ny, padded), sizeof dev_error, cudaMemcpyDeviceToHost,
+                      s));
   HM_CUDA_TRY(cudaStreamSynchronize(s));
   if (dev_error) return hm::fail(HM_ERR_TIMEOUT, "hm_flow_simulation: tile loads timed out on the device");
   return HM_OK;
@@ -455,10 +457,12 @@ int hm_flow_simulation_device(hm_context *ctx, const float *z, int nx, int ny, f
   int st = hm::flow_check_args(z, depth_map, water_depth, nx, ny, iterations, dt);
   if (st) return st;
   if ((st = hm::use_device(ctx->device))) return st;
-  void *ws = nullptr;
-  if ((st = hm::workspace(ctx, hm::flow_scratch_bytes(nx, ny), &ws))) return st;
+  const bool padded = hm::flow_wants_padding(z, nx, ny, iterations);
+  void      *ws = nullptr;
+  if ((st = hm::workspace(ctx, hm::flow_scratch_bytes(nx, ny, padded), &ws))) return st;
   return hm::flow_simulation_core(z, nx, ny, water_height, depth_map, iterations, dt, flux_diffusion,
-                                  flux_diffusion_strength, dry_out_ratio, water_depth, ws, (cudaStream_t)stream);
+                                  flux_diffusion_strength, dry_out_ratio, water_depth, ws, (cudaStream_t)stream,
+                                  padded);
 }
 
 int hm_flow_simulation_viscous(hm_context *ctx, const float *z, int nx, int ny, float water_height,
@@ -524,8 +528,10 @@ int hm_vpipes(hm_context *ctx, float *z, int nx, int ny, const hm_vpipes_params 
   const size_t nbytes = n * sizeof(float);
   size_t       fields = 1 + (rain_map ? 1 : 0) + (water_depth ? 1 : 0) + (sediment ? 1 : 0) + (vel_u ? 1 : 0) +
                   (vel_v ? 1 : 0);
-  size_t total = fields * align_up(nbytes, 256) + align_up(hm::vpipes_scratch_bytes(nx, ny), 256);
-  void  *ws = nullptr;
+  const bool   padded = hm::vpipes_wants_padding(nullptr, nx, ny, p.iterations); /* z goes to an aligned grid */
+  const size_t scratch = hm::vpipes_scratch_bytes(nx, ny, padded);
+  size_t       total = fields * align_up(nbytes, 256) + align_up(scratch, 256);
+  void        *ws = nullptr;
   if ((st = hm::workspace(ctx, total, &ws))) return st;
   Slab         sl{(char *)ws};
   float       *dz = sl.take(n);
@@ -534,11 +540,11 @@ int hm_vpipes(hm_context *ctx, float *z, int nx, int ny, const hm_vpipes_params 
   float       *ds = sediment ? sl.take(n) : nullptr;
   float       *du = vel_u ? sl.take(n) : nullptr;
   float       *dv = vel_v ? sl.take(n) : nullptr;
-  void        *scr = sl.take_bytes(hm::vpipes_scratch_bytes(nx, ny));
+  void        *scr = sl.take_bytes(scratch);
   cudaStream_t s = ctx->stream;
   HM_CUDA_TRY(cudaMemcpyAsync(dz, z, nbytes, cudaMemcpyHostToDevice, s));
   if (dr) HM_CUDA_TRY(cudaMemcpyAsync(dr, rain_map, nbytes, cudaMemcpyHostToDevice, s));
-  st = hm::vpipes_core(dz, nx, ny, p, dr, dd, ds, du, dv, scr, s);
+  st = hm::vpipes_core(dz, nx, ny, p, dr, dd, ds, du, dv, scr, s, padded);
   if (st)
   {
     cudaStreamSynchronize(s);
@@ -547,7 +553,7 @@ int hm_vpipes(hm_context *ctx, float *z, int nx, int ny, const hm_vpipes_params 
   /* a tile whose loads timed out wrote nothing: report it before the
    * results reach the caller's buffers, which then keep their contents */
   unsigned dev_error = 0;
-  HM_CUDA_TRY(cudaMemcpyAsync(&dev_error, hm::vpipes_error_word(scr, nx, ny), sizeof dev_error,
+  HM_CUDA_TRY(cudaMemcpyAsync(&dev_error, hm::vpipes_error_word(scr, nx, ny, padded), sizeof dev_error,
                               cudaMemcpyDeviceToHost, s));
   HM_CUDA_TRY(cudaStreamSynchronize(s));
   if (dev_error) return hm::fail(HM_ERR_TIMEOUT, "hm_vpipes: tile loads timed out on the device");
@@ -572,9 +578,11 @@ int hm_vpipes_device(hm_context *ctx, float *z, int nx, int ny, const hm_vpipes_
   int st = hm::vpipes_check_args(z, nx, ny, &p);
   if (st) return st;
   if ((st = hm::use_device(ctx->device))) return st;
-  void *ws = nullptr;
-  if ((st = hm::workspace(ctx, hm::vpipes_scratch_bytes(nx, ny), &ws))) return st;
-  return hm::vpipes_core(z, nx, ny, p, rain_map, water_depth, sediment, vel_u, vel_v, ws, (cudaStream_t)stream);
+  const bool padded = hm::vpipes_wants_padding(z, nx, ny, p.iterations);
+  void      *ws = nullptr;
+  if ((st = hm::workspace(ctx, hm::vpipes_scratch_bytes(nx, ny, padded), &ws))) return st;
+  return hm::vpipes_core(z, nx, ny, p, rain_map, water_depth, sediment, vel_u, vel_v, ws, (cudaStream_t)stream,
+                         padded);
 }
 
 

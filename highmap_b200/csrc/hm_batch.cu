@@ -199,11 +199,11 @@ __global__ void __launch_bounds__(BT, BATCH_CTAS_PER_SM)
       const int   x0 = tl.y * FT_TX, y0 = tl.z * FT_TY;
       const int   step = s_step;
       if (step == 0)
-        fwe_stage_cp_async(s_io, J.nx, J.ny, x0, y0, sm);
+        fwe_stage_cp_async(s_io, J.nx, J.ny, J.nx, x0, y0, sm);
       else if (stage16_tile(s_io, J.nx, J.ny, x0, y0))
         fwe_stage_cp_async16_step(s_io, J.u[(step & 1) ^ 1], J.v[(step & 1) ^ 1], J.nx, x0, y0, sm);
       else
-        fwe_stage_cp_async_step(s_io, J.u[(step & 1) ^ 1], J.v[(step & 1) ^ 1], J.nx, J.ny, x0, y0, sm);
+        fwe_stage_cp_async_step(s_io, J.u[(step & 1) ^ 1], J.v[(step & 1) ^ 1], J.nx, J.ny, J.nx, x0, y0, sm);
       __syncthreads();
       if (step > 0) advect_region1<false>(s_c, s_io.s1_prev, x0, y0, sm);
       if (J.maintain)
@@ -433,7 +433,7 @@ int finalize_job(hm_batch *b, HJob &h)
     if (f.z != j.z) HM_CUDA_TRY(cudaMemcpyAsync(j.z, f.z, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
     if (j.water_depth)
     {
-      int rc = hm::vpipes_final_depth(f.d, j.rain_map, h.dev.sc, par, h.dev.maintain != 0, j.water_depth, n, s);
+      int rc = hm::vpipes_final_depth(f.d, j.rain_map, h.dev.sc, par, h.dev.maintain != 0, j.water_depth, j.nx, j.ny, s);
       if (rc) return rc;
     }
     if (j.sediment) HM_CUDA_TRY(cudaMemcpyAsync(j.sediment, f.s, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -751,7 +751,7 @@ int hm_batch_add(hm_batch *b, const hm_job *job, int *job_id)
     const size_t parts = std::max(tiles, hm::vpipes_init_partials());
     d.sc = (hm::VpScalars *)((char *)d.partials + align_up(parts * sizeof(double), 256));
     const float init_depth = p.initial_water < 0.f ? p.water_height : p.initial_water;
-    if ((st = hm::vpipes_init(A, job->rain_map, (size_t)job->nx * job->ny, init_depth, d.sc, d.partials, b->stream)))
+    if ((st = hm::vpipes_init(A, job->rain_map, job->nx, job->ny, init_depth, d.sc, d.partials, b->stream)))
       return st;
   }
   h.live = true;
@@ -957,7 +957,8 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
     l->work += work(k);
     l->bytes = std::max(l->bytes, j.kind == HM_JOB_THERMAL
                                       ? hm::thermal_scratch_floats(j.nx, j.ny, j.deposition_map != nullptr) * sizeof(float)
-                                      : hm::vpipes_scratch_bytes(j.nx, j.ny));
+                                      : hm::vpipes_scratch_bytes(
+                                            j.nx, j.ny, hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations)));
   }
   cudaEvent_t fork = nullptr;
   if (!st && !large.empty())
@@ -1003,7 +1004,7 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
           hm_vpipes_params p = j.vpipes;
           p.iterations = j.iterations;
           rc = hm::vpipes_core(j.z, j.nx, j.ny, p, j.rain_map, j.water_depth, j.sediment, j.vel_u, j.vel_v, l.mem,
-                               l.s);
+                               l.s, hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations));
         }
         if (rc) return rc;
       }

@@ -11,8 +11,9 @@
  * state stays in HBM, and the dry-out is a max reduction plus one
  * elementwise pass.
  *
- * State: depth and the four fluxes in two copies (A, B), the terrain read
- * in place, a zero sediment grid (staged, unused).  Gravity, pipe area and
+ * State: depth and the four fluxes in two copies (A, B); the terrain is
+ * read in place, or from a copy where its rows miss the TMA rules (the
+ * state's rows are then padded to a multiple of 4 floats).  Gravity, pipe area and
  * pipe length are 1, evaporation 0, as in the reference's kernels.
  */
 #include <cuda_runtime.h>
@@ -29,26 +30,36 @@ namespace hm
 namespace
 {
 
-/* d = water_height * depth_map; fluxes of copy A and the sediment grid 0 */
+/* grid-stride index q of nx-float rows as an index of ld-float rows */
+__device__ __forceinline__ size_t padded_index(size_t q, int nx, int ld)
+{
+  return ld == nx ? q : q + (q / (size_t)nx) * (size_t)(ld - nx);
+}
+
+/* d = water_height * depth_map, fluxes of copy A 0; the terrain into zc
+ * where it is copied */
 __global__ void k_flow_init(float *__restrict__ d, const float *__restrict__ depth_map, float water_height,
                             float *__restrict__ fl, float *__restrict__ fr, float *__restrict__ ft,
-                            float *__restrict__ fb, float *__restrict__ s0, size_t n)
+                            float *__restrict__ fb, const float *__restrict__ z, float *__restrict__ zc, size_t n,
+                            int nx, int ld)
 {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
   {
-    d[k] = __fmul_rn(water_height, depth_map[k]);
-    fl[k] = fr[k] = ft[k] = fb[k] = s0[k] = 0.f;
+    const size_t k = padded_index(q, nx, ld);
+    d[k] = __fmul_rn(water_height, depth_map[q]);
+    fl[k] = fr[k] = ft[k] = fb[k] = 0.f;
+    if (zc) zc[k] = z[q];
   }
 }
 
 /* max of the depth (Array::max); depths are >= 0 (or -0), so the bit
  * patterns of the non-negative values order like the values */
-__global__ void k_flow_max(const float *__restrict__ d, size_t n, unsigned *__restrict__ out)
+__global__ void k_flow_max(const float *__restrict__ d, size_t n, unsigned *__restrict__ out, int nx, int ld)
 {
   unsigned m = 0u;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
   {
-    const float v = d[k];
+    const float v = d[padded_index(k, nx, ld)];
     const unsigned b = v > 0.f ? __float_as_uint(v) : 0u;
     m = b > m ? b : m;
   }
@@ -63,23 +74,34 @@ __global__ void k_flow_max(const float *__restrict__ d, size_t n, unsigned *__re
 /* water_depth_dry_out (water_depth.cpp:59-64): d = max(0, d - ratio * dmax),
  * written to the output */
 __global__ void k_flow_dry_out(const float *__restrict__ d, const unsigned *__restrict__ dmax_bits, float ratio,
-                               float *__restrict__ out, size_t n)
+                               float *__restrict__ out, size_t n, int nx, int ld)
 {
   const float drop = __fmul_rn(ratio, __uint_as_float(*dmax_bits));
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
   {
-    const float w = __fsub_rn(d[k], drop);
+    const float w = __fsub_rn(d[padded_index(k, nx, ld)], drop);
     out[k] = 0.f < w ? w : 0.f;
   }
 }
 
 } // namespace
 
-size_t flow_scratch_bytes(int nx, int ny)
+static size_t flow_state_floats(int nx, int ny, bool padded)
 {
-  /* depth and fluxes of two copies, the zero sediment grid, a max slot,
-   * the scalar block (its error word records TMA load timeouts) */
-  return align_up((size_t)nx * ny, 64) * sizeof(float) * 11 + 256 + align_up(sizeof(VpScalars), 256);
+  return align_up((padded ? align_up((size_t)nx, 4) : (size_t)nx) * ny, 64);
+}
+
+bool flow_wants_padding(const float *z, int nx, int ny, int iterations)
+{
+  return iterations > 0 && nx >= 40 && ny >= FT_H2 && (long long)nx * ny <= (1ll << 28) &&
+         (nx % 4 != 0 || ((uintptr_t)z & 15u) != 0);
+}
+
+size_t flow_scratch_bytes(int nx, int ny, bool padded)
+{
+  /* depth and fluxes of two copies, the terrain's copy, a max slot, the
+   * scalar block (its error word records TMA load timeouts) */
+  return flow_state_floats(nx, ny, padded) * sizeof(float) * 11 + 256 + align_up(sizeof(VpScalars), 256);
 }
 
 int flow_check_args(const float *z, const float *depth_map, const float *out, int nx, int ny, int iterations,
@@ -96,16 +118,18 @@ int flow_check_args(const float *z, const float *depth_map, const float *out, in
 
 int flow_simulation_core(const float *z, int nx, int ny, float water_height, const float *depth_map, int iterations,
                          float dt, int flux_diffusion, float flux_diffusion_strength, float dry_out_ratio,
-                         float *water_depth, void *scratch, cudaStream_t s)
+                         float *water_depth, void *scratch, cudaStream_t s, bool padded)
 {
   const size_t n = (size_t)nx * ny;
-  const size_t na = align_up(n, 64);
+  const size_t na = flow_state_floats(nx, ny, padded);
+  const int    ld = padded ? (int)align_up((size_t)nx, 4) : nx;
   float       *base = (float *)scratch;
-  float       *dA = base, *dB = base + na, *s0 = base + 10 * na;
+  float       *dA = base, *dB = base + na, *zc = padded ? base + 10 * na : nullptr;
+  float       *zt = padded ? zc : const_cast<float *>(z); /* read only */
   unsigned    *dmax = (unsigned *)(base + 11 * na);
   VpScalars   *sc = (VpScalars *)((char *)(base + 11 * na) + 256);
-  VpFields     A{const_cast<float *>(z), dA, s0, base + 2 * na, base + 3 * na, base + 4 * na, base + 5 * na};
-  VpFields     B{const_cast<float *>(z), dB, s0, base + 6 * na, base + 7 * na, base + 8 * na, base + 9 * na};
+  VpFields     A{zt, dA, nullptr, base + 2 * na, base + 3 * na, base + 4 * na, base + 5 * na};
+  VpFields     B{zt, dB, nullptr, base + 6 * na, base + 7 * na, base + 8 * na, base + 9 * na};
 
   hm_vpipes_params p;
   hm_vpipes_default_params(&p);
@@ -115,10 +139,11 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
   p.flux_diffusion_strength = flux_diffusion_strength;
   p.evap_rate = 0.f;
   p.maintain_water_volume = 0;
-  const VpConst c = vpipes_consts(nx, ny, p);
+  VpConst c = vpipes_consts(nx, ny, p);
+  c.ld = ld;
 
   HM_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(VpScalars), s));
-  k_flow_init<<<592, 256, 0, s>>>(dA, depth_map, water_height, A.fl, A.fr, A.ft, A.fb, s0, n);
+  k_flow_init<<<592, 256, 0, s>>>(dA, depth_map, water_height, A.fl, A.fr, A.ft, A.fb, z, zc, n, nx, ld);
   HM_LAUNCH_CHECK("k_flow_init");
 
   FweIo io;
@@ -130,12 +155,12 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
   {
     auto al8 = [](const void *q) { return ((uintptr_t)q & 7u) == 0; };
     const void *outs[] = {A.d, A.fl, A.fr, A.ft, A.fb, B.d, B.fl, B.fr, B.ft, B.fb};
-    bool        ok = nx % 2 == 0;
+    bool        ok = ld % 2 == 0;
     for (const void *q : outs) ok = ok && al8(q);
     io.vec = ok ? 1 : 0;
   }
   FweMaps    maps[2];
-  const bool tma = fwe_maps(A, nx, ny, &maps[0]) && fwe_maps(B, nx, ny, &maps[1]);
+  const bool tma = fwe_maps(A, nx, ny, ld, &maps[0]) && fwe_maps(B, nx, ny, ld, &maps[1]);
   const dim3 g1((nx + FT_TX - 1) / FT_TX, (ny + FT_TY - 1) / FT_TY);
   VpFields  *cur = &A, *nxt = &B;
   for (int it = 0; it < iterations; it++)
@@ -153,19 +178,22 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
   if (dry_out_ratio != 0.f)
   {
     HM_CUDA_TRY(cudaMemsetAsync(dmax, 0, sizeof(unsigned), s));
-    k_flow_max<<<592, 256, 0, s>>>(cur->d, n, dmax);
+    k_flow_max<<<592, 256, 0, s>>>(cur->d, n, dmax, nx, ld);
     HM_LAUNCH_CHECK("k_flow_max");
-    k_flow_dry_out<<<592, 256, 0, s>>>(cur->d, dmax, dry_out_ratio, water_depth, n);
+    k_flow_dry_out<<<592, 256, 0, s>>>(cur->d, dmax, dry_out_ratio, water_depth, n, nx, ld);
     HM_LAUNCH_CHECK("k_flow_dry_out");
   }
+  else if (ld != nx)
+    HM_CUDA_TRY(cudaMemcpy2DAsync(water_depth, (size_t)nx * sizeof(float), cur->d, (size_t)ld * sizeof(float),
+                                  (size_t)nx * sizeof(float), ny, cudaMemcpyDeviceToDevice, s));
   else
     HM_CUDA_TRY(cudaMemcpyAsync(water_depth, cur->d, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
   return HM_OK;
 }
 
-const unsigned *flow_error_word(const void *scratch, int nx, int ny)
+const unsigned *flow_error_word(const void *scratch, int nx, int ny, bool padded)
 {
-  const size_t na = align_up((size_t)nx * ny, 64);
+  const size_t na = flow_state_floats(nx, ny, padded);
   return &((const VpScalars *)((const char *)((const float *)scratch + 11 * na) + 256))->error;
 }
 

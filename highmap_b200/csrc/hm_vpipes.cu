@@ -41,22 +41,29 @@
 namespace hm
 {
 
+static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
+
 constexpr int VP_NT = 256;
 constexpr unsigned VP_INIT_BLOCKS = 296;
 
 /* ---- init --------------------------------------------------------- */
 
 /* d = initial depth * rain, s = f = 0; fp64 partial sums of d and rain
- * (hydraulic_vpipes_gpu.cpp:36-55). */
+ * (hydraulic_vpipes_gpu.cpp:36-55).  z_in: the caller's heights, copied
+ * into the state's own z (padded rows), or null when that is the caller's
+ * grid.  The sums run over the cells in the same order either way. */
 __global__ void __launch_bounds__(VP_NT)
-    k_vp_init(VpFields f, const float *rain, size_t n, float init_depth, double *partials)
+    k_vp_init(VpFields f, const float *rain, size_t n, float init_depth, double *partials, const float *z_in, int nx,
+              int ld)
 {
   const unsigned bid = blockIdx.x;
   double         sd = 0.0, sr = 0.0;
-  for (size_t k = bid * (size_t)VP_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * VP_NT)
+  for (size_t q = bid * (size_t)VP_NT + threadIdx.x; q < n; q += (size_t)gridDim.x * VP_NT)
   {
-    float r = rain ? rain[k] : 1.f;
-    float d = fmul(init_depth, r);
+    const size_t k = ld == nx ? q : q + (q / (size_t)nx) * (size_t)(ld - nx);
+    float        r = rain ? rain[q] : 1.f;
+    float        d = fmul(init_depth, r);
+    if (z_in) f.z[k] = z_in[q];
     f.d[k] = d;
     f.s[k] = 0.f;
     f.fl[k] = 0.f;
@@ -110,14 +117,17 @@ __global__ void k_vp_final_depth(const float *__restrict__ d,
                                  const VpScalars *__restrict__ sc,
                                  int parity,
                                  float *__restrict__ out,
-                                 size_t n)
+                                 size_t n,
+                                 int    nx,
+                                 int    ld)
 {
   const float add = MAINTAIN ? sc->add[parity] : 0.f;
   const float rvol = MAINTAIN ? sc->rvol : 1.f;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
   {
-    float r = rain ? rain[k] : 1.f;
-    out[k] = depth_d1<MAINTAIN, false>(d[k], r, add, rvol, 0.f);
+    const size_t k = ld == nx ? q : q + (q / (size_t)nx) * (size_t)(ld - nx);
+    float        r = rain ? rain[q] : 1.f;
+    out[q] = depth_d1<MAINTAIN, false>(d[k], r, add, rvol, 0.f);
   }
 }
 
@@ -125,10 +135,11 @@ __global__ void k_vp_final_depth(const float *__restrict__ d,
 /* host side                                                          */
 /* ------------------------------------------------------------------ */
 
-int vpipes_init(const VpFields &A, const float *rain, size_t n, float init_depth, VpScalars *sc, double *partials,
-                cudaStream_t s)
+int vpipes_init(const VpFields &A, const float *rain, int nx, int ny, float init_depth, VpScalars *sc,
+                double *partials, cudaStream_t s, const float *z_in, int ld)
 {
-  k_vp_init<<<VP_INIT_BLOCKS, VP_NT, 0, s>>>(A, rain, n, init_depth, partials);
+  k_vp_init<<<VP_INIT_BLOCKS, VP_NT, 0, s>>>(A, rain, (size_t)nx * ny, init_depth, partials, z_in, nx,
+                                             ld > 0 ? ld : nx);
   HM_LAUNCH_CHECK("k_vp_init");
   k_vp_init_finish<<<1, VP_NT, 0, s>>>(sc, partials, VP_INIT_BLOCKS);
   HM_LAUNCH_CHECK("k_vp_init_finish");
@@ -136,10 +147,12 @@ int vpipes_init(const VpFields &A, const float *rain, size_t n, float init_depth
 }
 
 int vpipes_final_depth(const float *d, const float *rain, const VpScalars *sc, int parity, bool maintain,
-                       float *out, size_t n, cudaStream_t s)
+                       float *out, int nx, int ny, cudaStream_t s, int ld)
 {
-  if (maintain) k_vp_final_depth<true><<<592, 256, 0, s>>>(d, rain, sc, parity, out, n);
-  else k_vp_final_depth<false><<<592, 256, 0, s>>>(d, rain, sc, parity, out, n);
+  const size_t n = (size_t)nx * ny;
+  if (ld <= 0) ld = nx;
+  if (maintain) k_vp_final_depth<true><<<592, 256, 0, s>>>(d, rain, sc, parity, out, n, nx, ld);
+  else k_vp_final_depth<false><<<592, 256, 0, s>>>(d, rain, sc, parity, out, n, nx, ld);
   HM_LAUNCH_CHECK("k_vp_final_depth");
   return HM_OK;
 }
@@ -220,9 +233,21 @@ static size_t defer_cap(int nx, int ny)
  * and writes its own) */
 constexpr size_t VP_GRIDS = 19;
 
-size_t vpipes_scratch_bytes(int nx, int ny)
+/* floats of one state grid: rows of nx, or padded to a multiple of 4 */
+static size_t state_floats(int nx, int ny, bool padded)
 {
-  const size_t n = align_up((size_t)nx * ny, 64);
+  return align_up((padded ? align_up((size_t)nx, 4) : (size_t)nx) * ny, 64);
+}
+
+bool vpipes_wants_padding(const float *z, int nx, int ny, int iterations)
+{
+  return iterations > 0 && nx >= 40 && ny >= FS_H && (long long)nx * ny <= (1ll << 28) &&
+         vpipes_pick_algo(nx, ny) == 0 && (nx % 4 != 0 || !aligned16(z));
+}
+
+size_t vpipes_scratch_bytes(int nx, int ny, bool padded)
+{
+  const size_t n = state_floats(nx, ny, padded);
   /* the grids, fp64 partials, the scalar block, the deferred list */
   return n * sizeof(float) * VP_GRIDS + partials_bytes(nx, ny) + align_up(sizeof(VpScalars), 256) +
          align_up(defer_cap(nx, ny) * sizeof(Deferred), 256);
@@ -233,6 +258,7 @@ VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p)
   VpConst c;
   c.nx = nx;
   c.ny = ny;
+  c.ld = nx;
   c.dt = p.dt;
   const float ga = p.gravity * p.pipe_area;
   c.dtga = p.dt * ga;
@@ -310,13 +336,14 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
   return fn;
 }
 
-/* map of an nx x ny fp32 grid read in boxes of 40 x box_rows, zeros outside */
-static bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, int box_rows)
+/* map of an nx x ny fp32 grid in rows of ld floats read in boxes of 40 x
+ * box_rows, zeros outside */
+static bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, int ld, int box_rows)
 {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
   cuuint64_t dims[2] = {(cuuint64_t)nx, (cuuint64_t)ny};
-  cuuint64_t strides[1] = {(cuuint64_t)nx * sizeof(float)};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(float)};
   cuuint32_t box[2] = {40u, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1u, 1u};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
@@ -324,29 +351,27 @@ static bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, i
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
-
-bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, AdvMaps *m)
+bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, int ld, AdvMaps *m)
 {
-  if (nx % 4 != 0 || nx < 40 || ny < FS_H) return false;
+  if (ld % 4 != 0 || nx < 40 || ny < FS_H) return false;
   if (!aligned16(u) || !aligned16(v) || !aligned16(s1)) return false;
-  return encode_grid_map(&m->u, u, nx, ny, FT_H1) && encode_grid_map(&m->v, v, nx, ny, FT_H1) &&
-         encode_grid_map(&m->s1, s1, nx, ny, FS_H);
+  return encode_grid_map(&m->u, u, nx, ny, ld, FT_H1) && encode_grid_map(&m->v, v, nx, ny, ld, FT_H1) &&
+         encode_grid_map(&m->s1, s1, nx, ny, ld, FS_H);
 }
 
 /* tensor maps of one state copy; false if the grid or buffers do not meet
  * the TMA rules (row pitch and bases 16-byte aligned, boxes no larger than
  * the grid) */
-bool fwe_maps(const VpFields &f, int nx, int ny, FweMaps *m)
+bool fwe_maps(const VpFields &f, int nx, int ny, int ld, FweMaps *m)
 {
-  if (nx % 4 != 0 || nx < 40 || ny < FT_H2) return false;
+  if (ld % 4 != 0 || nx < 40 || ny < FT_H2) return false;
   const float *all[7] = {f.z, f.d, f.s, f.fl, f.fr, f.ft, f.fb};
   for (const float *q : all)
     if (!aligned16(q)) return false;
-  return encode_grid_map(&m->z, f.z, nx, ny, FT_H2) && encode_grid_map(&m->d, f.d, nx, ny, FT_H2) &&
-         encode_grid_map(&m->s, f.s, nx, ny, FT_H1) && encode_grid_map(&m->fl, f.fl, nx, ny, FT_H1) &&
-         encode_grid_map(&m->fr, f.fr, nx, ny, FT_H1) && encode_grid_map(&m->ft, f.ft, nx, ny, FT_H1) &&
-         encode_grid_map(&m->fb, f.fb, nx, ny, FT_H1);
+  return encode_grid_map(&m->z, f.z, nx, ny, ld, FT_H2) && encode_grid_map(&m->d, f.d, nx, ny, ld, FT_H2) &&
+         (!f.s || encode_grid_map(&m->s, f.s, nx, ny, ld, FT_H1)) && encode_grid_map(&m->fl, f.fl, nx, ny, ld, FT_H1) &&
+         encode_grid_map(&m->fr, f.fr, nx, ny, ld, FT_H1) && encode_grid_map(&m->ft, f.ft, nx, ny, ld, FT_H1) &&
+         encode_grid_map(&m->fb, f.fb, nx, ny, ld, FT_H1);
 }
 
 /* The steps of vpipes_core with the tiled kernels.  The first step is
@@ -359,7 +384,8 @@ bool fwe_maps(const VpFields &f, int nx, int ny, FweMaps *m)
  * after the first go in pairs through k_vp_tb2, which writes the pair's
  * s1, u, v into the copy its first step would have written (the copy of
  * the step before the pair is still being read), so the copies alternate
- * once per pair; a step left over at the end runs alone. */
+ * once per pair; a step left over at the end runs alone.  The state grids
+ * have rows of c.ld floats, the caller's rows of nx. */
 static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &p, const VpConst &c, VpFields &A,
                               VpFields &B, float *const u_buf[2], float *const v_buf[2], float *const s1_buf[2],
                               const float *rain, float *water_depth, float *sediment, float *vel_u, float *vel_v,
@@ -368,9 +394,11 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
   const size_t n = (size_t)nx * ny;
   FweMaps      maps[2];
   AdvMaps      am[2];
-  const bool   tma = allow_tma && fwe_maps(A, nx, ny, &maps[0]) && fwe_maps(B, nx, ny, &maps[1]);
-  const bool   step_tma = tma && adv_maps(u_buf[0], v_buf[0], s1_buf[0], nx, ny, &am[0]) &&
-                        adv_maps(u_buf[1], v_buf[1], s1_buf[1], nx, ny, &am[1]);
+  const int    ld = c.ld;
+  const bool   in_step = ld == nx; /* the last step writes the velocity outputs itself */
+  const bool   tma = allow_tma && fwe_maps(A, nx, ny, ld, &maps[0]) && fwe_maps(B, nx, ny, ld, &maps[1]);
+  const bool   step_tma = tma && adv_maps(u_buf[0], v_buf[0], s1_buf[0], nx, ny, ld, &am[0]) &&
+                        adv_maps(u_buf[1], v_buf[1], s1_buf[1], nx, ny, ld, &am[1]);
   FweIo        io;
   memset(&io, 0, sizeof io);
   io.rain = rain;
@@ -380,20 +408,20 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
   io.kexp_one = p.k_discharge_exp == 1.f;
   io.tma_extra_tx = g_tma_extra_tx;
   {
-    /* pair stores: an even row length and 8-byte aligned outputs */
+    /* pair stores: an even row stride and 8-byte aligned outputs */
     auto al8 = [](const void *q) { return ((uintptr_t)q & 7u) == 0; };
     const void *outs[] = {A.z,      A.d,      A.fl,     A.fr,     A.ft,      A.fb,      B.z,   B.d,   B.fl, B.fr,
-                          B.ft,     B.fb,     s1_buf[0], s1_buf[1], u_buf[0], u_buf[1], v_buf[0], v_buf[1], vel_u,
-                          vel_v};
-    bool        ok = nx % 2 == 0;
+                          B.ft,     B.fb,     s1_buf[0], s1_buf[1], u_buf[0], u_buf[1], v_buf[0], v_buf[1],
+                          in_step ? vel_u : nullptr, in_step ? vel_v : nullptr};
+    bool        ok = ld % 2 == 0;
     for (const void *q : outs) ok = ok && al8(q);
     io.vec = ok ? 1 : 0;
-    /* 16-byte staging copies: a row length that is a multiple of 4 and
+    /* 16-byte staging copies: a row stride that is a multiple of 4 and
      * 16-byte aligned inputs */
     auto al16 = [](const void *q) { return ((uintptr_t)q & 15u) == 0; };
     const void *ins[] = {A.z, A.d, A.fl, A.fr, A.ft, A.fb, B.z,      B.d,      B.fl,     B.fr,
                          B.ft, B.fb, s1_buf[0], s1_buf[1], u_buf[0], u_buf[1], v_buf[0], v_buf[1]};
-    bool        ok16 = nx % 4 == 0;
+    bool        ok16 = ld % 4 == 0;
     for (const void *q : ins) ok16 = ok16 && al16(q);
     io.stage16 = ok16 ? 1 : 0;
   }
@@ -401,6 +429,7 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
   const int  row_groups = (ny + ADV_R - 1) / ADV_R;
   const dim3 g2((nx + 255) / 256, row_groups < 65535 ? row_groups : 65535);
   VpFields  *cur = &A, *nxt = &B;
+  float     *s_last = A.s; /* sediment after the last step; step 0 reads its zeros before */
   int        parity = 0;
   int        buf = 0; /* copy of u, v, s1 the current step writes */
   for (int it = 0; it < p.iterations; it++)
@@ -427,7 +456,7 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
       if (rc) return rc;
       if (last)
       {
-        k_vp_advect<ADV_R><<<g2, 256, 0, s>>>(tb.s1, tb.u, tb.v, nxt->s, c);
+        k_vp_advect<ADV_R><<<g2, 256, 0, s>>>(tb.s1, tb.u, tb.v, s_last, c);
         HM_LAUNCH_CHECK("k_vp_advect");
       }
       VpFields *t = cur;
@@ -444,8 +473,8 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     io.u = u_buf[buf];
     io.v = v_buf[buf];
     io.s1_prev = s1_buf[buf ^ 1];
-    io.u_out = last ? vel_u : nullptr;
-    io.v_out = last ? vel_v : nullptr;
+    io.u_out = last && in_step ? vel_u : nullptr;
+    io.v_out = last && in_step ? vel_v : nullptr;
     if (io.u_out && !io.v_out) io.v_out = io.v;
     if (io.v_out && !io.u_out) io.u_out = io.u;
     io.parity = parity;
@@ -460,7 +489,7 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
      * last step's runs here */
     if (last)
     {
-      k_vp_advect<ADV_R><<<g2, 256, 0, s>>>(io.s1, io.u, io.v, nxt->s, c);
+      k_vp_advect<ADV_R><<<g2, 256, 0, s>>>(io.s1, io.u, io.v, s_last, c);
       HM_LAUNCH_CHECK("k_vp_advect");
     }
     VpFields *t = cur;
@@ -469,13 +498,26 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     parity ^= 1;
     buf ^= 1;
   }
-  if (cur->z != z) HM_CUDA_TRY(cudaMemcpyAsync(z, cur->z, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  if (water_depth)
+  /* results into the caller's grids (rows of nx) */
+  auto result = [&](float *dst, const float *src) -> int {
+    if (!dst || src == dst) return HM_OK;
+    if (ld == nx) HM_CUDA_TRY(cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    else
+      HM_CUDA_TRY(cudaMemcpy2DAsync(dst, (size_t)nx * sizeof(float), src, (size_t)ld * sizeof(float),
+                                    (size_t)nx * sizeof(float), ny, cudaMemcpyDeviceToDevice, s));
+    return HM_OK;
+  };
+  int rc;
+  if ((rc = result(z, cur->z))) return rc;
+  if (water_depth &&
+      (rc = vpipes_final_depth(cur->d, rain, sc, parity, p.maintain_water_volume != 0, water_depth, nx, ny, s, ld)))
+    return rc;
+  if ((rc = result(sediment, s_last))) return rc;
+  if (!in_step && p.iterations > 0)
   {
-    int rc = vpipes_final_depth(cur->d, rain, sc, parity, p.maintain_water_volume != 0, water_depth, n, s);
-    if (rc) return rc;
+    if ((rc = result(vel_u, u_buf[buf ^ 1]))) return rc;
+    if ((rc = result(vel_v, v_buf[buf ^ 1]))) return rc;
   }
-  if (sediment) HM_CUDA_TRY(cudaMemcpyAsync(sediment, cur->s, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
   if (p.iterations == 0)
   {
     if (vel_u) HM_CUDA_TRY(cudaMemsetAsync(vel_u, 0, n * sizeof(float), s));
@@ -484,9 +526,9 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
   return HM_OK;
 }
 
-const unsigned *vpipes_error_word(const void *scratch_buf, int nx, int ny)
+const unsigned *vpipes_error_word(const void *scratch_buf, int nx, int ny, bool padded)
 {
-  const size_t na = align_up((size_t)nx * ny, 64);
+  const size_t na = state_floats(nx, ny, padded);
   const char  *partials = (const char *)scratch_buf + VP_GRIDS * na * sizeof(float);
   return &((const VpScalars *)(partials + partials_bytes(nx, ny)))->error;
 }
@@ -501,10 +543,11 @@ int vpipes_core(float *z,
                 float *vel_u,
                 float *vel_v,
                 void *scratch_buf,
-                cudaStream_t s)
+                cudaStream_t s,
+                bool padded)
 {
   const size_t n = (size_t)nx * ny;
-  const size_t na = align_up(n, 64);
+  const size_t na = state_floats(nx, ny, padded);
   float       *base = (float *)scratch_buf;
   VpFields     A, B;
   A.z = z;
@@ -532,19 +575,28 @@ int vpipes_core(float *z,
   df.count = sc->defer_count;
   df.cap = (unsigned)defer_cap(nx, ny);
 
-  const VpConst c = vpipes_consts(nx, ny, p);
+  VpConst     c = vpipes_consts(nx, ny, p);
+  /* padded: the state's rows take the next multiple of 4 floats and copy
+   * A's z is a grid of its own, in the place of copy B's sediment, which
+   * the tiled steps do not use (they take A's zeros in the first step and
+   * leave the last advection's result in A) */
+  if (padded)
+  {
+    c.ld = (int)align_up((size_t)nx, 4);
+    A.z = B.s;
+  }
   const float   init_depth = p.initial_water < 0.f ? p.water_height : p.initial_water;
 
   {
-    int rc = vpipes_init(A, rain, n, init_depth, sc, partials, s);
+    int rc = vpipes_init(A, rain, nx, ny, init_depth, sc, partials, s, padded ? z : nullptr, c.ld);
     if (rc) return rc;
   }
 
   const FusedCfg cfg = vpipes_pick_config(nx, ny);
   const int      algo = vpipes_pick_algo(nx, ny);
-  if (algo == 0 || algo == 2 || algo == 3)
+  if (padded || algo == 0 || algo == 2 || algo == 3)
     return vpipes_tiled_steps(z, nx, ny, p, c, A, B, u2, v2, s12, rain, water_depth, sediment, vel_u, vel_v, sc,
-                              partials, algo != 2, algo == 3 ? 2 : 1, s);
+                              partials, padded || algo != 2, !padded && algo == 3 ? 2 : 1, s);
   VpStep         st;
   st.rain = rain;
   st.H = cfg.h;
@@ -577,7 +629,7 @@ int vpipes_core(float *z,
 
   if (water_depth)
   {
-    int rc = vpipes_final_depth(cur->d, rain, sc, parity, p.maintain_water_volume != 0, water_depth, n, s);
+    int rc = vpipes_final_depth(cur->d, rain, sc, parity, p.maintain_water_volume != 0, water_depth, nx, ny, s);
     if (rc) return rc;
   }
   if (sediment) HM_CUDA_TRY(cudaMemcpyAsync(sediment, cur->s, n * sizeof(float), cudaMemcpyDeviceToDevice, s));

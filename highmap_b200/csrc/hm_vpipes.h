@@ -9,29 +9,39 @@
 namespace hm
 {
 int    vpipes_check_args(const float *z, int nx, int ny, const hm_vpipes_params *p);
-size_t vpipes_scratch_bytes(int nx, int ny);
+/* Whether a solve should keep its state in rows padded to a multiple of 4
+ * floats, with a copy of z: where nx or z miss the TMA rules, the copy
+ * (8 B per cell in, 8 out) buys the TMA-staged kernels for every step:
+ * 1023 x 767, rain map and top-up, 50 steps, 1575 us with clamped 4-byte
+ * copies, 1394 us padded.  Not above 2^28 cells, so that memory limits stay where
+ * they are, nor where another kernel is asked for or tuned. */
+bool   vpipes_wants_padding(const float *z, int nx, int ny, int iterations);
+size_t vpipes_scratch_bytes(int nx, int ny, bool padded);
 /* Device pointers; ordered on s.  rain and the outputs are nullable. */
 int    vpipes_core(float *z, int nx, int ny, const hm_vpipes_params &p, const float *rain, float *water_depth,
-                   float *sediment, float *vel_u, float *vel_v, void *scratch_buf, cudaStream_t s);
+                   float *sediment, float *vel_u, float *vel_v, void *scratch_buf, cudaStream_t s, bool padded);
 struct VpFields;
 struct VpScalars;
 struct VpConst;
 VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p);
-/* initial state of copy A (depth, zero sediment and fluxes) and V0, R */
-int     vpipes_init(const VpFields &A, const float *rain, size_t n, float init_depth, VpScalars *sc,
-                    double *partials, cudaStream_t s);
+/* initial state of copy A (depth, zero sediment and fluxes; z from z_in
+ * where given) in rows of ld floats (0: nx), and V0, R */
+int     vpipes_init(const VpFields &A, const float *rain, int nx, int ny, float init_depth, VpScalars *sc,
+                    double *partials, cudaStream_t s, const float *z_in = nullptr, int ld = 0);
 /* device address of the solve's error word (bit 0: a tile's TMA loads
  * timed out and the tile was skipped) inside the scratch of vpipes_core */
-const unsigned *vpipes_error_word(const void *scratch_buf, int nx, int ny);
+const unsigned *vpipes_error_word(const void *scratch_buf, int nx, int ny, bool padded);
 /* flow_simulation (hm_flow.cu): device pointers, ordered on s; scratch of
  * flow_scratch_bytes; water_depth receives the final depth */
 int             flow_check_args(const float *z, const float *depth_map, const float *out, int nx, int ny,
                                 int iterations, float dt);
-size_t          flow_scratch_bytes(int nx, int ny);
+bool            flow_wants_padding(const float *z, int nx, int ny, int iterations); /* as vpipes_wants_padding */
+size_t          flow_scratch_bytes(int nx, int ny, bool padded);
 int             flow_simulation_core(const float *z, int nx, int ny, float water_height, const float *depth_map,
                                      int iterations, float dt, int flux_diffusion, float flux_diffusion_strength,
-                                     float dry_out_ratio, float *water_depth, void *scratch, cudaStream_t s);
-const unsigned *flow_error_word(const void *scratch, int nx, int ny);
+                                     float dry_out_ratio, float *water_depth, void *scratch, cudaStream_t s,
+                                     bool padded);
+const unsigned *flow_error_word(const void *scratch, int nx, int ny, bool padded);
 /* flow_simulation_viscous (hm_vflow.cu): device pointers, ordered on s;
  * scratch of vflow_scratch_bytes; water_depth receives the final depth */
 int             vflow_check_args(const float *z, const float *depth_map, const float *out, int nx, int ny,
@@ -42,9 +52,10 @@ int             vflow_core(const float *z, int nx, int ny, float water_height, c
                            void *scratch, cudaStream_t s);
 /* fp64 partial-sum slots vpipes_init needs */
 size_t  vpipes_init_partials();
-/* water-depth output: stored depth plus the top-up of the last step */
+/* water-depth output: stored depth (rows of ld floats, 0: nx) plus the
+ * top-up of the last step */
 int     vpipes_final_depth(const float *d, const float *rain, const VpScalars *sc, int parity, bool maintain,
-                           float *out, size_t n, cudaStream_t s);
+                           float *out, int nx, int ny, cudaStream_t s, int ld = 0);
 } // namespace hm
 
 #endif

@@ -58,6 +58,7 @@ __device__ __forceinline__ float powr(float b, float e) { return __double2float_
 struct VpConst
 {
   int   nx, ny;
+  int   ld;          /* row stride of the state grids in floats (>= nx; the caller's grids have rows of nx) */
   float dt;
   float dtga;        /* dt * (gravity * pipe_area)                    */
   float pl;          /* pipe length                                    */

@@ -126,10 +126,10 @@ struct FweIo
   const float *rain;
   int          parity;
   int          maintain, diffusion, pl_one, kexp_one;
-  float       *u_out, *v_out; /* last step: velocity outputs, nullable */
-  int          vec;           /* nx even and every output 8-byte aligned: pair stores */
+  float       *u_out, *v_out; /* last step: velocity outputs (rows of c.ld), both or neither */
+  int          vec;           /* even row stride and every output 8-byte aligned: pair stores */
   int          flow_only;     /* flow_simulation step (FWE_FLOWONLY kernels) */
-  int          stage16;       /* nx a multiple of 4 and every staged grid 16-byte aligned: a tile whose
+  int          stage16;       /* row stride a multiple of 4 and every staged grid 16-byte aligned: a tile whose
                                * boxes lie inside the grid may stage them in 16-byte copies */
   unsigned     tma_extra_tx;  /* bytes a TMA tile's barrier expects beyond its boxes: 0, or the
                                * test hook's count, which makes every tile's wait run out */
@@ -150,8 +150,9 @@ struct AdvMaps
   CUtensorMap u, v, s1;
 };
 
-/* bytes the seven TMA boxes deliver */
+/* bytes the seven TMA boxes deliver, and the six without the sediment */
 constexpr unsigned FWE_TMA_BYTES = 4u * 40u * (2u * FT_H2 + 5u * FT_H1);
+constexpr unsigned FLOW_TMA_BYTES = 4u * 40u * (2u * FT_H2 + 4u * FT_H1);
 /* bytes the nine boxes of k_vp_step_tma deliver: group A (the previous
  * step's u, v and s1, and the stored depth), on which the advection and
  * the depth pass run while group B (z and the four old fluxes) is still
@@ -164,21 +165,21 @@ static_assert(STEP_TMA_BYTES_A + STEP_TMA_BYTES_B == STEP_TMA_BYTES, "the two gr
 /* cp.async staging: z, d on the halo-2 region; s and old fluxes on the
  * halo-1 region; loads clamped to the grid, so every raw neighbour read is
  * the reference's clamp-to-edge read */
-__device__ __forceinline__ void fwe_stage_cp_async(const FweIo &io, int nx, int ny, int x0, int y0, FweSmem &sm)
+__device__ __forceinline__ void fwe_stage_cp_async(const FweIo &io, int nx, int ny, int ld, int x0, int y0, FweSmem &sm)
 {
   const int tid = threadIdx.x;
   for (int e = tid; e < FT_W2 * FT_H2; e += FT_NT)
   {
     const int    ly = e / FT_W2, lx = e - ly * FT_W2;
-    const size_t k = (size_t)clampi(y0 - 2 + ly, 0, ny - 1) * nx + clampi(x0 - 2 + lx, 0, nx - 1);
+    const size_t k = (size_t)clampi(y0 - 2 + ly, 0, ny - 1) * ld + clampi(x0 - 2 + lx, 0, nx - 1);
     cp_async4(&sm.z[ly][lx + 2], io.in.z + k);
     cp_async4(&sm.d[ly][lx + 2], io.in.d + k);
   }
   for (int e = tid; e < FT_W1 * FT_H1; e += FT_NT)
   {
     const int    ly = e / FT_W1, lx = e - ly * FT_W1;
-    const size_t k = (size_t)clampi(y0 - 1 + ly, 0, ny - 1) * nx + clampi(x0 - 1 + lx, 0, nx - 1);
-    cp_async4(&sm.s[ly][lx + 3], io.in.s + k);
+    const size_t k = (size_t)clampi(y0 - 1 + ly, 0, ny - 1) * ld + clampi(x0 - 1 + lx, 0, nx - 1);
+    if (!io.flow_only) cp_async4(&sm.s[ly][lx + 3], io.in.s + k);
     cp_async4(&sm.fo[0][ly][lx + 3], io.in.fl + k);
     cp_async4(&sm.fo[1][ly][lx + 3], io.in.fr + k);
     cp_async4(&sm.fo[2][ly][lx + 3], io.in.ft + k);
@@ -195,13 +196,13 @@ __device__ __forceinline__ void fwe_stage_cp_async(const FweIo &io, int nx, int 
  * are read nowhere else).  io.u, io.v are this step's outputs; the
  * previous step's velocity comes in as u_prev, v_prev. */
 __device__ __forceinline__ void fwe_stage_cp_async_step(const FweIo &io, const float *u_prev, const float *v_prev,
-                                                        int nx, int ny, int x0, int y0, FweSmem &sm)
+                                                        int nx, int ny, int ld, int x0, int y0, FweSmem &sm)
 {
   const int tid = threadIdx.x;
   for (int e = tid; e < FT_W2 * FT_H2; e += FT_NT)
   {
     const int    ly = e / FT_W2, lx = e - ly * FT_W2;
-    const size_t k = (size_t)clampi(y0 - 2 + ly, 0, ny - 1) * nx + clampi(x0 - 2 + lx, 0, nx - 1);
+    const size_t k = (size_t)clampi(y0 - 2 + ly, 0, ny - 1) * ld + clampi(x0 - 2 + lx, 0, nx - 1);
     cp_async4(&sm.z[ly][lx + 2], io.in.z + k);
     cp_async4(&sm.d[ly][lx + 2], io.in.d + k);
   }
@@ -209,7 +210,7 @@ __device__ __forceinline__ void fwe_stage_cp_async_step(const FweIo &io, const f
   {
     const int    ly = e / FT_W1, lx = e - ly * FT_W1;
     const int    gx = x0 - 1 + lx, gy = y0 - 1 + ly;
-    const size_t k = (size_t)clampi(gy, 0, ny - 1) * nx + clampi(gx, 0, nx - 1);
+    const size_t k = (size_t)clampi(gy, 0, ny - 1) * ld + clampi(gx, 0, nx - 1);
     cp_async4(&sm.fo[0][ly][lx + 3], io.in.fl + k);
     cp_async4(&sm.fo[1][ly][lx + 3], io.in.fr + k);
     cp_async4(&sm.fo[2][ly][lx + 3], io.in.ft + k);
@@ -224,7 +225,7 @@ __device__ __forceinline__ void fwe_stage_cp_async_step(const FweIo &io, const f
   {
     const int ly = e / FW, lx = e - ly * FW;
     const int gx = x0 - 4 + lx, gy = y0 - 4 + ly;
-    if (gx >= 0 && gx < nx && gy >= 0 && gy < ny) cp_async4(&sm.adv.s1[ly][lx], io.s1_prev + (size_t)gy * nx + gx);
+    if (gx >= 0 && gx < nx && gy >= 0 && gy < ny) cp_async4(&sm.adv.s1[ly][lx], io.s1_prev + (size_t)gy * ld + gx);
   }
   cp_async_commit();
   cp_async_wait<0>();
@@ -249,21 +250,21 @@ __device__ __forceinline__ void cp_async16(float *smem, const float *gmem)
  * at the same places (and the box columns that the clamped form leaves
  * unwritten, which no pass reads). */
 __device__ __forceinline__ void fwe_stage_cp_async16_step(const FweIo &io, const float *u_prev, const float *v_prev,
-                                                          int nx, int x0, int y0, FweSmem &sm)
+                                                          int ld, int x0, int y0, FweSmem &sm)
 {
   constexpr int Q = FW / 4; /* 16-byte copies per box row */
   const int     tid = threadIdx.x;
   for (int e = tid; e < Q * FT_H2; e += FT_NT)
   {
     const int    ly = e / Q, c = 4 * (e - ly * Q);
-    const size_t k = (size_t)(y0 - 2 + ly) * nx + (x0 - 4 + c);
+    const size_t k = (size_t)(y0 - 2 + ly) * ld + (x0 - 4 + c);
     cp_async16(&sm.z[ly][c], io.in.z + k);
     cp_async16(&sm.d[ly][c], io.in.d + k);
   }
   for (int e = tid; e < Q * FT_H1; e += FT_NT)
   {
     const int    ly = e / Q, c = 4 * (e - ly * Q);
-    const size_t k = (size_t)(y0 - 1 + ly) * nx + (x0 - 4 + c);
+    const size_t k = (size_t)(y0 - 1 + ly) * ld + (x0 - 4 + c);
     cp_async16(&sm.fo[0][ly][c], io.in.fl + k);
     cp_async16(&sm.fo[1][ly][c], io.in.fr + k);
     cp_async16(&sm.fo[2][ly][c], io.in.ft + k);
@@ -274,7 +275,7 @@ __device__ __forceinline__ void fwe_stage_cp_async16_step(const FweIo &io, const
   for (int e = tid; e < Q * FS_H; e += FT_NT)
   {
     const int ly = e / Q, c = 4 * (e - ly * Q);
-    cp_async16(&sm.adv.s1[ly][c], io.s1_prev + (size_t)(y0 - 4 + ly) * nx + (x0 - 4 + c));
+    cp_async16(&sm.adv.s1[ly][c], io.s1_prev + (size_t)(y0 - 4 + ly) * ld + (x0 - 4 + c));
   }
   cp_async_commit();
   cp_async_wait<0>();
@@ -317,13 +318,14 @@ __device__ __forceinline__ void fwe_fix_edges(int nx, int ny, int x0, int y0, Fw
   }
 }
 
-/* TMA staging: thread 0 arms the barrier and issues the seven box loads;
- * every thread waits (bounded).  Boxes read zeros outside the grid, so on
+/* TMA staging: thread 0 arms the barrier and issues the seven box loads
+ * (six without the sediment, WITH_S false); every thread waits (bounded).  Boxes read zeros outside the grid, so on
  * tiles that touch the grid's edge the cells outside are then overwritten
  * with their clamp-to-edge values (the clamped cell is always inside the
  * box; the edge test depends only on the tile, so the barrier inside it is
  * uniform).  Returns false, uniformly across the CTA, if the loads did not
  * complete in time. */
+template <bool WITH_S>
 __device__ __forceinline__ bool fwe_stage_tma(const FweMaps &maps, int nx, int ny, int x0, int y0, FweSmem &sm,
                                               unsigned extra_tx)
 {
@@ -336,10 +338,10 @@ __device__ __forceinline__ bool fwe_stage_tma(const FweMaps &maps, int nx, int n
   __syncthreads();
   if (tid == 0)
   {
-    mbar_arrive_expect_tx(&sm.bar, FWE_TMA_BYTES + extra_tx);
+    mbar_arrive_expect_tx(&sm.bar, (WITH_S ? FWE_TMA_BYTES : FLOW_TMA_BYTES) + extra_tx);
     tma_load_2d(&sm.z[0][0], &maps.z, x0 - 4, y0 - 2, &sm.bar);
     tma_load_2d(&sm.d[0][0], &maps.d, x0 - 4, y0 - 2, &sm.bar);
-    tma_load_2d(&sm.s[0][0], &maps.s, x0 - 4, y0 - 1, &sm.bar);
+    if (WITH_S) tma_load_2d(&sm.s[0][0], &maps.s, x0 - 4, y0 - 1, &sm.bar);
     tma_load_2d(&sm.fo[0][0][0], &maps.fl, x0 - 4, y0 - 1, &sm.bar);
     tma_load_2d(&sm.fo[1][0][0], &maps.fr, x0 - 4, y0 - 1, &sm.bar);
     tma_load_2d(&sm.fo[2][0][0], &maps.ft, x0 - 4, y0 - 1, &sm.bar);
@@ -348,7 +350,7 @@ __device__ __forceinline__ bool fwe_stage_tma(const FweMaps &maps, int nx, int n
   bool ok = mbar_wait_bounded(&sm.bar, 0);
   if (!ok) ok = mbar_wait_bounded(&sm.bar, 0); /* loads still in flight: give them a second window */
   if (!__syncthreads_and(ok)) return false;
-  fwe_fix_edges<true>(nx, ny, x0, y0, sm);
+  fwe_fix_edges<WITH_S>(nx, ny, x0, y0, sm);
   return true;
 }
 
@@ -421,7 +423,7 @@ __device__ __forceinline__ bool fwe_wait_tma_step_b(int nx, int ny, int x0, int 
 __device__ __forceinline__ void advect_cell(const VpConst &c, const float *__restrict__ s1g, int x0, int y0, int gx,
                                             int gy, int l, int cc, FweSmem &sm)
 {
-  const int   nx = c.nx, ny = c.ny;
+  const int   nx = c.nx, ny = c.ny, ld = c.ld;
   const float uu = sm.adv.u[gy - (y0 - 1)][gx - (x0 - 4)];
   const float vv = sm.adv.v[gy - (y0 - 1)][gx - (x0 - 4)];
   const float x = fsub((float)gx, fmul(c.dt, uu));
@@ -453,11 +455,11 @@ __device__ __forceinline__ void advect_cell(const VpConst &c, const float *__res
     }
     else
     {
-      const float *r = s1g + (size_t)tp.j0 * nx + tp.i0;
+      const float *r = s1g + (size_t)tp.j0 * ld + tp.i0;
       g00 = __ldg(r);
       g10 = __ldg(r + 1);
-      g01 = __ldg(r + nx);
-      g11 = __ldg(r + nx + 1);
+      g01 = __ldg(r + ld);
+      g11 = __ldg(r + ld + 1);
     }
     sm.s[l][cc] = blend(tp, g00, g10, g01, g11);
     return;
@@ -475,7 +477,7 @@ __device__ __forceinline__ void advect_cell(const VpConst &c, const float *__res
   }
   else
   {
-    const size_t r0 = (size_t)t.j0 * nx, r1 = (size_t)t.j1 * nx;
+    const size_t r0 = (size_t)t.j0 * ld, r1 = (size_t)t.j1 * ld;
     g00 = __ldg(s1g + r0 + t.i0);
     g10 = __ldg(s1g + r0 + t.i1);
     g01 = __ldg(s1g + r1 + t.i0);
@@ -676,7 +678,7 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
         water_cell<false>(c, d1.x, flc.x, frc.x, ftc.x, fbc.x, frw0, fle0, ftn.x, fbs.x, d2a, ua, va);
         water_cell<false>(c, d1.y, flc.y, frc.y, ftc.y, fbc.y, frc.x, fle1, ftn.y, fbs.y, d2b, ub, vb);
       }
-      const size_t k = (size_t)gy * nx + gx;
+      const size_t k = (size_t)gy * c.ld + gx;
       const bool   vec = INNER || io.vec != 0;
       if (FLOW_ONLY)
       {
@@ -753,7 +755,7 @@ template <bool MAINTAIN, int F>
 __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F)) k_vp_fwe(FweIo io, VpConst c, VpScalars *sc, double *partials)
 {
   __shared__ FweSmem sm;
-  fwe_stage_cp_async(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm);
+  fwe_stage_cp_async(io, c.nx, c.ny, c.ld, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm);
   __syncthreads();
   if (fwe_inner_tile(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY))
     fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
@@ -770,7 +772,7 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
     k_vp_fwe_tma(FweIo io, const __grid_constant__ FweMaps maps, VpConst c, VpScalars *sc, double *partials)
 {
   __shared__ FweSmem sm;
-  if (!fwe_stage_tma(maps, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm, io.tma_extra_tx))
+  if (!fwe_stage_tma<(F & FWE_FLOWONLY) == 0>(maps, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm, io.tma_extra_tx))
   {
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
     if (MAINTAIN)
@@ -800,8 +802,8 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
 {
   __shared__ FweSmem sm;
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
-  if (stage16_tile(io, c.nx, c.ny, x0, y0)) fwe_stage_cp_async16_step(io, u_prev, v_prev, c.nx, x0, y0, sm);
-  else fwe_stage_cp_async_step(io, u_prev, v_prev, c.nx, c.ny, x0, y0, sm);
+  if (stage16_tile(io, c.nx, c.ny, x0, y0)) fwe_stage_cp_async16_step(io, u_prev, v_prev, c.ld, x0, y0, sm);
+  else fwe_stage_cp_async_step(io, u_prev, v_prev, c.nx, c.ny, c.ld, x0, y0, sm);
   __syncthreads();
   /* the advected sediment is written here and read after fwe_compute's
    * first barrier */
@@ -887,12 +889,13 @@ struct TbIo
 };
 int launch_vp_tb2(const TbIo &io, const VpConst &c, cudaStream_t s);
 
-/* tensor maps of one state copy (hm_vpipes.cu); false if the grid or the
- * buffers do not meet the TMA rules (row pitch and bases 16-byte aligned,
- * boxes no larger than the grid) */
-bool fwe_maps(const VpFields &f, int nx, int ny, FweMaps *m);
+/* tensor maps of one state copy in rows of ld floats (hm_vpipes.cu); false
+ * if the grid or the buffers do not meet the TMA rules (row pitch and bases
+ * 16-byte aligned, boxes no larger than the grid).  f.s may be null (the
+ * flow-only step). */
+bool fwe_maps(const VpFields &f, int nx, int ny, int ld, FweMaps *m);
 /* tensor maps of one copy of s1, u, v for k_vp_step_tma; false as above */
-bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, AdvMaps *m);
+bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, int ld, AdvMaps *m);
 
 /* template flags of a step's options */
 inline int fwe_flags(const FweIo &io, const VpConst &c)
@@ -970,7 +973,7 @@ __device__ __forceinline__ void advect_rows(const float *__restrict__ s1,
 #pragma unroll
   for (int q = 0; q < R; q++)
   {
-    const size_t k = (size_t)min(jb + q, c.ny - 1) * c.nx + i;
+    const size_t k = (size_t)min(jb + q, c.ny - 1) * c.ld + i;
     uu[q] = __ldg(u + k);
     vv[q] = __ldg(v + k);
   }
@@ -983,7 +986,7 @@ __device__ __forceinline__ void advect_rows(const float *__restrict__ s1,
     const float  x = fsub((float)i, fmul(c.dt, uu[q]));
     const float  y = fsub((float)j, fmul(c.dt, vv[q]));
     t[q] = linear_tap(x, y, c.nx, c.ny);
-    const size_t r0 = (size_t)t[q].j0 * c.nx, r1 = (size_t)t[q].j1 * c.nx;
+    const size_t r0 = (size_t)t[q].j0 * c.ld, r1 = (size_t)t[q].j1 * c.ld;
     g[q][0] = __ldg(s1 + r0 + t[q].i0);
     g[q][1] = __ldg(s1 + r0 + t[q].i1);
     g[q][2] = __ldg(s1 + r1 + t[q].i0);
@@ -991,7 +994,7 @@ __device__ __forceinline__ void advect_rows(const float *__restrict__ s1,
   }
 #pragma unroll
   for (int q = 0; q < R; q++)
-    if (jb + q < c.ny) s_out[(size_t)(jb + q) * c.nx + i] = blend(t[q], g[q][0], g[q][1], g[q][2], g[q][3]);
+    if (jb + q < c.ny) s_out[(size_t)(jb + q) * c.ld + i] = blend(t[q], g[q][0], g[q][1], g[q][2], g[q][3]);
 }
 
 template <int R>
