@@ -115,6 +115,7 @@ __device__ __forceinline__ void job_io(const BJob &J, int step, FweIo &io)
   io.pl_one = J.pl_one;
   io.kexp_one = J.kexp_one;
   const bool last = step == J.iters - 1;
+  io.last = last;
   io.u_out = last ? J.u_out : nullptr;
   io.v_out = last ? J.v_out : nullptr;
   if (io.u_out && !io.v_out) io.v_out = io.v;
@@ -751,7 +752,8 @@ int hm_batch_add(hm_batch *b, const hm_job *job, int *job_id)
     const size_t parts = std::max(tiles, hm::vpipes_init_partials());
     d.sc = (hm::VpScalars *)((char *)d.partials + align_up(parts * sizeof(double), 256));
     const float init_depth = p.initial_water < 0.f ? p.water_height : p.initial_water;
-    if ((st = hm::vpipes_init(A, job->rain_map, job->nx, job->ny, init_depth, d.sc, d.partials, b->stream)))
+    if ((st = hm::vpipes_init(A, job->rain_map, job->nx, job->ny, init_depth, d.sc, d.partials, b->stream,
+                              !d.maintain && p.iterations > 0 ? p.rain_per_step : 0.f)))
       return st;
   }
   h.live = true;

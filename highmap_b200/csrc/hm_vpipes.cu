@@ -51,10 +51,12 @@ constexpr unsigned VP_INIT_BLOCKS = 296;
 /* d = initial depth * rain, s = f = 0; fp64 partial sums of d and rain
  * (hydraulic_vpipes_gpu.cpp:36-55).  z_in: the caller's heights, copied
  * into the state's own z (padded rows), or null when that is the caller's
- * grid.  The sums run over the cells in the same order either way. */
+ * grid.  The sums run over the cells in the same order either way.
+ * first_rain: the per-step rain of the first step, which the tiled steps
+ * without the volume top-up find in the stored depth (FweIo). */
 __global__ void __launch_bounds__(VP_NT)
     k_vp_init(VpFields f, const float *rain, size_t n, float init_depth, double *partials, const float *z_in, int nx,
-              int ld)
+              int ld, float first_rain)
 {
   const unsigned bid = blockIdx.x;
   double         sd = 0.0, sr = 0.0;
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(VP_NT)
     float        r = rain ? rain[q] : 1.f;
     float        d = fmul(init_depth, r);
     if (z_in) f.z[k] = z_in[q];
-    f.d[k] = d;
+    f.d[k] = first_rain != 0.f ? fadd(d, fmul(first_rain, r)) : d;
     f.s[k] = 0.f;
     f.fl[k] = 0.f;
     f.fr[k] = 0.f;
@@ -136,10 +138,10 @@ __global__ void k_vp_final_depth(const float *__restrict__ d,
 /* ------------------------------------------------------------------ */
 
 int vpipes_init(const VpFields &A, const float *rain, int nx, int ny, float init_depth, VpScalars *sc,
-                double *partials, cudaStream_t s, const float *z_in, int ld)
+                double *partials, cudaStream_t s, float first_rain, const float *z_in, int ld)
 {
   k_vp_init<<<VP_INIT_BLOCKS, VP_NT, 0, s>>>(A, rain, (size_t)nx * ny, init_depth, partials, z_in, nx,
-                                             ld > 0 ? ld : nx);
+                                             ld > 0 ? ld : nx, first_rain);
   HM_LAUNCH_CHECK("k_vp_init");
   k_vp_init_finish<<<1, VP_NT, 0, s>>>(sc, partials, VP_INIT_BLOCKS);
   HM_LAUNCH_CHECK("k_vp_init_finish");
@@ -276,9 +278,6 @@ VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p)
   c.keep = 1.f - p.dt * p.evap_rate;
   c.rps = p.rain_per_step;
   c.fnx = (float)nx;
-  /* nx - 0.5 is a float exactly while nx < 2^23 */
-  c.xhi = nx < (1 << 22) ? (float)nx - 0.5f : 0.f;
-  c.yhi = ny < (1 << 22) ? (float)ny - 0.5f : 0.f;
   return c;
 }
 
@@ -447,6 +446,7 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
       tb.s1 = s1_buf[buf];
       tb.u = u_buf[buf];
       tb.v = v_buf[buf];
+      tb.last = last;
       tb.u_out = last ? vel_u : nullptr;
       tb.v_out = last ? vel_v : nullptr;
       tb.diffusion = io.diffusion;
@@ -473,6 +473,7 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     io.u = u_buf[buf];
     io.v = v_buf[buf];
     io.s1_prev = s1_buf[buf ^ 1];
+    io.last = last;
     io.u_out = last && in_step ? vel_u : nullptr;
     io.v_out = last && in_step ? vel_v : nullptr;
     if (io.u_out && !io.v_out) io.v_out = io.v;
@@ -587,14 +588,17 @@ int vpipes_core(float *z,
   }
   const float   init_depth = p.initial_water < 0.f ? p.water_height : p.initial_water;
 
+  const FusedCfg cfg = vpipes_pick_config(nx, ny);
+  const int      algo = vpipes_pick_algo(nx, ny);
+  const bool     tiled = padded || algo == 0 || algo == 2 || algo == 3;
   {
-    int rc = vpipes_init(A, rain, nx, ny, init_depth, sc, partials, s, padded ? z : nullptr, c.ld);
+    const bool pre = tiled && !p.maintain_water_volume && p.iterations > 0;
+    int rc = vpipes_init(A, rain, nx, ny, init_depth, sc, partials, s, pre ? p.rain_per_step : 0.f,
+                         padded ? z : nullptr, c.ld);
     if (rc) return rc;
   }
 
-  const FusedCfg cfg = vpipes_pick_config(nx, ny);
-  const int      algo = vpipes_pick_algo(nx, ny);
-  if (padded || algo == 0 || algo == 2 || algo == 3)
+  if (tiled)
     return vpipes_tiled_steps(z, nx, ny, p, c, A, B, u2, v2, s12, rain, water_depth, sediment, vel_u, vel_v, sc,
                               partials, padded || algo != 2, !padded && algo == 3 ? 2 : 1, s);
   VpStep         st;

@@ -24,10 +24,11 @@ struct VpFields;
 struct VpScalars;
 struct VpConst;
 VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p);
-/* initial state of copy A (depth, zero sediment and fluxes; z from z_in
- * where given) in rows of ld floats (0: nx), and V0, R */
+/* initial state of copy A (depth, with the first step's rain where
+ * first_rain is set; zero sediment and fluxes; z from z_in where given) in
+ * rows of ld floats (0: nx), and V0, R */
 int     vpipes_init(const VpFields &A, const float *rain, int nx, int ny, float init_depth, VpScalars *sc,
-                    double *partials, cudaStream_t s, const float *z_in = nullptr, int ld = 0);
+                    double *partials, cudaStream_t s, float first_rain, const float *z_in = nullptr, int ld = 0);
 /* device address of the solve's error word (bit 0: a tile's TMA loads
  * timed out and the tile was skipped) inside the scratch of vpipes_core */
 const unsigned *vpipes_error_word(const void *scratch_buf, int nx, int ny, bool padded);

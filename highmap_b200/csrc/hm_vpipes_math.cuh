@@ -38,8 +38,15 @@ __device__ __forceinline__ float fdiv_z(float a, float b)
 /* the reference's max / min as the oracle spells them: a > b ? a : b */
 __device__ __forceinline__ float rmax(float a, float b) { return a > b ? a : b; }
 __device__ __forceinline__ float rmin(float a, float b) { return a < b ? a : b; }
-/* a > b ? x : y */
-__device__ __forceinline__ float sel_gt(float a, float b, float x, float y) { return a > b ? x : y; }
+/* rmax(a, b) with NaN only in b and no zeros of opposite sign (or where
+ * the sign of a zero does not matter): one instruction instead of a compare
+ * and a select */
+__device__ __forceinline__ float rmaxn(float a, float b)
+{
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 
 __device__ __forceinline__ float hyp(float x, float y)
 {
@@ -71,9 +78,6 @@ struct VpConst
   float keep;        /* 1 - dt * evap_rate                              */
   float rps;         /* rain per step                                   */
   float fnx;         /* (float)nx, the slope scale of :156              */
-  float xhi, yhi;    /* nx - 0.5, ny - 0.5 (exact; 0 for grids too wide to
-                      * hold them exactly): sample points in [0.5, xhi) x
-                      * [0.5, yhi) need no mirror and no index clamps      */
 };
 
 /* Depth at the start of a step: the stored evaporated depth, plus the
@@ -116,10 +120,11 @@ __device__ __forceinline__ void flow_cell(const VpConst &c,
     qt = fdiv(qt, pl);
     qb = fdiv(qb, pl);
   }
-  T nl = rmax(zero, fadd(fl, ql));
-  T nr = rmax(zero, fadd(fr, qr));
-  T nt = rmax(zero, fadd(ft, qt));
-  T nb = rmax(zero, fadd(fb, qb));
+  /* (a flux is never -0, so neither is its sum with a product) */
+  T nl = rmaxn(zero, fadd(fl, ql));
+  T nr = rmaxn(zero, fadd(fr, qr));
+  T nt = rmaxn(zero, fadd(ft, qt));
+  T nb = rmaxn(zero, fadd(fb, qb));
   if (DIFFUSION)
   {
     const T c1 = bc<T>(c.c1);
@@ -138,8 +143,7 @@ __device__ __forceinline__ void flow_cell(const VpConst &c,
    * divisor is 1 */
   const bool wet = sum > bc<T>(1e-5f);
   T          kq = fdiv(num, wet ? fmul(sum, bc<T>(c.dt)) : bc<T>(1.f));
-  T          k = wet ? kq : zero;
-  k = rmin(rmax(k, zero), bc<T>(1.f));
+  T          k = wet ? __saturatef(kq) : zero; /* NaN clamps to 0, as k > 0 ? k : 0 does */
   fl = fmul(nl, k);
   fr = fmul(nr, k);
   ft = fmul(nt, k);
@@ -156,16 +160,15 @@ __device__ __forceinline__ void water_cell(const VpConst &c,
                                            T &d2, T &u, T &v)
 {
   T dv = fmul(bc<T>(c.dt), fsub(fsub(fsub(fsub(fadd(fadd(fadd(frw, ftn), fle), fbs), flc), frc), ftc), fbc));
-  d2 = rmax(bc<T>(0.f), fadd(d1c, PL_ONE ? dv : fdiv(dv, bc<T>(c.pl2))));
+  d2 = rmaxn(bc<T>(0.f), fadd(d1c, PL_ONE ? dv : fdiv(dv, bc<T>(c.pl2))));
   T un = fmul(bc<T>(0.5f), fsub(fadd(fsub(frw, flc), frc), fle));
   T vn = fmul(bc<T>(0.5f), fsub(fadd(fsub(ftn, fbc), ftc), fbs));
-  T dmean = rmax(bc<T>(c.vel_floor), d2);
+  T dmean = rmaxn(bc<T>(c.vel_floor), d2);
   u = fdiv(un, dmean);
   v = fdiv(vn, dmean);
 }
 
-/* Erosion / deposition for one cell from the old z and s around it; both
- * branches of :170-183 are formed and one is selected. */
+/* Erosion / deposition for one cell from the old z and s around it. */
 template <bool KEXP_ONE, class T>
 __device__ __forceinline__ void erosion_cell(const VpConst &c,
                                              T zc, T sc,
@@ -178,8 +181,8 @@ __device__ __forceinline__ void erosion_cell(const VpConst &c,
   T       dzx = fmul(half, fsub(fadd(fsub(ze, zw), se), sw));
   T       dzy = fmul(half, fsub(fadd(fsub(zs, zn), ss), sn));
   T       talus = hyp(dzx, dzy);
-  T       dzn = rmax(bc<T>(1e-3f), fmul(bc<T>(c.fnx), talus));
-  T       salpha = rmax(bc<T>(0.01f), fdiv(dzn, hyp(bc<T>(1.f), dzn)));
+  T       dzn = rmaxn(bc<T>(1e-3f), fmul(bc<T>(c.fnx), talus));
+  T       salpha = rmaxn(bc<T>(0.01f), fdiv(dzn, hyp(bc<T>(1.f), dzn)));
   T       speed = hyp(u, v);
   /* d2 is zero on dry cells (about 6 % of the cells after a few hundred
    * steps of the 4096^2 benchmark, in over 90 % of the warps) */
@@ -187,10 +190,12 @@ __device__ __forceinline__ void erosion_cell(const VpConst &c,
   T       discharge = fmul(depth, speed);
   T       pw = KEXP_ONE ? discharge : powr(discharge, c.k_exp);
   T       capa = fmul(fmul(bc<T>(c.k_capacity), pw), salpha);
-  T       ero = fmul(bc<T>(c.k_erode), fsub(capa, sc));
-  T       dep = fmul(bc<T>(c.k_depose), fsub(sc, capa));
-  z_out = sel_gt(capa, sc, fsub(zc, ero), fadd(zc, dep));
-  s_out = sel_gt(capa, sc, fadd(sc, ero), fsub(sc, dep));
+  /* erosion moves k_erode (capa - s) from z to s, deposition k_depose
+   * (s - capa) from s to z: the same sums with the sign of the difference
+   * in the product (rounding is symmetric) */
+  T m = fmul(capa > sc ? bc<T>(c.k_erode) : bc<T>(c.k_depose), fsub(capa, sc));
+  z_out = fsub(zc, m);
+  s_out = fadd(sc, m);
 }
 
 /* Mirror an unnormalised coordinate with period 2 * n (texel units):

@@ -153,7 +153,7 @@ __device__ __forceinline__ void tb_flux_g(const TbIo &io, const VpConst &c, int 
   auto         zz = [&](int a, int b) { return __ldg(z + tb_k(c, a, b)); };
   auto         dd = [&](int a, int b) {
     const size_t k = tb_k(c, a, b);
-    return tb_d1(c, io.rain, __ldg(d + k), k);
+    return __ldg(d + k);
   };
   const size_t k = (size_t)j * c.nx + i;
   fl = __ldg(io.in.fl + k);
@@ -187,7 +187,7 @@ __device__ __noinline__ float tb_s1_at(const TbIo io, const VpConst c, int i, in
   tb_flux_g<F>(io, c, i, jp, t0, t1, t2, fbs);
   const size_t k = (size_t)j * c.nx + i;
   float        d2, u, v;
-  tb_water<F>(c, io, tb_d1(c, io.rain, __ldg(io.in.d + k), k), fl, fr, ft, fb, frw, fle, ftn, fbs, d2, u, v);
+  tb_water<F>(c, io, __ldg(io.in.d + k), fl, fr, ft, fb, frw, fle, ftn, fbs, d2, u, v);
   const float *z = io.in.z;
   float        zo, so;
   tb_erosion<F>(c, io, __ldg(z + k), tb_sed_g(io, c, i, j), __ldg(z + tb_k(c, i - 1, j)), __ldg(z + tb_k(c, i + 1, j)),
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(TB_NT, 4) k_vp_tb2(TbIo io, VpConst c)
       const size_t k = (size_t)gy * nx + gx;
       const int    i = at(gx, gy);
       Z[i] = __ldg(io.in.z + k);
-      D[i] = tb_d1(c, io.rain, __ldg(io.in.d + k), k);
+      D[i] = __ldg(io.in.d + k); /* the start depth: the step before added its rain */
     }
     const TbRegion r1 = tb_region<TX, TY>(x0, y0, TB_H1, nx, ny);
     for (int e0 = tid; e0 < r1.cnt; e0 += TB_AB * TB_NT)
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(TB_NT, 4) k_vp_tb2(TbIo io, VpConst c)
       tb_erosion<F>(c, io, ZN[p.c], S[p.c], ZN[p.w], ZN[p.e], ZN[p.n], ZN[p.s], S[p.w], S[p.e], S[p.n], S[p.s], d2, u,
                  v, zo, so);
       io.out.z[k] = zo;
-      io.out.d[k] = fmul(d2, c.keep);
+      io.out.d[k] = io.last ? fmul(d2, c.keep) : tb_d1(c, io.rain, fmul(d2, c.keep), k);
       io.out.fl[k] = fl;
       io.out.fr[k] = fr;
       io.out.ft[k] = ft;

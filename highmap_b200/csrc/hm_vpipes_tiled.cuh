@@ -40,6 +40,8 @@
 #ifndef HM_VPIPES_TILED_CUH
 #define HM_VPIPES_TILED_CUH
 
+#include <type_traits>
+
 #include "hm_reduce.cuh"
 #include "hm_vpipes_fused.cuh"
 #include "hm_vpipes_math.cuh"
@@ -117,7 +119,13 @@ struct FweSmem
 };
 static_assert(sizeof(AdvStage) <= sizeof(float) * 4 * FT_H1 * FW, "advect-in staging fits the new-flux arrays");
 
-/* the step's grids: old state in, new state out, plus this step's s1, u, v */
+/* The step's grids: old state in, new state out, plus this step's s1, u, v.
+ * The stored depth is the evaporated depth (the result after the last
+ * step).  Without the volume top-up a step stores it with the next step's
+ * rain already added (the same two roundings), so the tiles stage the start
+ * depth itself: 10 instructions per cell fewer than a pass over the staged
+ * region.  With the top-up, which needs the sum over all cells first, the
+ * next step adds top-up and rain. */
 struct FweIo
 {
   VpState      in;
@@ -128,6 +136,7 @@ struct FweIo
   int          maintain, diffusion, pl_one, kexp_one;
   float       *u_out, *v_out; /* last step: velocity outputs (rows of c.ld), both or neither */
   int          vec;           /* even row stride and every output 8-byte aligned: pair stores */
+  int          last;          /* last step of the solve */
   int          flow_only;     /* flow_simulation step (FWE_FLOWONLY kernels) */
   int          stage16;       /* row stride a multiple of 4 and every staged grid 16-byte aligned: a tile whose
                                * boxes lie inside the grid may stage them in 16-byte copies */
@@ -154,13 +163,13 @@ struct AdvMaps
 constexpr unsigned FWE_TMA_BYTES = 4u * 40u * (2u * FT_H2 + 5u * FT_H1);
 constexpr unsigned FLOW_TMA_BYTES = 4u * 40u * (2u * FT_H2 + 4u * FT_H1);
 /* bytes the nine boxes of k_vp_step_tma deliver: group A (the previous
- * step's u, v and s1, and the stored depth), on which the advection and
- * the depth pass run while group B (z and the four old fluxes) is still
- * arriving */
-constexpr unsigned STEP_TMA_BYTES = 4u * 40u * (2u * FT_H2 + 6u * FT_H1 + FS_H);
-constexpr unsigned STEP_TMA_BYTES_A = 4u * 40u * (FT_H2 + 2u * FT_H1 + FS_H);
+ * step's u, v and s1), on which the advection runs while group B (z and the
+ * four old fluxes) is still arriving; the stored depth is in group A with
+ * the volume top-up, whose depth pass runs beside the advection, else in
+ * group B */
+constexpr unsigned STEP_TMA_BYTES_A = 4u * 40u * (2u * FT_H1 + FS_H);
 constexpr unsigned STEP_TMA_BYTES_B = 4u * 40u * (FT_H2 + 4u * FT_H1);
-static_assert(STEP_TMA_BYTES_A + STEP_TMA_BYTES_B == STEP_TMA_BYTES, "the two groups are the nine boxes");
+constexpr unsigned STEP_TMA_BYTES_D = 4u * 40u * FT_H2;
 
 /* cp.async staging: z, d on the halo-2 region; s and old fluxes on the
  * halo-1 region; loads clamped to the grid, so every raw neighbour read is
@@ -355,13 +364,14 @@ __device__ __forceinline__ bool fwe_stage_tma(const FweMaps &maps, int nx, int n
 }
 
 /* TMA staging of k_vp_step_tma in two groups on two barriers.  Group A:
- * the previous step's u and v (region 1), its s1 (rows y0-4 .. y0+19) and
- * the stored depth d (region 2), waited for here.  Group B: z (region 2)
- * and the old fluxes (region 1), waited for by fwe_wait_tma_step_b after
- * the advection and the depth pass have run on group A, so those overlap
- * its arrival.  Returns false, uniformly across the CTA, if group A did
+ * the previous step's u and v (region 1) and its s1 (rows y0-4 .. y0+19),
+ * waited for here.  Group B: z (region 2) and the old fluxes (region 1),
+ * waited for by fwe_wait_tma_step_b after the advection (and the depth
+ * pass) have run on group A, so those overlap its arrival.  The stored
+ * depth d (region 2) is in group A if D_FIRST.  Returns false, uniformly across the CTA, if group A did
  * not complete in time; group B's loads are then given their own windows
  * to land before the CTA leaves. */
+template <bool D_FIRST>
 __device__ __forceinline__ bool fwe_stage_tma_step(const FweMaps &maps, const AdvMaps &am, int x0, int y0,
                                                    FweSmem &sm, unsigned extra_tx)
 {
@@ -375,13 +385,14 @@ __device__ __forceinline__ bool fwe_stage_tma_step(const FweMaps &maps, const Ad
   __syncthreads();
   if (tid == 0)
   {
-    mbar_arrive_expect_tx(&sm.bar, STEP_TMA_BYTES_A + extra_tx);
+    mbar_arrive_expect_tx(&sm.bar, STEP_TMA_BYTES_A + (D_FIRST ? STEP_TMA_BYTES_D : 0u) + extra_tx);
     tma_load_2d(&sm.adv.u[0][0], &am.u, x0 - 4, y0 - 1, &sm.bar);
     tma_load_2d(&sm.adv.v[0][0], &am.v, x0 - 4, y0 - 1, &sm.bar);
     tma_load_2d(&sm.adv.s1[0][0], &am.s1, x0 - 4, y0 - 4, &sm.bar);
-    tma_load_2d(&sm.d[0][0], &maps.d, x0 - 4, y0 - 2, &sm.bar);
-    mbar_arrive_expect_tx(&sm.bar2, STEP_TMA_BYTES_B);
+    if (D_FIRST) tma_load_2d(&sm.d[0][0], &maps.d, x0 - 4, y0 - 2, &sm.bar);
+    mbar_arrive_expect_tx(&sm.bar2, STEP_TMA_BYTES_B + (D_FIRST ? 0u : STEP_TMA_BYTES_D));
     tma_load_2d(&sm.z[0][0], &maps.z, x0 - 4, y0 - 2, &sm.bar2);
+    if (!D_FIRST) tma_load_2d(&sm.d[0][0], &maps.d, x0 - 4, y0 - 2, &sm.bar2);
     tma_load_2d(&sm.fo[0][0][0], &maps.fl, x0 - 4, y0 - 1, &sm.bar2);
     tma_load_2d(&sm.fo[1][0][0], &maps.fr, x0 - 4, y0 - 1, &sm.bar2);
     tma_load_2d(&sm.fo[2][0][0], &maps.ft, x0 - 4, y0 - 1, &sm.bar2);
@@ -418,72 +429,58 @@ __device__ __forceinline__ bool fwe_wait_tma_step_b(int nx, int ny, int x0, int 
  * the staged s1 box (columns x0-4 .. x0+35, rows y0-4 .. y0+19) read shared
  * memory, the rest s1 in global memory.  INNER: region 1 lies inside the
  * grid, so no cell is clamped. */
+/* the lower-left texels whose four taps lie in the staged s1 box and in the
+ * grid: lo <= i < lo + n on each axis */
+struct AdvBox
+{
+  int      lo_x, lo_y;
+  unsigned n_x, n_y;
+};
+__device__ __forceinline__ AdvBox adv_box(int nx, int ny, int x0, int y0)
+{
+  AdvBox b;
+  b.lo_x = max(0, x0 - 4);
+  b.lo_y = max(0, y0 - 4);
+  /* (a grid side of 2^23 or more never takes the box: its indices would not
+   * be exact in a float) */
+  b.n_x = nx < (1 << 23) ? (unsigned)max(0, min(nx - 2, x0 + FW - 6) - b.lo_x + 1) : 0u;
+  b.n_y = ny < (1 << 23) ? (unsigned)max(0, min(ny - 2, y0 + FS_H - 6) - b.lo_y + 1) : 0u;
+  return b;
+}
+
 /* advected sediment of one region-1 cell: column gx, row gy of the grid
  * (clamped), at shared-memory row l and column cc */
-__device__ __forceinline__ void advect_cell(const VpConst &c, const float *__restrict__ s1g, int x0, int y0, int gx,
-                                            int gy, int l, int cc, FweSmem &sm)
+__device__ __forceinline__ void advect_cell(const VpConst &c, const float *__restrict__ s1g, const AdvBox &bx, int x0,
+                                            int y0, int gx, int gy, int l, int cc, FweSmem &sm)
 {
   const int   nx = c.nx, ny = c.ny, ld = c.ld;
   const float uu = sm.adv.u[gy - (y0 - 1)][gx - (x0 - 4)];
   const float vv = sm.adv.v[gy - (y0 - 1)][gx - (x0 - 4)];
   const float x = fsub((float)gx, fmul(c.dt, uu));
   const float y = fsub((float)gy, fmul(c.dt, vv));
-  if (x >= 0.5f && x < c.xhi && y >= 0.5f && y < c.yhi)
+  /* floor by adding 2^23 rounded down: 2^23 + floor(v) for v in [0, 2^23),
+   * whose integer is in the low bits (a quarter of the cost of two floors
+   * and two conversions, which share the 4-lane unit with the divisions);
+   * a negative, huge or NaN v gives an index outside the box */
+  const float xm = fsub(x, 0.5f), ym = fsub(y, 0.5f);
+  const float tx = __fadd_rd(xm, 8388608.f), ty = __fadd_rd(ym, 8388608.f);
+  const int   i0 = __float_as_int(tx) - 0x4b000000, j0 = __float_as_int(ty) - 0x4b000000;
+  if ((unsigned)(i0 - bx.lo_x) < bx.n_x && (unsigned)(j0 - bx.lo_y) < bx.n_y)
   {
-    /* The sample point lies inside the texel centres: the mirror of
-     * linear_tap returns the coordinate itself, floor(x - 0.5) lies in
-     * [0, nx - 2], so i0 needs no clamp and i1 = i0 + 1 (rows likewise).
-     * The same rounded operations as linear_tap, without the identities. */
-    Tap         tp;
-    const float xm = fsub(x, 0.5f), ym = fsub(y, 0.5f);
-    const float fx = floorf(xm), fy = floorf(ym);
-    tp.a = fsub(xm, fx);
-    tp.b = fsub(ym, fy);
-    tp.i0 = (int)fx;
-    tp.j0 = (int)fy;
-    tp.i1 = tp.i0 + 1;
-    tp.j1 = tp.j0 + 1;
-    const int bi = tp.i0 - (x0 - 4), bj = tp.j0 - (y0 - 4);
-    float     g00, g10, g01, g11;
-    if ((unsigned)bi < (unsigned)(FW - 1) && (unsigned)bj < (unsigned)(FS_H - 1))
-    {
-      const float *r = &sm.adv.s1[bj][bi];
-      g00 = r[0];
-      g10 = r[1];
-      g01 = r[FW];
-      g11 = r[FW + 1];
-    }
-    else
-    {
-      const float *r = s1g + (size_t)tp.j0 * ld + tp.i0;
-      g00 = __ldg(r);
-      g10 = __ldg(r + 1);
-      g01 = __ldg(r + ld);
-      g11 = __ldg(r + ld + 1);
-    }
-    sm.s[l][cc] = blend(tp, g00, g10, g01, g11);
+    /* The four texels lie in the staged box and i0 in [0, nx - 2]: the
+     * mirror of linear_tap returns the coordinate itself and nothing is
+     * clamped.  The same rounded operations without the identities. */
+    Tap t;
+    t.a = fsub(xm, fsub(tx, 8388608.f));
+    t.b = fsub(ym, fsub(ty, 8388608.f));
+    const float *r = &sm.adv.s1[j0 - (y0 - 4)][i0 - (x0 - 4)];
+    sm.s[l][cc] = blend(t, r[0], r[1], r[FW], r[FW + 1]);
     return;
   }
-  const Tap t = linear_tap(x, y, nx, ny);
-  const int bi0 = t.i0 - (x0 - 4), bi1 = t.i1 - (x0 - 4);
-  const int   bj0 = t.j0 - (y0 - 4), bj1 = t.j1 - (y0 - 4);
-  float       g00, g10, g01, g11;
-  if (bi0 >= 0 && bi1 < FW && bj0 >= 0 && bj1 < FS_H)
-  {
-    g00 = sm.adv.s1[bj0][bi0];
-    g10 = sm.adv.s1[bj0][bi1];
-    g01 = sm.adv.s1[bj1][bi0];
-    g11 = sm.adv.s1[bj1][bi1];
-  }
-  else
-  {
-    const size_t r0 = (size_t)t.j0 * ld, r1 = (size_t)t.j1 * ld;
-    g00 = __ldg(s1g + r0 + t.i0);
-    g10 = __ldg(s1g + r0 + t.i1);
-    g01 = __ldg(s1g + r1 + t.i0);
-    g11 = __ldg(s1g + r1 + t.i1);
-  }
-  sm.s[l][cc] = blend(t, g00, g10, g01, g11);
+  const Tap    t = linear_tap(x, y, nx, ny);
+  const size_t r0 = (size_t)t.j0 * ld, r1 = (size_t)t.j1 * ld;
+  sm.s[l][cc] = blend(t, __ldg(s1g + r0 + t.i0), __ldg(s1g + r0 + t.i1), __ldg(s1g + r1 + t.i0),
+                      __ldg(s1g + r1 + t.i1));
 }
 
 /* rows of region 1 one thread advects */
@@ -501,14 +498,15 @@ __device__ __forceinline__ void advect_region1(const VpConst &c, const float *__
   const int t = threadIdx.x;
   if (t >= FT_W1 * (FT_H1 / ADV_ROWS)) return;
   const int cc = 3 + t % FT_W1, l0 = ADV_ROWS * (t / FT_W1);
-  int       gx = x0 - 4 + cc;
+  const AdvBox bx = adv_box(c.nx, c.ny, x0, y0);
+  int          gx = x0 - 4 + cc;
   if (!INNER) gx = clampi(gx, 0, c.nx - 1);
 #pragma unroll
   for (int r = 0; r < ADV_ROWS; r++)
   {
     int gy = y0 - 1 + l0 + r;
     if (!INNER) gy = clampi(gy, 0, c.ny - 1);
-    advect_cell(c, s1g, x0, y0, gx, gy, l0 + r, cc, sm);
+    advect_cell(c, s1g, bx, x0, y0, gx, gy, l0 + r, cc, sm);
   }
 }
 
@@ -568,9 +566,9 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
   const bool     pl_one = GEN ? io.pl_one != 0 : true;
   const bool     kexp_one = GEN ? io.kexp_one != 0 : true;
 
-  /* stored depth -> depth at the start of the step, region 2 (columns
-   * x0-2 .. x0+33 = smem 2 .. 37), 18 pairs per row */
-  for (int e = tid; e < 18 * FT_H2; e += FT_NT)
+  /* with the top-up: stored depth -> depth at the start of the step, region
+   * 2 (columns x0-2 .. x0+33 = smem 2 .. 37), 18 pairs per row */
+  for (int e = MAINTAIN ? tid : 18 * FT_H2; e < 18 * FT_H2; e += FT_NT)
   {
     const int q = e / 18, cc = 2 + 2 * (e - q * 18);
     float2    dd = lds2(&sm.d[q][cc]);
@@ -593,7 +591,9 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
     }
     sts2(&sm.d[q][cc], dd.x, dd.y);
   }
-  __syncthreads();
+  /* the staged (and advected) fields are complete; mid() has a barrier of
+   * its own when it waits for something */
+  if (MAINTAIN || std::is_same<Mid, NoMid>::value) __syncthreads();
 
   double part = 0.0;
   if (mid())
@@ -693,7 +693,20 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
       }
       else
       {
-        const float dea = fmul(d2a, c.keep), deb = fmul(d2b, c.keep);
+        float dea = fmul(d2a, c.keep), deb = fmul(d2b, c.keep);
+        if (!MAINTAIN && rain_step && !io.last)
+        {
+          /* the next step's rain */
+          float r0 = 1.f, r1 = 1.f;
+          if (rain_map)
+          {
+            const float *r = io.rain + (size_t)gy * nx + gx;
+            r0 = __ldg(r);
+            if (second) r1 = __ldg(r + 1);
+          }
+          dea = fadd(dea, fmul(c.rps, r0));
+          deb = fadd(deb, fmul(c.rps, r1));
+        }
         /* what the water pass produced, stored before the erosion arithmetic
          * so its registers are free there (the stores go through generic
          * pointers, so the compiler keeps them after the shared-memory loads
@@ -829,7 +842,7 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
 {
   __shared__ FweSmem sm;
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
-  if (!fwe_stage_tma_step(maps, am, x0, y0, sm, io.tma_extra_tx))
+  if (!fwe_stage_tma_step<MAINTAIN>(maps, am, x0, y0, sm, io.tma_extra_tx))
   {
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
     if (MAINTAIN)
@@ -886,6 +899,7 @@ struct TbIo
   float       *s1, *u, *v;                /* step t+1's eroded sediment and velocity      */
   float       *u_out, *v_out;             /* velocity outputs when t+1 is the last step, nullable */
   int          diffusion, pl_one, kexp_one;
+  int          last;                      /* t+1 is the last step: out.d without the next step's rain */
 };
 int launch_vp_tb2(const TbIo &io, const VpConst &c, cudaStream_t s);
 
