@@ -13,6 +13,7 @@
  */
 #include <cuda_runtime.h>
 
+#include "hm_chain.cuh"
 #include "hm_internal.h"
 #include "hm_thermal.h"
 
@@ -24,9 +25,10 @@ namespace
 
 /* sediment of the previous layer (from the settled grid, or 0 on the
  * first), plus one layer; the grid to settle = terrain + sediment */
-__global__ void k_dep_layer(const float *__restrict__ z, float *__restrict__ smap, float *__restrict__ ztot,
-                            float step, int first, size_t n)
+__global__ void k_dep_layer(const float *__restrict__ z, float *__restrict__ smap, float *ztot, float step, int first,
+                            size_t n)
 {
+  chain_wait();
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
   {
     float s = 0.f;
@@ -43,9 +45,11 @@ __global__ void k_dep_layer(const float *__restrict__ z, float *__restrict__ sma
 
 /* last layer's sediment; z = z + sediment, blended with the input where a
  * mask is given (lerp, math.cpp:183-195) */
-__global__ void k_dep_final(float *__restrict__ z, const float *__restrict__ ztot, const float *__restrict__ mask,
+__global__ void k_dep_final(float *__restrict__ z, const float *ztot, const float *__restrict__ mask,
                             float *__restrict__ depo, int settled, size_t n)
 {
+  chain_wait();
+  ztot = produced(ztot);
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
   {
     float s = 0.f;
@@ -84,13 +88,13 @@ int deposition_core(int device, float *z, int nx, int ny, const float *talus, fl
   const float step = max_deposition / (float)iterations;
   for (int it = 0; it < iterations; it++)
   {
-    k_dep_layer<<<592, 256, 0, s>>>(z, smap, ztot, step, it == 0, n);
+    chain_launch(it > 0, k_dep_layer, dim3(592), dim3(256), s, z, smap, ztot, step, it == 0 ? 1 : 0, n);
     HM_LAUNCH_CHECK("k_dep_layer");
     int rc = thermal_core(device, ztot, nx, ny, talus, 0.f, thermal_subiterations, nullptr, nullptr, nullptr, nullptr,
-                          tws, s);
+                          tws, s, false, true);
     if (rc) return rc;
   }
-  k_dep_final<<<592, 256, 0, s>>>(z, ztot, mask, depo, iterations > 0, n);
+  chain_launch(iterations > 0, k_dep_final, dim3(592), dim3(256), s, z, ztot, mask, depo, iterations > 0 ? 1 : 0, n);
   HM_LAUNCH_CHECK("k_dep_final");
   return HM_OK;
 }

@@ -168,8 +168,8 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
     io.in = VpState{cur->z, cur->d, cur->s, cur->fl, cur->fr, cur->ft, cur->fb};
     io.out = VpStateOut{nxt->z, nxt->d, nxt->s, nxt->fl, nxt->fr, nxt->ft, nxt->fb, nullptr, nullptr};
     io.parity = it & 1;
-    const int rc = tma ? launch_fwe_tma(io, maps[cur == &A ? 0 : 1], c, sc, nullptr, g1, s)
-                       : launch_fwe_cp_async(io, c, sc, nullptr, g1, s);
+    const int rc = tma ? launch_fwe_tma(io, maps[cur == &A ? 0 : 1], c, sc, nullptr, g1, s, it > 0)
+                       : launch_fwe_cp_async(io, c, sc, nullptr, g1, s, it > 0);
     if (rc) return rc;
     VpFields *t = cur;
     cur = nxt;

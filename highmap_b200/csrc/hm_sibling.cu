@@ -134,9 +134,11 @@ constexpr int SS_NT = 256, SS2_NT = 128, SS_H = 16; /* as the thermal sweeps */
 
 template <int RULE>
 __global__ void __launch_bounds__(SS_NT)
-    k_sibling_sweep(const float *__restrict__ a, float *__restrict__ b, int nx, int ny, const float *__restrict__ talus,
+    k_sibling_sweep(const float *a, float *__restrict__ b, int nx, int ny, const float *__restrict__ talus,
                     const float *__restrict__ zmax, float intensity)
 {
+  chain_wait();
+  a = produced(a);
   const int wx = (blockIdx.x * (SS_NT / 32) + (threadIdx.x >> 5)) * 32;
   if (wx >= nx) return; /* the whole warp */
   const int y0 = blockIdx.y * SS_H;
@@ -146,9 +148,11 @@ __global__ void __launch_bounds__(SS_NT)
 
 template <int RULE>
 __global__ void __launch_bounds__(SS2_NT)
-    k_sibling_sweep2(const float *__restrict__ a, float *__restrict__ b, int nx, int ny,
+    k_sibling_sweep2(const float *a, float *__restrict__ b, int nx, int ny,
                      const float *__restrict__ talus, const float *__restrict__ zmax, float intensity)
 {
+  chain_wait();
+  a = produced(a);
   const int wx = (blockIdx.x * (SS2_NT / 32) + (threadIdx.x >> 5)) * 64;
   if (wx >= nx) return; /* the whole warp */
   const int y0 = blockIdx.y * SS_H;
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(SS2_NT)
 /* T steps of a 3 x 3 rule per launch (hm_thermal_block.cuh) */
 template <int RULE, int ROWS, bool VEC>
 __global__ void __launch_bounds__(TBK_NT)
-    k_sibling_block(const float *__restrict__ a, float *__restrict__ b, int nx, int ny, const float *__restrict__ talus,
+    k_sibling_block(const float *a, float *__restrict__ b, int nx, int ny, const float *__restrict__ talus,
                     const float *__restrict__ zmax, float intensity, int T)
 {
   thermal_block<RULE != HM_RIB, SiblingRule<RULE>, ROWS, VEC>(a, b, nx, ny, talus, 0.f, zmax, T, blockIdx.x,
@@ -168,18 +172,19 @@ __global__ void __launch_bounds__(TBK_NT)
 
 template <int RULE>
 void launch_sibling_block(const float *a, float *b, int nx, int ny, const float *talus, const float *zmax,
-                          float intensity, int T, int rows, bool vec, cudaStream_t s)
+                          float intensity, int T, int rows, bool vec, cudaStream_t s, bool chained)
 {
   auto k = rows == 1 ? (vec ? k_sibling_block<RULE, 1, true> : k_sibling_block<RULE, 1, false>)
                      : (vec ? k_sibling_block<RULE, 2, true> : k_sibling_block<RULE, 2, false>);
-  k<<<tbk_grid(nx, ny, BlockPlan{T, rows, 1}), TBK_NT, 0, s>>>(a, b, nx, ny, talus, zmax, intensity, T);
+  chain_launch(chained, k, tbk_grid(nx, ny, BlockPlan{T, rows, 1}), dim3(TBK_NT), s, a, b, nx, ny, talus, zmax,
+               intensity, T);
 }
 
 /* thermal_olsen and thermal_flatten: radius-2 reads, a shared-memory tile
  * per CTA (intensity: flatten's sigma_inf, p1 its sigma_sup) */
 template <int RULE>
 __global__ void __launch_bounds__(SB_TX *SB_TY)
-    k_sibling_step(const float *__restrict__ a,
+    k_sibling_step(const float *a,
                    float *__restrict__ b,
                    int nx,
                    int ny,
@@ -189,13 +194,15 @@ __global__ void __launch_bounds__(SB_TX *SB_TY)
                    float p1)
 {
   __shared__ float t[SB_TY + 2 * SB_H][SB_TX + 2 * SB_H];
+  chain_wait();
+  a = produced(a);
   const int x0 = blockIdx.x * SB_TX, y0 = blockIdx.y * SB_TY;
   const int tid = threadIdx.y * SB_TX + threadIdx.x;
   for (int e = tid; e < (SB_TY + 2 * SB_H) * (SB_TX + 2 * SB_H); e += SB_TX * SB_TY)
   {
     const int ly = e / (SB_TX + 2 * SB_H), lx = e - ly * (SB_TX + 2 * SB_H);
     const int gx = min(max(x0 - SB_H + lx, 0), nx - 1), gy = min(max(y0 - SB_H + ly, 0), ny - 1);
-    t[ly][lx] = __ldg(a + (size_t)gy * nx + gx);
+    t[ly][lx] = a[(size_t)gy * nx + gx];
   }
   __syncthreads();
   /* flatten: the steepest descent of every cell of the tile and its 1-cell
@@ -239,7 +246,7 @@ __global__ void __launch_bounds__(SB_TX *SB_TY)
     if (!(i >= bw && i < nx - bw && j >= bw && j < ny - bw))
     {
       const int ci = min(max(i, bw), nx - bw - 1), cj = min(max(j, bw), ny - bw - 1);
-      b[idx] = __ldg(a + (size_t)cj * nx + ci);
+      b[idx] = a[(size_t)cj * nx + ci];
       return;
     }
     const float    c2 = 1.414213562f;
@@ -287,7 +294,7 @@ __global__ void __launch_bounds__(SB_TX *SB_TY)
     if (!(i >= bw && i < nx - bw && j >= bw && j < ny - bw))
     {
       const int ci = min(max(i, bw), nx - bw - 1), cj = min(max(j, bw), ny - bw - 1);
-      b[idx] = __ldg(a + (size_t)cj * nx + ci);
+      b[idx] = a[(size_t)cj * nx + ci];
       return;
     }
     /* thermal_flatten.cl visits the neighbours from a rotating start
@@ -404,9 +411,11 @@ int sibling_core(int device, int rule, float *z, int nx, int ny, const float *ta
     float    *dst = buf[l & 1];
     const int T = plan.T == 1 ? 1 : block_steps(plan, iterations, l);
 #define HM_SIB_SWEEP(R)                                                                                                \
-  if (plan.T > 1) launch_sibling_block<R>(src, dst, nx, ny, talus, zmax, intensity, T, plan.rows, pairs, s);            \
-  else if (pairs) k_sibling_sweep2<R><<<g2, SS2_NT, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity);                  \
-  else k_sibling_sweep<R><<<g1, SS_NT, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity);
+  if (plan.T > 1)                                                                                                      \
+    launch_sibling_block<R>(src, dst, nx, ny, talus, zmax, intensity, T, plan.rows, pairs, s, l > 0);                  \
+  else                                                                                                                 \
+    chain_launch(l > 0, pairs ? k_sibling_sweep2<R> : k_sibling_sweep<R>, pairs ? g2 : g1,                             \
+                 dim3(pairs ? SS2_NT : SS_NT), s, src, dst, nx, ny, talus, zmax, intensity);
     switch (rule)
     {
     case HM_RIDGE: HM_SIB_SWEEP(HM_RIDGE) break;
@@ -414,8 +423,10 @@ int sibling_core(int device, int rule, float *z, int nx, int ny, const float *ta
     case HM_SCHOTT: HM_SIB_SWEEP(HM_SCHOTT) break;
     case HM_INFLATE: HM_SIB_SWEEP(HM_INFLATE) break;
     case HM_RIB: HM_SIB_SWEEP(HM_RIB) break;
-    case HM_FLATTEN: k_sibling_step<HM_FLATTEN><<<grid, block, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity, p1); break;
-    default: k_sibling_step<HM_OLSEN><<<grid, block, 0, s>>>(src, dst, nx, ny, talus, zmax, intensity, p1);
+    case HM_FLATTEN: 
+      chain_launch(l > 0, k_sibling_step<HM_FLATTEN>, grid, block, s, src, dst, nx, ny, talus, zmax, intensity, p1);
+      break;
+    default: chain_launch(l > 0, k_sibling_step<HM_OLSEN>, grid, block, s, src, dst, nx, ny, talus, zmax, intensity, p1);
     }
 #undef HM_SIB_SWEEP
     HM_LAUNCH_CHECK("k_sibling_step");
@@ -423,7 +434,7 @@ int sibling_core(int device, int rule, float *z, int nx, int ny, const float *ta
   }
   float *dep = want_depo ? depo : nullptr;
   if (rule != HM_RIB && nx >= 4 && ny >= 4 && (src != z || !keep_z))
-    return thermal_out(src, z, nx, ny, dep, mask, s, rule != HM_SCREE);
+    return thermal_out(src, z, nx, ny, dep, mask, s, rule != HM_SCREE, plan.launches > 0);
   /* in place: a deeper border, a grid narrower than 4, or no steps */
   const size_t bytes = (size_t)nx * ny * sizeof(float);
   float       *z0 = nullptr;

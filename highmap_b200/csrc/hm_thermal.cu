@@ -56,7 +56,7 @@ constexpr int SW_H = 16;   /* output rows per CTA (a multiple of SW_P)      */
  * (hm_thermal_sweep.cuh). */
 template <bool TMAP, int BED>
 __global__ void __launch_bounds__(SW_NT)
-    k_thermal_sweep(const float *__restrict__ a,
+    k_thermal_sweep(const float *a,
                     float *__restrict__ b,
                     int nx,
                     int ny,
@@ -65,6 +65,8 @@ __global__ void __launch_bounds__(SW_NT)
                     const float *__restrict__ bedrock,
                     int first)
 {
+  chain_wait();
+  a = produced(a);
   const int wx = (blockIdx.x * (SW_NT / 32) + (threadIdx.x >> 5)) * 32;
   if (wx >= nx) return; /* the whole warp: no CTA barrier in this kernel */
   const int y0 = blockIdx.y * SW_H;
@@ -77,7 +79,7 @@ constexpr int S2_NT = 128; /* 4 warps; a warp owns 64 columns */
 
 template <bool TMAP, int BED>
 __global__ void __launch_bounds__(S2_NT)
-    k_thermal_sweep2(const float *__restrict__ a,
+    k_thermal_sweep2(const float *a,
                      float *__restrict__ b,
                      int nx,
                      int ny,
@@ -86,6 +88,8 @@ __global__ void __launch_bounds__(S2_NT)
                      const float *__restrict__ bedrock,
                      int first)
 {
+  chain_wait();
+  a = produced(a);
   const int wx = (blockIdx.x * (S2_NT / 32) + (threadIdx.x >> 5)) * 64;
   if (wx >= nx) return; /* the whole warp: no CTA barrier in this kernel */
   const int y0 = blockIdx.y * SW_H;
@@ -98,7 +102,7 @@ __global__ void __launch_bounds__(S2_NT)
 
 template <bool TMAP, int BED, int ROWS, bool VEC>
 __global__ void __launch_bounds__(TBK_NT)
-    k_thermal_block(const float *__restrict__ a,
+    k_thermal_block(const float *a,
                     float *__restrict__ b,
                     int nx,
                     int ny,
@@ -190,13 +194,13 @@ __global__ void k_thermal_final(float *__restrict__ z,
  * where every border cell is a function of interior cells alone: columns
  * from the two inward ones of their row, then rows from the two inward
  * rows (whose end cells are the column pass's). */
-__device__ __forceinline__ float bordered_row(const float *__restrict__ r, int i, int nx)
+__device__ __forceinline__ float bordered_row(const float *r, int i, int nx)
 {
   if (i == 0) return __fsub_rn(__fmul_rn(2.f, r[1]), r[2]);
   if (i == nx - 1) return __fsub_rn(__fmul_rn(2.f, r[nx - 2]), r[nx - 3]);
   return r[i];
 }
-__device__ __forceinline__ float bordered(const float *__restrict__ s, int i, int j, int nx, int ny)
+__device__ __forceinline__ float bordered(const float *s, int i, int j, int nx, int ny)
 {
   if (j == 0 || j == ny - 1)
   {
@@ -211,6 +215,7 @@ __device__ __forceinline__ float bordered(const float *__restrict__ s, int i, in
 __global__ void __launch_bounds__(256) k_border(float *z, int nx, int ny)
 {
   const long long n = 2ll * nx + 2ll * (ny - 2);
+  chain_wait();
   for (long long k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
   {
     int i, j;
@@ -233,10 +238,12 @@ __global__ void __launch_bounds__(256) k_border(float *z, int nx, int ny)
  * map against the input heights z still holds, mask blend; 256 cells of a
  * row per CTA and turn. */
 __global__ void __launch_bounds__(256)
-    k_thermal_out(const float *__restrict__ s, float *__restrict__ z, float *__restrict__ depo,
+    k_thermal_out(const float *s, float *__restrict__ z, float *__restrict__ depo,
                   const float *__restrict__ mask, int nx, int ny, int depo_abs)
 {
   const int i = blockIdx.x * 256 + threadIdx.x;
+  chain_wait();
+  s = produced(s);
   if (i >= nx) return;
   for (int j = blockIdx.y; j < ny; j += gridDim.y)
   {
@@ -289,37 +296,37 @@ static int kernel_bed_mode(const float *bed, int bed_mode, bool auto_bed)
  * access (even nx, 8-byte aligned grids), else the one-column sweep */
 template <bool TMAP, int BED>
 static void launch_step(const float *a, float *b, int nx, int ny, const float *talus, float tv,
-                        const float *bed, int first, cudaStream_t s)
+                        const float *bed, int first, cudaStream_t s, bool chained)
 {
   auto al8 = [](const void *p) { return ((uintptr_t)p & 7u) == 0; };
   if (nx % 2 == 0 && al8(a) && al8(b) && (!TMAP || al8(talus)) && (BED == BED_NONE || al8(bed)))
   {
     dim3 grid((nx + 2 * S2_NT - 1) / (2 * S2_NT), (ny + SW_H - 1) / SW_H);
-    k_thermal_sweep2<TMAP, BED><<<grid, S2_NT, 0, s>>>(a, b, nx, ny, talus, tv, bed, first);
+    chain_launch(chained, k_thermal_sweep2<TMAP, BED>, grid, dim3(S2_NT), s, a, b, nx, ny, talus, tv, bed, first);
     return;
   }
   dim3 grid((nx + SW_NT - 1) / SW_NT, (ny + SW_H - 1) / SW_H);
-  k_thermal_sweep<TMAP, BED><<<grid, SW_NT, 0, s>>>(a, b, nx, ny, talus, tv, bed, first);
+  chain_launch(chained, k_thermal_sweep<TMAP, BED>, grid, dim3(SW_NT), s, a, b, nx, ny, talus, tv, bed, first);
 }
 
 template <bool TMAP>
 static void step_dispatch_t(const float *a, float *b, int nx, int ny, const float *talus, float tv,
-                            const float *bed, int mode, int first, cudaStream_t s)
+                            const float *bed, int mode, int first, cudaStream_t s, bool chained)
 {
   switch (mode)
   {
-  case BED_NONE: launch_step<TMAP, BED_NONE>(a, b, nx, ny, talus, tv, bed, first, s); break;
-  case BED_INTENDED: launch_step<TMAP, BED_INTENDED>(a, b, nx, ny, talus, tv, bed, first, s); break;
-  case BED_LITERAL: launch_step<TMAP, BED_LITERAL>(a, b, nx, ny, talus, tv, bed, first, s); break;
-  default: launch_step<TMAP, BED_AUTO>(a, b, nx, ny, talus, tv, bed, first, s); break;
+  case BED_NONE: launch_step<TMAP, BED_NONE>(a, b, nx, ny, talus, tv, bed, first, s, chained); break;
+  case BED_INTENDED: launch_step<TMAP, BED_INTENDED>(a, b, nx, ny, talus, tv, bed, first, s, chained); break;
+  case BED_LITERAL: launch_step<TMAP, BED_LITERAL>(a, b, nx, ny, talus, tv, bed, first, s, chained); break;
+  default: launch_step<TMAP, BED_AUTO>(a, b, nx, ny, talus, tv, bed, first, s, chained); break;
   }
 }
 
 static void step_dispatch(const float *a, float *b, int nx, int ny, const float *talus, float tv,
-                          const float *bed, int mode, int first, cudaStream_t s)
+                          const float *bed, int mode, int first, cudaStream_t s, bool chained)
 {
-  if (talus) step_dispatch_t<true>(a, b, nx, ny, talus, tv, bed, mode, first, s);
-  else step_dispatch_t<false>(a, b, nx, ny, talus, tv, bed, mode, first, s);
+  if (talus) step_dispatch_t<true>(a, b, nx, ny, talus, tv, bed, mode, first, s, chained);
+  else step_dispatch_t<false>(a, b, nx, ny, talus, tv, bed, mode, first, s, chained);
 }
 
 /* post-processing of a finished thermal solve (z holds the last step):
@@ -348,51 +355,52 @@ int thermal_finish(int device, float *z, int nx, int ny, const float *z0, float 
 }
 
 int thermal_out(const float *src, float *z, int nx, int ny, float *depo, const float *mask, cudaStream_t s,
-                bool depo_abs)
+                bool depo_abs, bool chained)
 {
   if (src == z && !depo && !mask && nx >= 4 && ny >= 4)
   {
     const long long n = 2ll * nx + 2ll * (ny - 2);
-    k_border<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(z, nx, ny);
+    chain_launch(chained, k_border, dim3((unsigned)((n + 255) / 256)), dim3(256), s, z, nx, ny);
     HM_LAUNCH_CHECK("k_border");
     return HM_OK;
   }
   const int gx = (nx + 255) / 256;
-  k_thermal_out<<<dim3(gx, ny < 32768 ? ny : 32768), 256, 0, s>>>(src, z, depo, mask, nx, ny, depo_abs ? 1 : 0);
+  chain_launch(chained, k_thermal_out, dim3(gx, ny < 32768 ? ny : 32768), dim3(256), s, src, z, depo, mask, nx, ny,
+               depo_abs ? 1 : 0);
   HM_LAUNCH_CHECK("k_thermal_out");
   return HM_OK;
 }
 
 template <bool TMAP, int BED>
 static void launch_block(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
-                         int T, int rows, int first, cudaStream_t s)
+                         int T, int rows, int first, cudaStream_t s, bool chained)
 {
   auto       al8 = [](const void *p) { return ((uintptr_t)p & 7u) == 0; };
   const bool vec = nx % 2 == 0 && al8(a) && al8(b) && (!TMAP || al8(talus)) && (BED == BED_NONE || al8(bed));
   const dim3 g = tbk_grid(nx, ny, BlockPlan{T, rows, 1});
   auto       k = rows == 1 ? (vec ? k_thermal_block<TMAP, BED, 1, true> : k_thermal_block<TMAP, BED, 1, false>)
                            : (vec ? k_thermal_block<TMAP, BED, 2, true> : k_thermal_block<TMAP, BED, 2, false>);
-  k<<<g, TBK_NT, 0, s>>>(a, b, nx, ny, talus, tv, bed, T, first);
+  chain_launch(chained, k, g, dim3(TBK_NT), s, a, b, nx, ny, talus, tv, bed, T, first);
 }
 
 template <bool TMAP>
 static void block_dispatch_t(const float *a, float *b, int nx, int ny, const float *talus, float tv,
-                             const float *bed, int mode, int T, int rows, int first, cudaStream_t s)
+                             const float *bed, int mode, int T, int rows, int first, cudaStream_t s, bool chained)
 {
   switch (mode)
   {
-  case BED_NONE: launch_block<TMAP, BED_NONE>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
-  case BED_INTENDED: launch_block<TMAP, BED_INTENDED>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
-  case BED_LITERAL: launch_block<TMAP, BED_LITERAL>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
-  default: launch_block<TMAP, BED_AUTO>(a, b, nx, ny, talus, tv, bed, T, rows, first, s); break;
+  case BED_NONE: launch_block<TMAP, BED_NONE>(a, b, nx, ny, talus, tv, bed, T, rows, first, s, chained); break;
+  case BED_INTENDED: launch_block<TMAP, BED_INTENDED>(a, b, nx, ny, talus, tv, bed, T, rows, first, s, chained); break;
+  case BED_LITERAL: launch_block<TMAP, BED_LITERAL>(a, b, nx, ny, talus, tv, bed, T, rows, first, s, chained); break;
+  default: launch_block<TMAP, BED_AUTO>(a, b, nx, ny, talus, tv, bed, T, rows, first, s, chained); break;
   }
 }
 
 static void block_dispatch(const float *a, float *b, int nx, int ny, const float *talus, float tv, const float *bed,
-                           int mode, int T, int rows, int first, cudaStream_t s)
+                           int mode, int T, int rows, int first, cudaStream_t s, bool chained)
 {
-  if (talus) block_dispatch_t<true>(a, b, nx, ny, talus, tv, bed, mode, T, rows, first, s);
-  else block_dispatch_t<false>(a, b, nx, ny, talus, tv, bed, mode, T, rows, first, s);
+  if (talus) block_dispatch_t<true>(a, b, nx, ny, talus, tv, bed, mode, T, rows, first, s, chained);
+  else block_dispatch_t<false>(a, b, nx, ny, talus, tv, bed, mode, T, rows, first, s, chained);
 }
 
 static int g_tb_rows = 0; /* tile rows of the blocked kernel (hm_thermal_set_launch); 0 = built-in */
@@ -429,7 +437,8 @@ int thermal_core(int device,
                  const hm_thermal_options *opts,
                  float *scratch_buf,
                  cudaStream_t s,
-                 bool auto_bed)
+                 bool auto_bed,
+                 bool chained)
 {
   hm_thermal_options o;
   hm_thermal_default_options(&o);
@@ -463,13 +472,13 @@ int thermal_core(int device,
     float *dst = buf[l & 1];
     if (plan.T == 1)
     {
-      step_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, l == 0, s);
+      step_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, l == 0, s, chained || l > 0);
       HM_LAUNCH_CHECK("k_thermal_sweep");
     }
     else
     {
       block_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, block_steps(plan, iterations, l), plan.rows,
-                     l == 0, s);
+                     l == 0, s, chained || l > 0);
       HM_LAUNCH_CHECK("k_thermal_block");
     }
     src = dst;
@@ -488,7 +497,7 @@ int thermal_core(int device,
     if (src != z) HM_CUDA_TRY(cudaMemcpyAsync(z, src, bytes, cudaMemcpyDeviceToDevice, s));
     return thermal_finish(device, z, nx, ny, z0, depo, mask, s);
   }
-  return thermal_out(src, z, nx, ny, depo, mask, s, false);
+  return thermal_out(src, z, nx, ny, depo, mask, s, false, chained || plan.launches > 0);
 }
 
 } // namespace hm

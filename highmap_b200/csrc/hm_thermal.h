@@ -13,10 +13,12 @@ int    thermal_check_args(const float *z, int nx, int ny, int iterations, const 
  * the input heights to the end (deposition map, mask, auto-bedrock) */
 size_t thermal_scratch_floats(int nx, int ny, bool need_z0);
 /* Device pointers; ordered on s.  talus NULL selects talus_value.
- * auto_bed: thermal_auto_bedrock (bedrock must be NULL; two grids). */
+ * auto_bed: thermal_auto_bedrock (bedrock must be NULL; two grids).
+ * chained: the launch before on s is one of a chain (hm_chain.cuh) that
+ * does not write talus or bedrock. */
 int    thermal_core(int device, float *z, int nx, int ny, const float *talus, float talus_value, int iterations,
                     const float *bedrock, float *depo, const float *mask, const hm_thermal_options *opts,
-                    float *scratch_buf, cudaStream_t s, bool auto_bed = false);
+                    float *scratch_buf, cudaStream_t s, bool auto_bed = false, bool chained = false);
 /* border extrapolation, deposition map and mask blend after the steps */
 int    thermal_finish(int device, float *z, int nx, int ny, const float *z0, float *depo, const float *mask,
                       cudaStream_t s, bool depo_abs = false, int nbuffer = 1);
@@ -24,7 +26,7 @@ int    thermal_finish(int device, float *z, int nx, int ny, const float *z0, flo
  * heights (src == z: the border alone, in place); grids of at least 4 x 4,
  * one border cell deep */
 int    thermal_out(const float *src, float *z, int nx, int ny, float *depo, const float *mask, cudaStream_t s,
-                   bool depo_abs);
+                   bool depo_abs, bool chained);
 /* sediment_deposition (hm_deposition.cu): device pointers, ordered on s */
 size_t deposition_scratch_floats(int nx, int ny);
 int    deposition_core(int device, float *z, int nx, int ny, const float *talus, float max_deposition,

@@ -29,6 +29,7 @@
 
 #include <cstdint>
 
+#include "hm_chain.cuh"
 #include "hm_thermal_sweep.cuh"
 
 namespace hm
@@ -54,16 +55,23 @@ __device__ __forceinline__ void pair_shift(PairRow &r)
 /* a lane's two columns of a row: one 8-byte load (VEC: nx even, 8-byte
  * aligned grid, x0 even), or one by one */
 template <bool VEC>
-__device__ __forceinline__ F2 pair_load(const float *__restrict__ row, int x0, int x1)
+__device__ __forceinline__ F2 pair_load(const float *row, int x0, int x1)
+{
+  return VEC ? ld2(row + x0) : pk(row[x0], row[x1]);
+}
+/* the same for a grid no launch of the chain writes */
+template <bool VEC>
+__device__ __forceinline__ F2 pair_ldg(const float *row, int x0, int x1)
 {
   return VEC ? ldg2(row + x0) : pk(__ldg(row + x0), __ldg(row + x1));
 }
 
-/* Tile (bx, by): T steps from a into b.  Loads are clamped to the grid;
+/* Tile (bx, by): T steps from a into b.  talus and extra are loaded before
+ * the wait for the launch before (hm_chain.cuh).  Loads are clamped to the grid;
  * what lies outside only feeds halo cells, since border cells copy their
  * inward neighbour. */
 template <bool TMAP, class R, int ROWS, bool VEC>
-__device__ __forceinline__ void thermal_block(const float *__restrict__ a,
+__device__ __forceinline__ void thermal_block(const float *a,
                                               float *__restrict__ b,
                                               int nx,
                                               int ny,
@@ -92,10 +100,14 @@ __device__ __forceinline__ void thermal_block(const float *__restrict__ a,
   for (int q = 0; q < ROWS; q++)
   {
     const size_t o = (size_t)min(max(j0 + q, 0), ny - 1) * nx;
-    v[q + 1].c = pair_load<VEC>(a + o, x0, x1);
-    tl[q] = R::talus_pair(TMAP ? pair_load<VEC>(talus + o, x0, x1) : pk1(talus_value));
-    ex[q] = R::EXTRA ? pair_load<VEC>(extra + o, x0, x1) : pk1(0.f);
+    tl[q] = R::talus_pair(TMAP ? pair_ldg<VEC>(talus + o, x0, x1) : pk1(talus_value));
+    ex[q] = R::EXTRA ? pair_ldg<VEC>(extra + o, x0, x1) : pk1(0.f);
   }
+  chain_wait();
+  a = produced(a);
+#pragma unroll
+  for (int q = 0; q < ROWS; q++)
+    v[q + 1].c = pair_load<VEC>(a + (size_t)min(max(j0 + q, 0), ny - 1) * nx, x0, x1);
   for (int t = 0; t < T; t++)
   {
     const int par = t & 1;

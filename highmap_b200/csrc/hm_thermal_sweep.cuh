@@ -11,7 +11,9 @@
  * parameter) are issued before any of them is used, which keeps enough
  * bytes in flight to cover the HBM latency: the plain kernels take 8 (4
  * row pairs), the batched form's persistent kernel fewer, as its
- * occupancy hides the latency instead.  Cell rule and border copies as the reference kernel
+ * occupancy hides the latency instead.  z is read by plain loads (the
+ * launch before may have written it, hm_chain.cuh), talus and bedrock,
+ * constant for the whole solve, by non-coherent ones.  Cell rule and border copies as the reference kernel
  * (HighMap/src/gpu_opencl/kernels/thermal.cl:26-100, Jacobi form; border
  * copies _common_index.cl:106-132).
  */
@@ -53,7 +55,7 @@ struct TalusExchange
  * shuffles), output rows y0 .. y1-1, the loads of P rows in flight
  * together.  The whole warp must call it. */
 template <bool TMAP, class R, int P = SW_P>
-__device__ __forceinline__ void thermal_sweep_warp(const float *__restrict__ a,
+__device__ __forceinline__ void thermal_sweep_warp(const float *a,
                                                    float *__restrict__ b,
                                                    int nx,
                                                    int ny,
@@ -76,10 +78,10 @@ __device__ __forceinline__ void thermal_sweep_warp(const float *__restrict__ a,
   float vc[P + 2], vl[P + 2], vr[P + 2];
   {
     const float *r0 = a + (size_t)max(y0 - 1, 0) * nx, *r1 = a + (size_t)y0 * nx;
-    vc[0] = __ldg(r0 + gxc);
-    vl[0] = __ldg(r0 + hx);
-    vc[1] = __ldg(r1 + gxc);
-    vl[1] = __ldg(r1 + hx);
+    vc[0] = r0[gxc];
+    vl[0] = r0[hx];
+    vc[1] = r1[gxc];
+    vl[1] = r1[hx];
 #pragma unroll
     for (int q = 0; q < 2; q++)
     {
@@ -95,8 +97,8 @@ __device__ __forceinline__ void thermal_sweep_warp(const float *__restrict__ a,
     for (int q = 0; q < P; q++)
     {
       const float *r = a + (size_t)min(j0 + 1 + q, ny - 1) * nx;
-      vc[q + 2] = __ldg(r + gxc);
-      vl[q + 2] = __ldg(r + hx); /* the halo value until the shuffles below */
+      vc[q + 2] = r[gxc];
+      vl[q + 2] = r[hx]; /* the halo value until the shuffles below */
       const size_t o = (size_t)min(j0 + q, ny - 1) * nx + gxc;
       tl[q] = TMAP ? __ldg(talus + o) : talus_value;
       bd[q] = R::EXTRA ? __ldg(bedrock + o) : 0.f;
@@ -147,6 +149,12 @@ __device__ __forceinline__ F2 ldg2(const float *p)
   r.v = __ldg(reinterpret_cast<const unsigned long long *>(p));
   return r;
 }
+__device__ __forceinline__ F2 ld2(const float *p)
+{
+  F2 r;
+  r.v = *reinterpret_cast<const unsigned long long *>(p);
+  return r;
+}
 __device__ __forceinline__ void st2(float *p, F2 v) { *reinterpret_cast<unsigned long long *>(p) = v.v; }
 
 /* One row of a lane's column pair: the pair (x, y), the pair one column to
@@ -167,7 +175,7 @@ __device__ __forceinline__ void pair_exchange(PairRow &r, int lane, float halo)
 }
 
 template <bool TMAP, class R, int P = S2_P>
-__device__ __forceinline__ void thermal_sweep2_warp(const float *__restrict__ a,
+__device__ __forceinline__ void thermal_sweep2_warp(const float *a,
                                                     float *__restrict__ b,
                                                     int nx,
                                                     int ny,
@@ -192,8 +200,8 @@ __device__ __forceinline__ void thermal_sweep2_warp(const float *__restrict__ a,
   const bool halo_lane = lane == 0 || lane == 31;
   auto load = [&](int r, int q) {
     const float *row = a + (size_t)r * nx;
-    v[q].c = ldg2(row + gxc);
-    halo[q] = halo_lane ? __ldg(row + hx) : 0.f;
+    v[q].c = ld2(row + gxc);
+    halo[q] = halo_lane ? row[hx] : 0.f;
   };
   load(max(y0 - 1, 0), 0);
   load(y0, 1);

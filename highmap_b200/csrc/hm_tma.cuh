@@ -108,6 +108,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
   return false;
 }
 
+/* start fetching a tensor map's descriptor */
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map)
+{
+  asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
 /* 2-D tile load: box of the tensor map at (x, y) into dst, completion
  * counted on bar.  x must be a multiple of 4 for 32-bit elements. */
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar)

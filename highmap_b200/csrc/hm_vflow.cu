@@ -42,6 +42,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "hm_chain.cuh"
 #include "hm_internal.h"
 #include "hm_vpipes.h"
 #include "hm_vpipes_math.cuh"
@@ -143,12 +144,14 @@ __global__ void __launch_bounds__(VF_NT) k_vflow_init(float *__restrict__ h, con
  * pair a cell with itself, as the clamped reads do. */
 constexpr int VT_X = 32, VT_Y = 8;
 
-__global__ void __launch_bounds__(VT_X *VT_Y) k_vflow_step(const float *__restrict__ z, const float *__restrict__ hin,
+__global__ void __launch_bounds__(VT_X *VT_Y) k_vflow_step(const float *__restrict__ z, const float *hin,
                                                           float *__restrict__ hout, int nx, int ny, VfScalars *sc,
                                                           VfConst c, int want_max)
 {
   __shared__ float me[VT_Y][VT_X + 1]; /* me[ty][tx + 1]: east face of (tx, ty); [ty][0]: west edge  */
   __shared__ float mn[VT_Y + 1][VT_X]; /* mn[ty + 1][tx]: north face of (tx, ty); [0][tx]: south edge */
+  chain_wait();
+  hin = produced(hin);
   const int  tx = threadIdx.x, ty = threadIdx.y;
   const int  i = blockIdx.x * VT_X + tx, j = blockIdx.y * VT_Y + ty;
   const bool in = i < nx && j < ny;
@@ -195,14 +198,14 @@ __global__ void __launch_bounds__(VT_X *VT_Y) k_vflow_step(const float *__restri
 constexpr int VB_NW = 16, VB_NT = 32 * VB_NW, VB_TY = 2 * VB_NW, VB_TMAX = 5;
 
 template <bool VEC>
-__device__ __forceinline__ float2 vb_load(const float *__restrict__ row, int x0, int x1)
+__device__ __forceinline__ float2 vb_load(const float *row, int x0, int x1)
 {
-  return VEC ? __ldg(reinterpret_cast<const float2 *>(row + x0)) : make_float2(__ldg(row + x0), __ldg(row + x1));
+  return VEC ? *reinterpret_cast<const float2 *>(row + x0) : make_float2(row[x0], row[x1]);
 }
 
 template <bool VEC>
 __global__ void __launch_bounds__(VB_NT)
-    k_vflow_block(const float *__restrict__ z, const float *__restrict__ hin, float *__restrict__ hout, int nx, int ny,
+    k_vflow_block(const float *__restrict__ z, const float *hin, float *__restrict__ hout, int nx, int ny,
                   VfScalars *sc, VfConst c, int T, int want_max)
 {
   __shared__ float2 rows[2][VB_NW][2][32];
@@ -221,11 +224,14 @@ __global__ void __launch_bounds__(VB_NT)
     zr[q] = vb_load<VEC>(z + o, x0, x1);
     if (q == 1 || q == 2)
     {
-      h[q] = vb_load<VEC>(hin + o, x0, x1);
       zw[q - 1] = __ldg(z + o + min(max(gx - 1, 0), nx - 1));
       ze[q - 1] = __ldg(z + o + min(max(gx + 2, 0), nx - 1));
     }
   }
+  chain_wait();
+  hin = produced(hin);
+#pragma unroll
+  for (int q = 1; q < 3; q++) h[q] = vb_load<VEC>(hin + (size_t)min(max(j0 + q - 1, 0), ny - 1) * nx, x0, x1);
   const float dt = sc->dt;
   const bool  wedge = gx == 0, e0 = gx == nx - 1, e1 = gx + 1 == nx - 1;
   for (int t = 0; t < T; t++)
@@ -299,9 +305,11 @@ __global__ void __launch_bounds__(VB_NT)
 }
 
 /* water_depth_dry_out: h -= ratio * hmax, then max(0, h) */
-__global__ void __launch_bounds__(VF_NT) k_vflow_dry_out(const float *__restrict__ h, const VfScalars *sc,
+__global__ void __launch_bounds__(VF_NT) k_vflow_dry_out(const float *h, VfScalars *sc,
                                                          float ratio, float *__restrict__ out, size_t n)
 {
+  chain_wait();
+  h = produced(h);
   const float drop = fmul(ratio, funkey(sc->hmax));
   for (size_t k = blockIdx.x * (size_t)VF_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * VF_NT)
   {
@@ -361,7 +369,7 @@ int vflow_core(const float *z, int nx, int ny, float water_height, const float *
     if (per == 1)
     {
       const dim3 tiles((nx + VT_X - 1) / VT_X, (ny + VT_Y - 1) / VT_Y);
-      k_vflow_step<<<tiles, dim3(VT_X, VT_Y), 0, s>>>(z, cur, nxt, nx, ny, sc, c, want_max);
+      chain_launch(it > 0, k_vflow_step, tiles, dim3(VT_X, VT_Y), s, z, cur, nxt, nx, ny, sc, c, want_max);
       HM_LAUNCH_CHECK("k_vflow_step");
     }
     else
@@ -369,8 +377,8 @@ int vflow_core(const float *z, int nx, int ny, float water_height, const float *
       const int  w = 64 - 4 * ((T + 1) / 2), hgt = VB_TY - 2 * T;
       const dim3 tiles((nx + w - 1) / w, (ny + hgt - 1) / hgt);
       const bool vec = nx % 2 == 0 && al8(z) && al8(cur) && al8(nxt);
-      if (vec) k_vflow_block<true><<<tiles, VB_NT, 0, s>>>(z, cur, nxt, nx, ny, sc, c, T, want_max);
-      else k_vflow_block<false><<<tiles, VB_NT, 0, s>>>(z, cur, nxt, nx, ny, sc, c, T, want_max);
+      chain_launch(it > 0, vec ? k_vflow_block<true> : k_vflow_block<false>, tiles, dim3(VB_NT), s, z, cur, nxt, nx, ny,
+                   sc, c, T, want_max);
       HM_LAUNCH_CHECK("k_vflow_block");
     }
     float *t = cur;
@@ -380,7 +388,7 @@ int vflow_core(const float *z, int nx, int ny, float water_height, const float *
   }
   if (dry_out_ratio != 0.f)
   {
-    k_vflow_dry_out<<<VF_GRID, VF_NT, 0, s>>>(cur, sc, dry_out_ratio, water_depth, n);
+    chain_launch(iterations > 0, k_vflow_dry_out, dim3(VF_GRID), dim3(VF_NT), s, cur, sc, dry_out_ratio, water_depth, n);
     HM_LAUNCH_CHECK("k_vflow_dry_out");
   }
   else if (cur != water_depth)

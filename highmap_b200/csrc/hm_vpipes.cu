@@ -484,7 +484,8 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     if (it > 0)
       rc = step_tma ? launch_step_tma(io, mp, am[buf ^ 1], c, sc, partials, g1, s)
                     : launch_step_cp_async(io, u_buf[buf ^ 1], v_buf[buf ^ 1], c, sc, partials, g1, s);
-    else rc = tma ? launch_fwe_tma(io, mp, c, sc, partials, g1, s) : launch_fwe_cp_async(io, c, sc, partials, g1, s);
+    else rc = tma ? launch_fwe_tma(io, mp, c, sc, partials, g1, s, false)
+                  : launch_fwe_cp_async(io, c, sc, partials, g1, s, false);
     if (rc) return rc;
     /* the advection of this step is folded into the next step's tiles; the
      * last step's runs here */

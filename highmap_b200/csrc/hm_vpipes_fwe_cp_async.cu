@@ -22,10 +22,10 @@ template <bool M, int F> struct CpAsyncKernel
 } // namespace
 
 int launch_fwe_cp_async(const FweIo &io, const VpConst &c, VpScalars *sc, double *partials, dim3 grid,
-                        cudaStream_t s)
+                        cudaStream_t s, bool chained)
 {
   return fwe_dispatch<CpAsyncKernel>(io.maintain != 0, fwe_flags(io, c), [&](auto kernel) -> int {
-    kernel<<<grid, FT_NT, 0, s>>>(io, c, sc, partials);
+    chain_launch(chained, kernel, grid, dim3(FT_NT), s, io, c, sc, partials);
     HM_LAUNCH_CHECK("k_vp_fwe");
     return HM_OK;
   });

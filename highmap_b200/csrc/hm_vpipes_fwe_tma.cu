@@ -22,10 +22,10 @@ template <bool M, int F> struct TmaKernel
 } // namespace
 
 int launch_fwe_tma(const FweIo &io, const FweMaps &maps, const VpConst &c, VpScalars *sc, double *partials,
-                   dim3 grid, cudaStream_t s)
+                   dim3 grid, cudaStream_t s, bool chained)
 {
   return fwe_dispatch<TmaKernel>(io.maintain != 0, fwe_flags(io, c), [&](auto kernel) -> int {
-    kernel<<<grid, FT_NT, 0, s>>>(io, maps, c, sc, partials);
+    chain_launch(chained, kernel, grid, dim3(FT_NT), s, io, maps, c, sc, partials);
     HM_LAUNCH_CHECK("k_vp_fwe_tma");
     return HM_OK;
   });

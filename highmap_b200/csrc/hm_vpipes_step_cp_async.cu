@@ -25,7 +25,7 @@ int launch_step_cp_async(const FweIo &io, const float *u_prev, const float *v_pr
                          double *partials, dim3 grid, cudaStream_t s)
 {
   return step_dispatch<StepCpKernel>(io.maintain != 0, fwe_flags(io, c), [&](auto kernel) -> int {
-    kernel<<<grid, FT_NT, 0, s>>>(io, u_prev, v_prev, c, sc, partials);
+    chain_launch(true, kernel, grid, dim3(FT_NT), s, io, u_prev, v_prev, c, sc, partials);
     HM_LAUNCH_CHECK("k_vp_step");
     return HM_OK;
   });

@@ -25,7 +25,7 @@ int launch_step_tma(const FweIo &io, const FweMaps &maps, const AdvMaps &am, con
                     double *partials, dim3 grid, cudaStream_t s)
 {
   return step_dispatch<StepKernel>(io.maintain != 0, fwe_flags(io, c), [&](auto kernel) -> int {
-    kernel<<<grid, FT_NT, 0, s>>>(io, maps, am, c, sc, partials);
+    chain_launch(true, kernel, grid, dim3(FT_NT), s, io, maps, am, c, sc, partials);
     HM_LAUNCH_CHECK("k_vp_step_tma");
     return HM_OK;
   });

@@ -42,6 +42,7 @@
 
 #include <type_traits>
 
+#include "hm_chain.cuh"
 #include "hm_reduce.cuh"
 #include "hm_vpipes_fused.cuh"
 #include "hm_vpipes_math.cuh"
@@ -343,7 +344,15 @@ __device__ __forceinline__ bool fwe_stage_tma(const FweMaps &maps, int nx, int n
   {
     mbar_init(&sm.bar, 1);
     mbar_fence_init();
+    tma_prefetch_map(&maps.z);
+    tma_prefetch_map(&maps.d);
+    if (WITH_S) tma_prefetch_map(&maps.s);
+    tma_prefetch_map(&maps.fl);
+    tma_prefetch_map(&maps.fr);
+    tma_prefetch_map(&maps.ft);
+    tma_prefetch_map(&maps.fb);
   }
+  chain_wait(); /* the launch before has written the grids */
   __syncthreads();
   if (tid == 0)
   {
@@ -381,7 +390,17 @@ __device__ __forceinline__ bool fwe_stage_tma_step(const FweMaps &maps, const Ad
     mbar_init(&sm.bar, 1);
     mbar_init(&sm.bar2, 1);
     mbar_fence_init();
+    tma_prefetch_map(&am.u);
+    tma_prefetch_map(&am.v);
+    tma_prefetch_map(&am.s1);
+    tma_prefetch_map(&maps.z);
+    tma_prefetch_map(&maps.d);
+    tma_prefetch_map(&maps.fl);
+    tma_prefetch_map(&maps.fr);
+    tma_prefetch_map(&maps.ft);
+    tma_prefetch_map(&maps.fb);
   }
+  chain_wait(); /* the step before has written the grids */
   __syncthreads();
   if (tid == 0)
   {
@@ -450,7 +469,7 @@ __device__ __forceinline__ AdvBox adv_box(int nx, int ny, int x0, int y0)
 
 /* advected sediment of one region-1 cell: column gx, row gy of the grid
  * (clamped), at shared-memory row l and column cc */
-__device__ __forceinline__ void advect_cell(const VpConst &c, const float *__restrict__ s1g, const AdvBox &bx, int x0,
+__device__ __forceinline__ void advect_cell(const VpConst &c, const float *s1g, const AdvBox &bx, int x0,
                                             int y0, int gx, int gy, int l, int cc, FweSmem &sm)
 {
   const int   nx = c.nx, ny = c.ny, ld = c.ld;
@@ -479,8 +498,7 @@ __device__ __forceinline__ void advect_cell(const VpConst &c, const float *__res
   }
   const Tap    t = linear_tap(x, y, nx, ny);
   const size_t r0 = (size_t)t.j0 * ld, r1 = (size_t)t.j1 * ld;
-  sm.s[l][cc] = blend(t, __ldg(s1g + r0 + t.i0), __ldg(s1g + r0 + t.i1), __ldg(s1g + r1 + t.i0),
-                      __ldg(s1g + r1 + t.i1));
+  sm.s[l][cc] = blend(t, s1g[r0 + t.i0], s1g[r0 + t.i1], s1g[r1 + t.i0], s1g[r1 + t.i1]);
 }
 
 /* rows of region 1 one thread advects */
@@ -491,7 +509,7 @@ constexpr int ADV_ROWS = 3;
  * and its gathers are in flight together (2 % fewer instructions per step
  * than one cell per loop item). */
 template <bool INNER>
-__device__ __forceinline__ void advect_region1(const VpConst &c, const float *__restrict__ s1g, int x0, int y0,
+__device__ __forceinline__ void advect_region1(const VpConst &c, const float *s1g, int x0, int y0,
                                                FweSmem &sm)
 {
   static_assert(FT_H1 % ADV_ROWS == 0, "region 1 splits into whole row groups");
@@ -768,6 +786,7 @@ template <bool MAINTAIN, int F>
 __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F)) k_vp_fwe(FweIo io, VpConst c, VpScalars *sc, double *partials)
 {
   __shared__ FweSmem sm;
+  chain_wait();
   fwe_stage_cp_async(io, c.nx, c.ny, c.ld, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm);
   __syncthreads();
   if (fwe_inner_tile(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY))
@@ -810,10 +829,11 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
  * step's velocity and eroded sediment. */
 template <bool MAINTAIN, int F>
 __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
-    k_vp_step(FweIo io, const float *__restrict__ u_prev, const float *__restrict__ v_prev, VpConst c,
+    k_vp_step(FweIo io, const float *u_prev, const float *v_prev, VpConst c,
               VpScalars *sc, double *partials)
 {
   __shared__ FweSmem sm;
+  chain_wait();
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
   if (stage16_tile(io, c.nx, c.ny, x0, y0)) fwe_stage_cp_async16_step(io, u_prev, v_prev, c.ld, x0, y0, sm);
   else fwe_stage_cp_async_step(io, u_prev, v_prev, c.nx, c.ny, c.ld, x0, y0, sm);
@@ -875,11 +895,12 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
 
 /* Launch one k_vp_fwe (tma false) or k_vp_fwe_tma (maps != NULL) step on
  * stream s with the kernel specialised for the step's options
- * (hm_vpipes_fwe_cp_async.cu, hm_vpipes_fwe_tma.cu). */
+ * (hm_vpipes_fwe_cp_async.cu, hm_vpipes_fwe_tma.cu), chained to the
+ * launch before it (hm_chain.cuh) or not; the later steps' are always. */
 int launch_fwe_cp_async(const FweIo &io, const VpConst &c, VpScalars *sc, double *partials, dim3 grid,
-                        cudaStream_t s);
+                        cudaStream_t s, bool chained);
 int launch_fwe_tma(const FweIo &io, const FweMaps &maps, const VpConst &c, VpScalars *sc, double *partials,
-                   dim3 grid, cudaStream_t s);
+                   dim3 grid, cudaStream_t s, bool chained);
 /* Launch one k_vp_step_tma step (hm_vpipes_step_tma.cu); io.s1_prev and am
  * hold the previous step's s1, u and v. */
 int launch_step_tma(const FweIo &io, const FweMaps &maps, const AdvMaps &am, const VpConst &c, VpScalars *sc,
