@@ -123,6 +123,8 @@ __device__ __forceinline__ void job_io(const BJob &J, int step, FweIo &io)
   io.vec = J.vec;
   io.stage16 = J.stage16;
   io.flow_only = 0;
+  io.sum_in = nullptr;
+  io.sum_out = nullptr;
 }
 
 template <bool TMAP, int BED>
@@ -208,9 +210,9 @@ __global__ void __launch_bounds__(BT, BATCH_CTAS_PER_SM)
       __syncthreads();
       if (step > 0) advect_region1<false>(s_c, s_io.s1_prev, x0, y0, sm);
       if (J.maintain)
-        fwe_compute<true, F>(s_io, s_c, J.sc, J.partials, tl.y, tl.z, J.nbx, J.nby, sm);
+        fwe_compute<true, F>(s_io, s_c, J.sc, J.partials, J.sc->add[s_io.parity], tl.y, tl.z, J.nbx, J.nby, sm);
       else
-        fwe_compute<false, F>(s_io, s_c, J.sc, J.partials, tl.y, tl.z, J.nbx, J.nby, sm);
+        fwe_compute<false, F>(s_io, s_c, J.sc, J.partials, 0.f, tl.y, tl.z, J.nbx, J.nby, sm);
     }
     else
     {

@@ -110,6 +110,14 @@ __global__ void __launch_bounds__(VP_NT) k_vp_init_finish(VpScalars *sc, const d
   }
 }
 
+/* the last step's top-up, for the water-depth output, from the water per
+ * tile (FweIo) */
+__global__ void __launch_bounds__(FT_NT) k_vp_top_up(const double *tiles, unsigned n, VpScalars *sc, int parity)
+{
+  const float add = tiles_top_up(tiles, n, sc);
+  if (threadIdx.x == 0) sc->add[parity] = add;
+}
+
 /* ---- outputs -------------------------------------------------------- */
 
 /* water depth output: the stored depth plus the last step's top-up */
@@ -199,7 +207,8 @@ static dim3 fused_grid(const FusedCfg &c, int nx, int ny)
   return dim3((nx + w - 1) / w, (ny + c.h - 1) / c.h);
 }
 
-static size_t partials_bytes(int nx, int ny)
+/* one of the two buffers of partial sums that the steps alternate between */
+static size_t partials_half(int nx, int ny)
 {
   /* one slot per block of the step grid: the tiled kernel's 32 x 16 tiles
    * outnumber the streaming kernel's strips and chunks */
@@ -209,6 +218,8 @@ static size_t partials_bytes(int nx, int ny)
   if (blocks < 2 * VP_INIT_BLOCKS) blocks = 2 * VP_INIT_BLOCKS;
   return align_up(blocks * sizeof(double), 256);
 }
+
+static size_t partials_bytes(int nx, int ny) { return 2 * partials_half(nx, ny); }
 
 int vpipes_check_args(const float *z, int nx, int ny, const hm_vpipes_params *p)
 {
@@ -427,6 +438,8 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
   const dim3 g1((nx + FT_TX - 1) / FT_TX, (ny + FT_TY - 1) / FT_TY);
   const int  row_groups = (ny + ADV_R - 1) / ADV_R;
   const dim3 g2((nx + 255) / 256, row_groups < 65535 ? row_groups : 65535);
+  double    *sums[2] = {partials, partials + partials_half(nx, ny) / sizeof(double)};
+  const bool direct_sum = io.maintain && g1.x * g1.y <= SUM_TILES_MAX;
   VpFields  *cur = &A, *nxt = &B;
   float     *s_last = A.s; /* sediment after the last step; step 0 reads its zeros before */
   int        parity = 0;
@@ -479,6 +492,8 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     if (io.u_out && !io.v_out) io.v_out = io.v;
     if (io.v_out && !io.u_out) io.u_out = io.u;
     io.parity = parity;
+    io.sum_out = direct_sum ? sums[it & 1] : nullptr;
+    io.sum_in = direct_sum && it > 0 ? sums[(it & 1) ^ 1] : nullptr;
     const FweMaps &mp = maps[cur == &A ? 0 : 1];
     int            rc;
     if (it > 0)
@@ -511,6 +526,11 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
   };
   int rc;
   if ((rc = result(z, cur->z))) return rc;
+  if (water_depth && direct_sum && p.iterations > 0)
+  {
+    k_vp_top_up<<<1, FT_NT, 0, s>>>(sums[(p.iterations - 1) & 1], g1.x * g1.y, sc, parity);
+    HM_LAUNCH_CHECK("k_vp_top_up");
+  }
   if (water_depth &&
       (rc = vpipes_final_depth(cur->d, rain, sc, parity, p.maintain_water_volume != 0, water_depth, nx, ny, s, ld)))
     return rc;

@@ -144,7 +144,50 @@ struct FweIo
   unsigned     tma_extra_tx;  /* bytes a TMA tile's barrier expects beyond its boxes: 0, or the
                                * test hook's count, which makes every tile's wait run out */
   const float *s1_prev;       /* k_vp_step(_tma): the previous step's eroded sediment */
+  /* Volume top-up: the step before's water per tile, which every CTA of
+   * this step sums for itself while its boxes are in flight, and this
+   * step's; null: sc->add and the last-CTA finish (grid_sum_commit). */
+  const double *sum_in;
+  double       *sum_out;
 };
+
+/* Most tiles of a grid whose steps sum the tiles' water themselves.  The
+ * last-CTA finish costs a fence and an atomic round trip at the end of
+ * every CTA (2300 of 9200 cycles at 256^2); the sum costs a load per 256
+ * tiles and thread, hidden behind the staging wait, but its traffic grows
+ * with the square of the tiles (33 MB of L2 reads per step at 2048). */
+constexpr unsigned SUM_TILES_MAX = 2048;
+
+/* The top-up of this step from the water per tile: the sum of
+ * grid_sum_commit in the same order.  For every thread of the CTA. */
+__device__ __forceinline__ float tiles_top_up(const double *tiles, unsigned n, const VpScalars *sc)
+{
+  __shared__ double sm[FT_NT / 32];
+  __shared__ float  s_add;
+  double            acc = 0.0;
+  for (unsigned k = threadIdx.x; k < n; k += FT_NT) acc += tiles[k];
+  const double total = block_sum<FT_NT>(acc, sm);
+  if (threadIdx.x == 0) s_add = fsub(sc->v0, (float)total);
+  __syncthreads();
+  return s_add;
+}
+
+/* this tile's water, at the end of the step; every thread of the CTA */
+__device__ __forceinline__ void tile_water_commit(const FweIo &io, VpScalars *sc, double *partials, double part,
+                                                  unsigned ntiles, unsigned tile)
+{
+  if (io.sum_out)
+  {
+    __shared__ double sm[FT_NT / 32];
+    const double      b = block_sum<FT_NT>(part, sm);
+    if (threadIdx.x == 0) io.sum_out[tile] = b;
+    return;
+  }
+  const float v0 = sc->v0;
+  float      *outp = &sc->add[io.parity ^ 1];
+  grid_sum_commit<FT_NT>(part, partials, &sc->ticket, ntiles, tile,
+                         [&](double total) { *outp = fsub(v0, (float)total); });
+}
 
 /* tensor maps of the seven input fields of one step (TMA staging):
  * z and d with a 40 x 20 box, s and the fluxes with a 40 x 18 box */
@@ -377,12 +420,13 @@ __device__ __forceinline__ bool fwe_stage_tma(const FweMaps &maps, int nx, int n
  * waited for here.  Group B: z (region 2) and the old fluxes (region 1),
  * waited for by fwe_wait_tma_step_b after the advection (and the depth
  * pass) have run on group A, so those overlap its arrival.  The stored
- * depth d (region 2) is in group A if D_FIRST.  Returns false, uniformly across the CTA, if group A did
+ * depth d (region 2) is in group A if D_FIRST.  between() runs while the
+ * boxes are in flight.  Returns false, uniformly across the CTA, if group A did
  * not complete in time; group B's loads are then given their own windows
  * to land before the CTA leaves. */
-template <bool D_FIRST>
+template <bool D_FIRST, class Between>
 __device__ __forceinline__ bool fwe_stage_tma_step(const FweMaps &maps, const AdvMaps &am, int x0, int y0,
-                                                   FweSmem &sm, unsigned extra_tx)
+                                                   FweSmem &sm, unsigned extra_tx, Between between)
 {
   const int tid = threadIdx.x;
   if (tid == 0)
@@ -417,6 +461,7 @@ __device__ __forceinline__ bool fwe_stage_tma_step(const FweMaps &maps, const Ad
     tma_load_2d(&sm.fo[2][0][0], &maps.ft, x0 - 4, y0 - 1, &sm.bar2);
     tma_load_2d(&sm.fo[3][0][0], &maps.fb, x0 - 4, y0 - 1, &sm.bar2);
   }
+  between();
   bool ok = mbar_wait_bounded(&sm.bar, 0);
   if (!ok) ok = mbar_wait_bounded(&sm.bar, 0); /* loads still in flight: give them a second window */
   if (__syncthreads_and(ok)) return true;
@@ -567,7 +612,7 @@ struct NoMid
 
 template <bool MAINTAIN, int F, bool INNER = false, class Mid = NoMid>
 __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, VpScalars *sc, double *partials,
-                                            int bx, int by, int nbx, int nby, FweSmem &sm, Mid mid = Mid())
+                                            float add, int bx, int by, int nbx, int nby, FweSmem &sm, Mid mid = Mid())
 {
   static_assert(FT_TX == 32 && FT_TY == 16 && FT_NT == 256, "one cell pair per thread in the water pass");
   constexpr bool GEN = (F & FWE_GENERIC) != 0;
@@ -576,7 +621,6 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
   const int      tid = threadIdx.x;
   const int      nx = c.nx, ny = c.ny;
   const int      x0 = bx * FT_TX, y0 = by * FT_TY;
-  const float    add = MAINTAIN ? sc->add[io.parity] : 0.f;
   const float    rvol = MAINTAIN ? sc->rvol : 1.f;
   const bool     rain_step = RT ? c.rps != 0.f : (F & FWE_RAINSTEP) != 0;
   const bool     rain_map = RT ? io.rain != nullptr : (F & FWE_RAINMAP) != 0;
@@ -766,13 +810,7 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
     }
   }
 
-  if (MAINTAIN)
-  {
-    const float v0 = sc->v0;
-    float      *outp = &sc->add[io.parity ^ 1];
-    grid_sum_commit<FT_NT>(part, partials, &sc->ticket, (unsigned)(nbx * nby), (unsigned)(by * nbx + bx),
-                           [&](double total) { *outp = fsub(v0, (float)total); });
-  }
+  if (MAINTAIN) tile_water_commit(io, sc, partials, part, (unsigned)(nbx * nby), (unsigned)(by * nbx + bx));
 }
 
 /* the tile at (x0, y0) and its 2-cell halo lie inside the grid, and the
@@ -789,10 +827,11 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F)) k_vp_fwe(FweIo io, V
   chain_wait();
   fwe_stage_cp_async(io, c.nx, c.ny, c.ld, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm);
   __syncthreads();
+  const float add = MAINTAIN ? sc->add[io.parity] : 0.f;
   if (fwe_inner_tile(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY))
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
   else
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
 }
 
 /* The same step with the input tiles fetched by TMA.  A tile whose loads
@@ -808,19 +847,14 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   {
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
     if (MAINTAIN)
-    {
-      const float v0 = sc->v0;
-      float      *outp = &sc->add[io.parity ^ 1];
-      grid_sum_commit<FT_NT>(0.0, partials, &sc->ticket, gridDim.x * gridDim.y,
-                             blockIdx.y * gridDim.x + blockIdx.x,
-                             [&](double total) { *outp = fsub(v0, (float)total); });
-    }
+      tile_water_commit(io, sc, partials, 0.0, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x);
     return;
   }
+  const float add = MAINTAIN ? sc->add[io.parity] : 0.f;
   if (fwe_inner_tile(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY))
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
   else
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
 }
 
 /* A step after the first with cp.async staging (grids the TMA rules
@@ -835,6 +869,9 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   __shared__ FweSmem sm;
   chain_wait();
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
+  float     add = 0.f;
+  if (MAINTAIN)
+    add = io.sum_in ? tiles_top_up(io.sum_in, gridDim.x * gridDim.y, sc) : sc->add[io.parity];
   if (stage16_tile(io, c.nx, c.ny, x0, y0)) fwe_stage_cp_async16_step(io, u_prev, v_prev, c.ld, x0, y0, sm);
   else fwe_stage_cp_async_step(io, u_prev, v_prev, c.nx, c.ny, c.ld, x0, y0, sm);
   __syncthreads();
@@ -843,12 +880,12 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   if (fwe_inner_tile(io, c.nx, c.ny, x0, y0))
   {
     advect_region1<true>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
   }
   else
   {
     advect_region1<false>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
   }
 }
 
@@ -862,17 +899,15 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
 {
   __shared__ FweSmem sm;
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
-  if (!fwe_stage_tma_step<MAINTAIN>(maps, am, x0, y0, sm, io.tma_extra_tx))
+  float     add = 0.f;
+  auto      top_up = [&]() {
+    if (MAINTAIN) add = io.sum_in ? tiles_top_up(io.sum_in, gridDim.x * gridDim.y, sc) : sc->add[io.parity];
+  };
+  if (!fwe_stage_tma_step<MAINTAIN>(maps, am, x0, y0, sm, io.tma_extra_tx, top_up))
   {
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
     if (MAINTAIN)
-    {
-      const float v0 = sc->v0;
-      float      *outp = &sc->add[io.parity ^ 1];
-      grid_sum_commit<FT_NT>(0.0, partials, &sc->ticket, gridDim.x * gridDim.y,
-                             blockIdx.y * gridDim.x + blockIdx.x,
-                             [&](double total) { *outp = fsub(v0, (float)total); });
-    }
+      tile_water_commit(io, sc, partials, 0.0, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x);
     return;
   }
   /* group B (z, fluxes) arrives during the advection and the depth pass */
@@ -884,12 +919,12 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   if (fwe_inner_tile(io, c.nx, c.ny, x0, y0))
   {
     advect_region1<true>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm, group_b);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm, group_b);
   }
   else
   {
     advect_region1<false>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm, group_b);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm, group_b);
   }
 }
 
