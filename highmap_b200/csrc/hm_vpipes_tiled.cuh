@@ -512,47 +512,13 @@ __device__ __forceinline__ AdvBox adv_box(int nx, int ny, int x0, int y0)
   return b;
 }
 
-/* advected sediment of one region-1 cell: column gx, row gy of the grid
- * (clamped), at shared-memory row l and column cc */
-__device__ __forceinline__ void advect_cell(const VpConst &c, const float *s1g, const AdvBox &bx, int x0,
-                                            int y0, int gx, int gy, int l, int cc, FweSmem &sm)
-{
-  const int   nx = c.nx, ny = c.ny, ld = c.ld;
-  const float uu = sm.adv.u[gy - (y0 - 1)][gx - (x0 - 4)];
-  const float vv = sm.adv.v[gy - (y0 - 1)][gx - (x0 - 4)];
-  const float x = fsub((float)gx, fmul(c.dt, uu));
-  const float y = fsub((float)gy, fmul(c.dt, vv));
-  /* floor by adding 2^23 rounded down: 2^23 + floor(v) for v in [0, 2^23),
-   * whose integer is in the low bits (a quarter of the cost of two floors
-   * and two conversions, which share the 4-lane unit with the divisions);
-   * a negative, huge or NaN v gives an index outside the box */
-  const float xm = fsub(x, 0.5f), ym = fsub(y, 0.5f);
-  const float tx = __fadd_rd(xm, 8388608.f), ty = __fadd_rd(ym, 8388608.f);
-  const int   i0 = __float_as_int(tx) - 0x4b000000, j0 = __float_as_int(ty) - 0x4b000000;
-  if ((unsigned)(i0 - bx.lo_x) < bx.n_x && (unsigned)(j0 - bx.lo_y) < bx.n_y)
-  {
-    /* The four texels lie in the staged box and i0 in [0, nx - 2]: the
-     * mirror of linear_tap returns the coordinate itself and nothing is
-     * clamped.  The same rounded operations without the identities. */
-    Tap t;
-    t.a = fsub(xm, fsub(tx, 8388608.f));
-    t.b = fsub(ym, fsub(ty, 8388608.f));
-    const float *r = &sm.adv.s1[j0 - (y0 - 4)][i0 - (x0 - 4)];
-    sm.s[l][cc] = blend(t, r[0], r[1], r[FW], r[FW + 1]);
-    return;
-  }
-  const Tap    t = linear_tap(x, y, nx, ny);
-  const size_t r0 = (size_t)t.j0 * ld, r1 = (size_t)t.j1 * ld;
-  sm.s[l][cc] = blend(t, s1g[r0 + t.i0], s1g[r0 + t.i1], s1g[r1 + t.i0], s1g[r1 + t.i1]);
-}
-
 /* rows of region 1 one thread advects */
 constexpr int ADV_ROWS = 3;
 
 /* Thread t < 204 takes column 3 + t % 34 of region 1 and its rows
- * ADV_ROWS (t / 34) .. + ADV_ROWS - 1: the column's index work is shared
- * and its gathers are in flight together (2 % fewer instructions per step
- * than one cell per loop item). */
+ * ADV_ROWS (t / 34) .. + ADV_ROWS - 1, as one straight chain where the taps
+ * of all three lie in the staged box (nearly always), so that their loads
+ * and blends overlap; else cell by cell. */
 template <bool INNER>
 __device__ __forceinline__ void advect_region1(const VpConst &c, const float *s1g, int x0, int y0,
                                                FweSmem &sm)
@@ -560,16 +526,58 @@ __device__ __forceinline__ void advect_region1(const VpConst &c, const float *s1
   static_assert(FT_H1 % ADV_ROWS == 0, "region 1 splits into whole row groups");
   const int t = threadIdx.x;
   if (t >= FT_W1 * (FT_H1 / ADV_ROWS)) return;
-  const int cc = 3 + t % FT_W1, l0 = ADV_ROWS * (t / FT_W1);
+  const int    cc = 3 + t % FT_W1, l0 = ADV_ROWS * (t / FT_W1);
   const AdvBox bx = adv_box(c.nx, c.ny, x0, y0);
   int          gx = x0 - 4 + cc;
   if (!INNER) gx = clampi(gx, 0, c.nx - 1);
+  float xm[ADV_ROWS], ym[ADV_ROWS], tx[ADV_ROWS], ty[ADV_ROWS];
+  bool  staged = true;
 #pragma unroll
   for (int r = 0; r < ADV_ROWS; r++)
   {
     int gy = y0 - 1 + l0 + r;
     if (!INNER) gy = clampi(gy, 0, c.ny - 1);
-    advect_cell(c, s1g, bx, x0, y0, gx, gy, l0 + r, cc, sm);
+    const float uu = sm.adv.u[gy - (y0 - 1)][gx - (x0 - 4)];
+    const float vv = sm.adv.v[gy - (y0 - 1)][gx - (x0 - 4)];
+    xm[r] = fsub(fsub((float)gx, fmul(c.dt, uu)), 0.5f);
+    ym[r] = fsub(fsub((float)gy, fmul(c.dt, vv)), 0.5f);
+    /* floor by adding 2^23 rounded down: 2^23 + floor(v) for v in [0, 2^23),
+     * whose integer is in the low bits (a quarter of the cost of two floors
+     * and two conversions, which share the 4-lane unit with the divisions);
+     * a negative, huge or NaN v gives an index outside the box */
+    tx[r] = __fadd_rd(xm[r], 8388608.f);
+    ty[r] = __fadd_rd(ym[r], 8388608.f);
+    staged = staged && (unsigned)(__float_as_int(tx[r]) - 0x4b000000 - bx.lo_x) < bx.n_x &&
+             (unsigned)(__float_as_int(ty[r]) - 0x4b000000 - bx.lo_y) < bx.n_y;
+  }
+  if (staged)
+  {
+    /* The texels lie in the staged box and i0 in [0, nx - 2]: the mirror of
+     * linear_tap returns the coordinate itself and nothing is clamped.  The
+     * same rounded operations without the identities. */
+#pragma unroll
+    for (int r = 0; r < ADV_ROWS; r++)
+    {
+      Tap p;
+      p.a = fsub(xm[r], fsub(tx[r], 8388608.f));
+      p.b = fsub(ym[r], fsub(ty[r], 8388608.f));
+      const float *q = &sm.adv.s1[0][0] + ((__float_as_int(ty[r]) - 0x4b000000 - (y0 - 4)) * FW +
+                                           (__float_as_int(tx[r]) - 0x4b000000 - (x0 - 4)));
+      sm.s[l0 + r][cc] = blend(p, q[0], q[1], q[FW], q[FW + 1]);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int r = 0; r < ADV_ROWS; r++)
+  {
+    /* s1 of the previous step is complete in global memory */
+    int gy = y0 - 1 + l0 + r;
+    if (!INNER) gy = clampi(gy, 0, c.ny - 1);
+    const float  uu = sm.adv.u[gy - (y0 - 1)][gx - (x0 - 4)];
+    const float  vv = sm.adv.v[gy - (y0 - 1)][gx - (x0 - 4)];
+    const Tap    p = linear_tap(fsub((float)gx, fmul(c.dt, uu)), fsub((float)gy, fmul(c.dt, vv)), c.nx, c.ny);
+    const size_t r0 = (size_t)p.j0 * c.ld, r1 = (size_t)p.j1 * c.ld;
+    sm.s[l0 + r][cc] = blend(p, s1g[r0 + p.i0], s1g[r0 + p.i1], s1g[r1 + p.i0], s1g[r1 + p.i1]);
   }
 }
 
