@@ -24,7 +24,9 @@
  *
  * Powers that are multiples of 1/2 from 1 to 4 (the default is 2.5) are
  * x^floor times sqrt(x) in fp64, at most five roundings of 2^-53: the same
- * accuracy at a fifth of pow's instructions.
+ * accuracy at a fifth of pow's instructions.  Those with a square root
+ * come from fp32 pairs where the rounding to fp32 is certain (nearly
+ * always), off the fp64 pipe and its conversions.
  *
  * Kernels
  *   k_vflow_block  up to VB_TMAX steps per launch on a 64 x 32 tile in
@@ -32,9 +34,8 @@
  *                  owns two rows, two columns per lane), up to 1.5 M
  *                  cells, where a step's launch (4.1 us of host time) is
  *                  longer than its arithmetic: 512^2, power 2.5, 200
- *                  steps 2.51 ms with one step per launch and pow, 0.94 ms
- *                  here (23 us a launch, bound by the fp64 pipe and its
- *                  conversions).
+ *                  steps 2.51 ms with one step per launch and pow, 0.76 ms
+ *                  here (0.86 with the powers in fp64).
  *   k_vflow_step   one step, a 32 x 8 tile in shared memory (larger grids).
  */
 #include <cuda_runtime.h>
@@ -83,10 +84,47 @@ struct VfConst
   int   half;
 };
 
+/* x^1.5, x^2.5 or x^3.5 (half 3, 5, 7) rounded as vf_pow rounds them, from
+ * fp32 arithmetic in unevaluated sums of two (error-free products;
+ * Dekker, Numer. Math. 18, 1971): the root is g + d r / 2 with g = RN(x r),
+ * r ~ 1 / sqrt(x), d = x - g g; the power is (h + l)(g + c).  Relative
+ * error under 2^-41; ok is cleared unless the float is the same 2^-40 to
+ * either side (3 in 10^5 fail), and for x outside [1e-8, 1e8] but 0. */
+__device__ __forceinline__ float half_pow_try(float x, int half, bool &ok)
+{
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fadd(x, 1.2e-38f)));
+  const float g = fmul(x, r);
+  const float cr = fmul(fmul(0.5f, r), __fmaf_rn(-g, g, x));
+  float       h = x, l = 0.f;
+  if (half > 3)
+  {
+    h = fmul(x, x);
+    l = __fmaf_rn(x, x, -h);
+    if (half > 5)
+    {
+      const float h3 = fmul(h, x);
+      l = __fmaf_rn(l, x, __fmaf_rn(h, x, -h3));
+      h = h3;
+    }
+  }
+  const float p = fmul(h, g);
+  const float lo = __fmaf_rn(l, g, __fmaf_rn(h, cr, __fmaf_rn(h, g, -p)));
+  const float p1 = fadd(p, __fmaf_rn(p, 0x1p-40f, lo)), p2 = fadd(p, __fmaf_rn(p, -0x1p-40f, lo));
+  ok = p1 == p2 && ((x >= 1e-8f && x <= 1e8f) || x == 0.f);
+  return p1;
+}
+
 /* x^power in fp64, rounded once (header) */
 __device__ __forceinline__ float vf_pow(float xf, const VfConst &c)
 {
   if (c.half == 0) return powr(xf, c.power);
+  if ((c.half & 1) && c.half > 1)
+  {
+    bool        ok;
+    const float p = half_pow_try(xf, c.half, ok);
+    if (ok) return p;
+  }
   const double x = (double)xf, x2 = __dmul_rn(x, x); /* the square is exact */
   double       r = c.half & 4 ? x2 : 1.0;            /* x^2 of 4 .. 7 halves */
   if (c.half == 8) r = __dmul_rn(x2, x2);
