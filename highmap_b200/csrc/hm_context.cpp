@@ -71,6 +71,22 @@ int workspace(hm_context *ctx, size_t bytes, void **out)
   return HM_OK;
 }
 
+void *pinned(hm_context *ctx, size_t bytes)
+{
+  if (ctx->pin_bytes >= bytes) return ctx->pin;
+  if (ctx->pin) cudaFreeHost(ctx->pin);
+  ctx->pin = nullptr;
+  ctx->pin_bytes = 0;
+  if (cudaHostAlloc(&ctx->pin, bytes, cudaHostAllocDefault) != cudaSuccess)
+  {
+    cudaGetLastError();
+    ctx->pin = nullptr;
+    return nullptr;
+  }
+  ctx->pin_bytes = bytes;
+  return ctx->pin;
+}
+
 int scratch(hm_context *ctx, size_t bytes, void **out)
 {
   bytes = align_up(bytes ? bytes : 256, 4096);
@@ -164,6 +180,9 @@ int hm_context_trim(hm_context *ctx)
   if (ctx->ws) HM_CUDA_TRY(cudaFree(ctx->ws));
   ctx->ws = nullptr;
   ctx->ws_bytes = 0;
+  if (ctx->pin) HM_CUDA_TRY(cudaFreeHost(ctx->pin));
+  ctx->pin = nullptr;
+  ctx->pin_bytes = 0;
   return HM_OK;
 }
 
@@ -174,6 +193,7 @@ int hm_context_destroy(hm_context *ctx)
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->ws) cudaFree(ctx->ws);
   if (ctx->scratch) cudaFree(ctx->scratch);
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return HM_OK;

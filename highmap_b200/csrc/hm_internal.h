@@ -19,6 +19,9 @@ struct hm_context
   cudaStream_t stream = nullptr; /* stream of the host-pointer calls */
   void        *ws = nullptr;     /* grow-only device workspace       */
   size_t       ws_bytes = 0;
+  void        *pin = nullptr;    /* pinned staging of the host-pointer calls, grow-only up to
+                                  * a few small grids (hm_api.cpp) */
+  size_t       pin_bytes = 0;
   /* small device area for reductions and per-call scalars */
   void        *scratch = nullptr;
   size_t       scratch_bytes = 0;
@@ -41,6 +44,10 @@ int         use_device(int device);
  * previous contents are not preserved across growth.  Growth synchronises
  * the device so no in-flight kernel can still use the old block. */
 int         workspace(hm_context *ctx, size_t bytes, void **out);
+/* Pinned host staging of at least `bytes`, or null where it cannot be had
+ * (the caller then copies from pageable memory).  No copy from or to the
+ * old block may be in flight. */
+void       *pinned(hm_context *ctx, size_t bytes);
 /* Scratch area for reductions (at least `bytes`). */
 int         scratch(hm_context *ctx, size_t bytes, void **out);
 
