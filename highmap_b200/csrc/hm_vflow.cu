@@ -392,9 +392,10 @@ int vflow_core(const float *z, int nx, int ny, float water_height, const float *
   k_vflow_init<<<VF_GRID, VF_NT, 0, s>>>(hA, depth_map, water_height, n, sc, c);
   HM_LAUNCH_CHECK("k_vflow_init");
   /* Steps per launch: 5 up to 1.5 M cells (two launches per time step
-   * update), one above, where the recomputed halo (1.6 x at 5) costs more
-   * than the launches. */
-  const int  per = n <= 1500000 ? VB_TMAX : 1;
+   * update), one above and for the powers that need pow, where the halo's
+   * arithmetic (1.8 x at 5) costs more than the launches (power 2.2,
+   * 224 x 129: 8.9 us per step with 5, 7.4 with one). */
+  const int  per = c.half != 0 && n <= 1500000 ? VB_TMAX : 1;
   auto       al8 = [](const void *p) { return ((uintptr_t)p & 7u) == 0; };
   float     *cur = hA, *nxt = hB;
   for (int it = 0; it < iterations;)
