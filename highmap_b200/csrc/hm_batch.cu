@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(BT, BATCH_CTAS_PER_SM)
   __shared__ FweIo   s_io;
   __shared__ VpConst s_c;
   __shared__ int     s_step;
+  chain_wait(); /* the round before has written the jobs' grids */
   int                next = PERSIST ? (threadIdx.x == 0 ? (int)atomicAdd(counter, 1u) : 0) : (int)blockIdx.x;
   for (;;)
   {
@@ -541,25 +542,13 @@ int launch_rounds(hm_batch *b, const Plan &pl)
       while (m > 0 && pl.rem[m - 1] <= r) m--;
       const size_t iv = tl.vcum[m], it = tl.tcum[m];
       const int total = (int)(iv + it);
-      if (b->one_tile)
-      {
-        const int grid = std::max(1, total);
-        if (tl.generic)
-          hm::k_batch_round<hm::FWE_GENERIC, false><<<grid, hm::BT, 0, b->stream>>>(
-              b->d_jobs, b->d_tiles, (int)iv, b->d_tiles + nv, (int)it, b->round + r, nullptr);
-        else
-          hm::k_batch_round<hm::FWE_RTOPTS, false><<<grid, hm::BT, 0, b->stream>>>(
-              b->d_jobs, b->d_tiles, (int)iv, b->d_tiles + nv, (int)it, b->round + r, nullptr);
-        HM_LAUNCH_CHECK("k_batch_round");
-        continue;
-      }
-      const int grid = std::max(1, std::min(tl.generic ? b->grid_cap_gen : b->grid_cap, total));
-      if (tl.generic)
-        hm::k_batch_round<hm::FWE_GENERIC, true><<<grid, hm::BT, 0, b->stream>>>(
-            b->d_jobs, b->d_tiles, (int)iv, b->d_tiles + nv, (int)it, b->round + r, b->d_counters + r);
-      else
-        hm::k_batch_round<hm::FWE_RTOPTS, true><<<grid, hm::BT, 0, b->stream>>>(
-            b->d_jobs, b->d_tiles, (int)iv, b->d_tiles + nv, (int)it, b->round + r, b->d_counters + r);
+      const int grid = std::max(1, b->one_tile ? total : std::min(tl.generic ? b->grid_cap_gen : b->grid_cap, total));
+      auto      kernel = b->one_tile ? (tl.generic ? hm::k_batch_round<hm::FWE_GENERIC, false>
+                                                   : hm::k_batch_round<hm::FWE_RTOPTS, false>)
+                                     : (tl.generic ? hm::k_batch_round<hm::FWE_GENERIC, true>
+                                                   : hm::k_batch_round<hm::FWE_RTOPTS, true>);
+      hm::chain_launch(r > 0, kernel, dim3(grid), dim3(hm::BT), b->stream, b->d_jobs, b->d_tiles, (int)iv,
+                       b->d_tiles + nv, (int)it, b->round + r, b->one_tile ? nullptr : b->d_counters + r);
       HM_LAUNCH_CHECK("k_batch_round");
     }
   }
@@ -911,35 +900,51 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
   hm_batch *b = nullptr;
   int       st = hm_batch_create(ctx, &b);
   if (st) return st;
-  /* Jobs of at least HM_BATCH_LARGE_CELLS cells fill the GPU on their
-   * own, and the plain step kernels (specialised on the step's
-   * options, TMA staging, five CTAs per SM) run them faster than the
-   * batch's generic tiles.  They go through the plain solvers on
-   * HM_BATCH_LANES side streams, each lane's jobs one after another, the
-   * lanes balanced by cell-updates (longest first onto the least loaded
-   * lane), beside the rounds of the smaller jobs.  The lanes are launched
-   * directly, before the rounds are captured, so they run while the graph
-   * is built; the batch stream joins them at the end.  On the 256-job mix
-   * of the batched benchmark, 2^20 cells and one lane ran 1.41x plain
-   * per-job calls; 2^18 and three lanes 1.34x, 2^20 and three lanes 1.29x,
-   * 2^18 and one lane 1.12x (bit-identical results in every case). */
+  /* Jobs that the plain solvers run faster than the batch's generic tiles
+   * go through them on side streams (lanes), each lane's jobs one after
+   * another, the lanes balanced by cell-updates (longest first onto the
+   * least loaded lane), beside the rounds of the other jobs.  The lanes are
+   * launched directly, before the rounds are captured, so they run while
+   * the graph is built; the batch stream joins them at the end.
+   *
+   * Jobs of at least HM_BATCH_LARGE_CELLS cells always go there.  Batches of
+   * at least LANES_MIN_S of plain-solver time (their cell-updates at the
+   * rates of large grids) use LANES lanes and send virtual-pipes jobs of at
+   * least LANES_VP_CELLS cells and all thermal jobs (several steps per
+   * launch) there too; smaller batches would spend more on the streams than
+   * they win.  48 jobs of 128 .. 1024 a side, up to 200 steps: the device
+   * work 14.8 ms with one lane from 2^20 cells, 10.8 ms this way (2^18 and 3
+   * lanes 12.9, 2^16 and 8 lanes 13.8). */
+  constexpr int       LANES = 4;
+  constexpr long long LANES_VP_CELLS = 1 << 17;
+  constexpr double    LANES_MIN_S = 4e-3;
+  double              plain_s = 0.0;
+  for (int k = 0; k < njobs; k++)
+    plain_s += (double)jobs[k].nx * jobs[k].ny * std::max(jobs[k].iterations, 0) /
+               (jobs[k].kind == HM_JOB_VPIPES ? 6e10 : 3e11);
+  const bool spread = plain_s >= LANES_MIN_S;
   struct Lane
   {
-    std::vector<int> jobs;
+    int              jobs = 0;
     size_t           bytes = 0;
     double           work = 0.0;
     void            *mem = nullptr;
     cudaStream_t     s = nullptr;
     cudaEvent_t      join = nullptr;
   };
-  Lane             lanes[HM_BATCH_LANES];
+  static_assert(HM_BATCH_LANES <= LANES, "room for the lanes");
+  Lane             lanes[LANES];
+  const int        nlanes = spread ? LANES : HM_BATCH_LANES;
   std::vector<int> large;
+  std::vector<Lane *> lane_of; /* of large[q] */
   int              maxit = 0;
   for (int k = 0; k < njobs && !st; k++)
   {
     const hm_job &j = jobs[k];
     if ((st = check_job(j))) break;
-    if ((long long)j.nx * j.ny >= HM_BATCH_LARGE_CELLS && j.iterations > 0)
+    const long long cells = (long long)j.nx * j.ny;
+    if (j.iterations > 0 && (cells >= HM_BATCH_LARGE_CELLS ||
+                             (spread && (j.kind == HM_JOB_THERMAL || cells >= LANES_VP_CELLS))))
     {
       large.push_back(k);
       continue;
@@ -954,10 +959,11 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
   for (int k : large)
   {
     Lane *l = &lanes[0];
-    for (Lane &c : lanes)
-      if (c.work < l->work) l = &c;
+    for (int c = 1; c < nlanes; c++)
+      if (lanes[c].work < l->work) l = &lanes[c];
     const hm_job &j = jobs[k];
-    l->jobs.push_back(k);
+    l->jobs++;
+    lane_of.push_back(l);
     l->work += work(k);
     l->bytes = std::max(l->bytes, j.kind == HM_JOB_THERMAL
                                       ? hm::thermal_scratch_floats(j.nx, j.ny, j.deposition_map != nullptr) * sizeof(float)
@@ -970,7 +976,7 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
     cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
     for (Lane &l : lanes)
     {
-      if (l.jobs.empty() || e != cudaSuccess) continue;
+      if (l.jobs == 0 || e != cudaSuccess) continue;
       e = cudaMallocFromPoolAsync(&l.mem, l.bytes, b->pool, b->stream);
       if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l.s, cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.join, cudaEventDisableTiming);
@@ -988,37 +994,37 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
     if (large.empty()) return HM_OK;
     HM_CUDA_TRY(cudaEventRecord(fork, b->stream));
     for (Lane &l : lanes)
+      if (l.jobs) HM_CUDA_TRY(cudaStreamWaitEvent(l.s, fork, 0));
+    /* job by job, so that all lanes start early */
+    for (size_t q = 0; q < large.size(); q++)
     {
-      if (l.jobs.empty()) continue;
-      HM_CUDA_TRY(cudaStreamWaitEvent(l.s, fork, 0));
-      for (int k : l.jobs)
+      const hm_job &j = jobs[large[q]];
+      Lane         &l = *lane_of[q];
+      int           rc;
+      if (j.kind == HM_JOB_THERMAL)
       {
-        const hm_job &j = jobs[k];
-        int           rc;
-        if (j.kind == HM_JOB_THERMAL)
-        {
-          hm_thermal_options o;
-          hm_thermal_default_options(&o);
-          o.bedrock_mode = j.bedrock_mode;
-          rc = hm::thermal_core(b->device, j.z, j.nx, j.ny, j.talus, j.talus_value, j.iterations, j.bedrock,
-                                j.deposition_map, nullptr, &o, (float *)l.mem, l.s);
-        }
-        else
-        {
-          hm_vpipes_params p = j.vpipes;
-          p.iterations = j.iterations;
-          rc = hm::vpipes_core(j.z, j.nx, j.ny, p, j.rain_map, j.water_depth, j.sediment, j.vel_u, j.vel_v, l.mem,
-                               l.s, hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations));
-        }
-        if (rc) return rc;
+        hm_thermal_options o;
+        hm_thermal_default_options(&o);
+        o.bedrock_mode = j.bedrock_mode;
+        rc = hm::thermal_core(b->device, j.z, j.nx, j.ny, j.talus, j.talus_value, j.iterations, j.bedrock,
+                              j.deposition_map, nullptr, &o, (float *)l.mem, l.s);
       }
-      HM_CUDA_TRY(cudaEventRecord(l.join, l.s));
+      else
+      {
+        hm_vpipes_params p = j.vpipes;
+        p.iterations = j.iterations;
+        rc = hm::vpipes_core(j.z, j.nx, j.ny, p, j.rain_map, j.water_depth, j.sediment, j.vel_u, j.vel_v, l.mem, l.s,
+                             hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations));
+      }
+      if (rc) return rc;
     }
+    for (Lane &l : lanes)
+      if (l.jobs) HM_CUDA_TRY(cudaEventRecord(l.join, l.s));
     return HM_OK;
   };
   auto join_large = [&]() -> int {
     for (Lane &l : lanes)
-      if (!l.jobs.empty()) HM_CUDA_TRY(cudaStreamWaitEvent(b->stream, l.join, 0));
+      if (l.jobs) HM_CUDA_TRY(cudaStreamWaitEvent(b->stream, l.join, 0));
     return HM_OK;
   };
   if (!st && use_graph && maxit > 0)
