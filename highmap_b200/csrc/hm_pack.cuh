@@ -36,6 +36,7 @@ __device__ __forceinline__ F2 pk(float a, float b)
   asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
   return r;
 }
+__device__ __forceinline__ F2    pk(float2 a) { return pk(a.x, a.y); }
 __device__ __forceinline__ F2    pk1(float a) { return pk(a, a); }
 __device__ __forceinline__ float2 up(F2 p)
 {

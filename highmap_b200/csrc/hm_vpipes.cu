@@ -289,6 +289,7 @@ VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p)
   c.keep = 1.f - p.dt * p.evap_rate;
   c.rps = p.rain_per_step;
   c.fnx = (float)nx;
+  c.nz = -0.f;
   return c;
 }
 

@@ -19,6 +19,8 @@
 #ifndef HM_VPIPES_MATH_CUH
 #define HM_VPIPES_MATH_CUH
 
+#include "hm_pack.cuh"
+
 namespace hm
 {
 
@@ -124,6 +126,7 @@ struct VpConst
   float keep;        /* 1 - dt * evap_rate                              */
   float rps;         /* rain per step                                   */
   float fnx;         /* (float)nx, the slope scale of :156              */
+  float nz;          /* -0, unknown to the compiler (mul2r)              */
 };
 
 /* Depth at the start of a step: the stored evaporated depth, plus the
@@ -251,6 +254,129 @@ __device__ __forceinline__ void erosion_cell(const VpConst &c,
   T m = fmul(capa > sc ? bc<T>(c.k_erode) : bc<T>(c.k_depose), fsub(capa, sc));
   z_out = fsub(zc, m);
   s_out = fadd(sc, m);
+}
+
+/* ---- two adjacent cells in packed arithmetic (hm_pack.cuh) ------------
+ * Pipe length and discharge exponent 1: the scalar passes operation by
+ * operation, divisions and selects per half.  The step is bound by issue
+ * slots (77 % busy at 2048 x 2048), and a packed operation takes one slot
+ * for two cells: 100 steps with rain 24.5 -> 23.6 ms at 4096 x 4096, 6.70 ->
+ * 6.55 ms at 2048 x 2048; with the top-up 33.0 -> 32.6 ms.  The step kernel
+ * has no register to spare (48): the first two hypots of the erosion pass
+ * stay per cell, because packed they cost spills and 10 % of the step. */
+
+__device__ __forceinline__ F2 max2n(float a, F2 b)
+{
+  const float2 v = up(b);
+  return pk(rmaxn(a, v.x), rmaxn(a, v.y));
+}
+
+/* flow_cell for a pair; w and e are the pairs one column to the west and
+ * to the east */
+template <bool DIFFUSION>
+__device__ __forceinline__ void flow_pair(const VpConst &c, F2 zc, F2 d1c, F2 zw, F2 d1w, F2 ze, F2 d1e, F2 zs, F2 d1s,
+                                          F2 zn, F2 d1n, F2 &fl, F2 &fr, F2 &ft, F2 &fb)
+{
+  const F2 nz = pk1(c.nz), dtga = pk1(c.dtga);
+  const F2 h0 = add2(zc, d1c);
+  F2 nl = max2n(0.f, add2(fl, mul2r(dtga, sub2(sub2(h0, zw), d1w), nz)));
+  F2 nr = max2n(0.f, add2(fr, mul2r(dtga, sub2(sub2(h0, ze), d1e), nz)));
+  F2 nt = max2n(0.f, add2(ft, mul2r(dtga, sub2(sub2(h0, zs), d1s), nz)));
+  F2 nb = max2n(0.f, add2(fb, mul2r(dtga, sub2(sub2(h0, zn), d1n), nz)));
+  if (DIFFUSION)
+  {
+    const F2 c1 = pk1(c.c1);
+    const F2 f_diff = mul2r(pk1(c.c0), add2(add2(add2(nl, nr), nt), nb), nz);
+    nl = add2(mul2r(c1, nl, nz), f_diff);
+    nr = add2(mul2r(c1, nr, nz), f_diff);
+    nt = add2(mul2r(c1, nt, nz), f_diff);
+    nb = add2(mul2r(c1, nb, nz), f_diff);
+  }
+  const F2     sum2 = add2(add2(add2(nl, nr), nt), nb);
+  const float2 sum = up(sum2), den = up(mul2(sum2, pk1(c.dt))), d = up(d1c);
+  const bool   wx = sum.x > 1e-5f, wy = sum.y > 1e-5f;
+  const float  qx = __saturatef(fdiv(d.x, wx ? den.x : 1.f)), qy = __saturatef(fdiv(d.y, wy ? den.y : 1.f));
+  const F2     k = pk(wx ? qx : 0.f, wy ? qy : 0.f);
+  fl = mul2(nl, k);
+  fr = mul2(nr, k);
+  ft = mul2(nt, k);
+  fb = mul2(nb, k);
+}
+
+/* water_cell for a pair */
+__device__ __forceinline__ void water_pair(const VpConst &c, F2 d1c, F2 flc, F2 frc, F2 ftc, F2 fbc, F2 frw, F2 fle,
+                                           F2 ftn, F2 fbs, F2 &d2, F2 &u, F2 &v)
+{
+  const F2 in = add2(add2(add2(frw, ftn), fle), fbs);
+  d2 = max2n(0.f, add2(d1c, mul2r(pk1(c.dt), sub2(sub2(sub2(sub2(in, flc), frc), ftc), fbc), pk1(c.nz))));
+  const float2 un = up(mul2(pk1(0.5f), sub2(add2(sub2(frw, flc), frc), fle)));
+  const float2 vn = up(mul2(pk1(0.5f), sub2(add2(sub2(ftn, fbc), ftc), fbs)));
+  const float2 dm = up(max2n(c.vel_floor, d2));
+  u = pk(fdiv(un.x, dm.x), fdiv(un.y, dm.y));
+  v = pk(fdiv(vn.x, dm.x), fdiv(vn.y, dm.y));
+}
+
+/* hyp_try for a pair */
+__device__ __forceinline__ F2 hyp_try2(F2 x2, F2 y2, F2 nz, bool &ok, F2 &rinv)
+{
+  const float2 x = up(x2), y = up(y2);
+  float        a0, a1, b0, b1;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(a0) : "f"(fabsf(x.x)), "f"(fabsf(y.x)));
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(a1) : "f"(fabsf(x.y)), "f"(fabsf(y.y)));
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(b0) : "f"(fabsf(x.x)), "f"(fabsf(y.x)));
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(b1) : "f"(fabsf(x.y)), "f"(fabsf(y.y)));
+  const F2 a = pk(a0, a1), b = pk(b0, b1), m1 = pk1(-1.f);
+  const F2 p = mul2r(a, a, nz);
+  const F2 s = fma2(b, b, p);
+  const F2 e = add2(fma2(b, b, sub2(p, s)), fma2(a, a, mul2(p, m1)));
+  const float2 st = up(add2(s, pk1(1.2e-38f)));
+  float        r0, r1;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(st.x));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(st.y));
+  const F2     r = pk(r0, r1);
+  const F2     g = mul2(s, r);
+  const F2     d = add2(fma2(mul2(g, m1), g, s), e);
+  const F2     l2 = fma2(d, mul2(r, pk1(0.5f * (1.f - 1e-5f))), g);
+  const float2 lo = up(l2), hi = up(fma2(d, mul2(r, pk1(0.5f * (1.f + 1e-5f))), g));
+  ok = ok && lo.x == hi.x && lo.y == hi.y && __float_as_uint(a0) - 1u >= 0x26901d7cu &&
+       __float_as_uint(a1) - 1u >= 0x26901d7cu;
+  rinv = r;
+  return l2;
+}
+
+/* erosion_cell for a pair */
+__device__ __forceinline__ void erosion_pair(const VpConst &c, F2 zc, F2 sc, F2 zw, F2 ze, F2 zn, F2 zs, F2 sw, F2 se,
+                                             F2 sn, F2 ss, F2 d2, F2 u, F2 v, F2 &z_out, F2 &s_out)
+{
+  const F2 nz = pk1(c.nz), half = pk1(0.5f);
+  const F2 dzx = mul2(half, sub2(add2(sub2(ze, zw), se), sw));
+  const F2 dzy = mul2(half, sub2(add2(sub2(zs, zn), ss), sn));
+  bool     ok = true;
+  float    r0, r1;
+  F2       r;
+  F2       speed = pk(hyp_try(lo(u), lo(v), ok, r0), hyp_try(hi(u), hi(v), ok, r1));
+  F2       dzn = max2n(1e-3f, mul2(pk1(c.fnx), pk(hyp_try(lo(dzx), lo(dzy), ok, r0), hyp_try(hi(dzx), hi(dzy), ok, r1))));
+  const F2 h = hyp_try2(pk1(1.f), dzn, nz, ok, r);
+  /* div_hyp */
+  const F2 nh = mul2(h, pk1(-1.f));
+  r = fma2(r, fma2(nh, r, pk1(1.f)), r);
+  F2 sa = mul2(dzn, r);
+  sa = fma2(fma2(nh, sa, dzn), r, sa);
+  if (!ok)
+  {
+    const float2 uu = up(u), vv = up(v), gx = up(dzx), gy = up(dzy);
+    speed = pk(hyp(uu.x, vv.x), hyp(uu.y, vv.y));
+    const float n0 = rmaxn(1e-3f, fmul(c.fnx, hyp(gx.x, gy.x))), n1 = rmaxn(1e-3f, fmul(c.fnx, hyp(gx.y, gy.y)));
+    sa = pk(fdiv(n0, hyp(1.f, n0)), fdiv(n1, hyp(1.f, n1)));
+  }
+  const float2 d = up(d2);
+  const F2     depth = pk(rmin(fdiv_z(d.x, c.water_height), c.ratio), rmin(fdiv_z(d.y, c.water_height), c.ratio));
+  const F2     capa = mul2r(mul2(pk1(c.k_capacity), mul2(depth, speed)), max2n(0.01f, sa), nz);
+  const float2 cp = up(capa), s = up(sc);
+  const F2     kk = pk(cp.x > s.x ? c.k_erode : c.k_depose, cp.y > s.y ? c.k_erode : c.k_depose);
+  const F2     m = mul2r(kk, sub2(capa, sc), nz);
+  z_out = sub2(zc, m);
+  s_out = add2(sc, m);
 }
 
 /* Mirror an unnormalised coordinate with period 2 * n (texel units):

@@ -695,8 +695,25 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
         const float  zw = sm.z[q][cc - 1], dw = sm.d[q][cc - 1], ze = sm.z[q][cc + 2], de = sm.d[q][cc + 2];
         float2       fl = lds2(&sm.fo[0][l][cc]), fr = lds2(&sm.fo[1][l][cc]), ft = lds2(&sm.fo[2][l][cc]),
                fb = lds2(&sm.fo[3][l][cc]);
-        flow1(zc.x, dc.x, zw, dw, zc.y, dc.y, zs.x, ds.x, zn.x, dn.x, fl.x, fr.x, ft.x, fb.x);
-        flow1(zc.y, dc.y, zc.x, dc.x, ze, de, zs.y, ds.y, zn.y, dn.y, fl.y, fr.y, ft.y, fb.y);
+        if (GEN) /* the packed forms take pipe length and exponent 1 */
+        {
+          flow1(zc.x, dc.x, zw, dw, zc.y, dc.y, zs.x, ds.x, zn.x, dn.x, fl.x, fr.x, ft.x, fb.x);
+          flow1(zc.y, dc.y, zc.x, dc.x, ze, de, zs.y, ds.y, zn.y, dn.y, fl.y, fr.y, ft.y, fb.y);
+        }
+        else
+        {
+          F2 l2 = pk(fl), r2 = pk(fr), t2 = pk(ft), b2 = pk(fb);
+          if (diffusion)
+            flow_pair<true>(c, pk(zc), pk(dc), pk(zw, zc.x), pk(dw, dc.x), pk(zc.y, ze), pk(dc.y, de), pk(zs), pk(ds),
+                            pk(zn), pk(dn), l2, r2, t2, b2);
+          else
+            flow_pair<false>(c, pk(zc), pk(dc), pk(zw, zc.x), pk(dw, dc.x), pk(zc.y, ze), pk(dc.y, de), pk(zs), pk(ds),
+                             pk(zn), pk(dn), l2, r2, t2, b2);
+          fl = up(l2);
+          fr = up(r2);
+          ft = up(t2);
+          fb = up(b2);
+        }
         sts2(&sm.fn[0][l][cc], fl.x, fl.y);
         sts2(&sm.fn[1][l][cc], fr.x, fr.y);
         sts2(&sm.fn[2][l][cc], ft.x, ft.y);
@@ -718,9 +735,9 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
 
     /* water and erosion on the tile: thread t takes row t / 16 and the pair
      * of tile columns 2 (t % 16), 2 (t % 16) + 1 */
-    const int ty = tid >> 4, pk = tid & 15;
-    const int gy = y0 + ty, gx = x0 + 2 * pk;
-    const int cc = 4 + 2 * pk; /* smem column of the first cell */
+    const int ty = tid >> 4, pr = tid & 15;
+    const int gy = y0 + ty, gx = x0 + 2 * pr;
+    const int cc = 4 + 2 * pr; /* smem column of the first cell */
     if (INNER || (gx < nx && gy < ny))
     {
       const bool second = INNER || gx + 1 < nx;
@@ -738,7 +755,14 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
       const float  frw0 = sm.fn[1][l][cw0], fle0 = sm.fn[0][l][ce0], fle1 = sm.fn[0][l][ce1];
       const float2 d1 = lds2(&sm.d[q][cc]);
       float        d2a, ua, va, d2b, ub, vb;
-      if (pl_one)
+      if (!GEN)
+      {
+        F2 d2, u, v;
+        water_pair(c, pk(d1), pk(flc), pk(frc), pk(ftc), pk(fbc), pk(frw0, frc.x), pk(fle0, fle1), pk(ftn), pk(fbs), d2,
+                   u, v);
+        d2a = lo(d2), d2b = hi(d2), ua = lo(u), ub = hi(u), va = lo(v), vb = hi(v);
+      }
+      else if (pl_one)
       {
         water_cell<true>(c, d1.x, flc.x, frc.x, ftc.x, fbc.x, frw0, fle0, ftn.x, fbs.x, d2a, ua, va);
         water_cell<true>(c, d1.y, flc.y, frc.y, ftc.y, fbc.y, frc.x, fle1, ftn.y, fbs.y, d2b, ub, vb);
@@ -800,7 +824,14 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
         const float2 s0 = lds2(&sm.s[l][cc]), sn = lds2(&sm.s[l - 1][cc]), ss = lds2(&sm.s[l + 1][cc]);
         const float  sw = sm.s[l][cc - 1], se = sm.s[l][cc + 2];
         float        zoa, soa, zob, sob;
-        if (kexp_one)
+        if (!GEN)
+        {
+          F2 zo, so;
+          erosion_pair(c, pk(zc), pk(s0), pk(zw, zc.x), pk(zc.y, ze), pk(zn), pk(zs), pk(sw, s0.x), pk(s0.y, se), pk(sn),
+                       pk(ss), pk(d2a, d2b), pk(ua, ub), pk(va, vb), zo, so);
+          zoa = lo(zo), zob = hi(zo), soa = lo(so), sob = hi(so);
+        }
+        else if (kexp_one)
         {
           erosion_cell<true>(c, zc.x, s0.x, zw, zc.y, zn.x, zs.x, sw, s0.y, sn.x, ss.x, d2a, ua, va, zoa, soa);
           erosion_cell<true>(c, zc.y, s0.y, zc.x, ze, zn.y, zs.y, s0.x, se, sn.y, ss.y, d2b, ub, vb, zob, sob);
