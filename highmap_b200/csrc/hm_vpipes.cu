@@ -110,11 +110,15 @@ __global__ void __launch_bounds__(VP_NT) k_vp_init_finish(VpScalars *sc, const d
   }
 }
 
-/* the last step's top-up, for the water-depth output, from the water per
- * tile (FweIo) */
+/* a step's top-up from the water per tile (FweIo): between the steps of
+ * grids of more than SUM_TILES_MAX tiles, and for the water-depth output
+ * after the last step of smaller ones.  It triggers before it waits: only
+ * the next step can start then, whose CTAs wait for this one. */
 __global__ void __launch_bounds__(FT_NT) k_vp_top_up(const double *tiles, unsigned n, VpScalars *sc, int parity)
 {
-  const float add = tiles_top_up(tiles, n, sc);
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const float add = tiles_top_up(produced(tiles), n, sc);
   if (threadIdx.x == 0) sc->add[parity] = add;
 }
 
@@ -493,7 +497,7 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     if (io.u_out && !io.v_out) io.v_out = io.v;
     if (io.v_out && !io.u_out) io.u_out = io.u;
     io.parity = parity;
-    io.sum_out = direct_sum ? sums[it & 1] : nullptr;
+    io.sum_out = sums[it & 1];
     io.sum_in = direct_sum && it > 0 ? sums[(it & 1) ^ 1] : nullptr;
     const FweMaps &mp = maps[cur == &A ? 0 : 1];
     int            rc;
@@ -503,6 +507,11 @@ static int vpipes_tiled_steps(float *z, int nx, int ny, const hm_vpipes_params &
     else rc = tma ? launch_fwe_tma(io, mp, c, sc, partials, g1, s, false)
                   : launch_fwe_cp_async(io, c, sc, partials, g1, s, false);
     if (rc) return rc;
+    if (io.maintain && !direct_sum && (!last || water_depth))
+    {
+      chain_launch(true, k_vp_top_up, 1, FT_NT, s, sums[it & 1], g1.x * g1.y, sc, parity ^ 1);
+      HM_LAUNCH_CHECK("k_vp_top_up");
+    }
     /* the advection of this step is folded into the next step's tiles; the
      * last step's runs here */
     if (last)

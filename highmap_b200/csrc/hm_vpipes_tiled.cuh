@@ -144,18 +144,22 @@ struct FweIo
   unsigned     tma_extra_tx;  /* bytes a TMA tile's barrier expects beyond its boxes: 0, or the
                                * test hook's count, which makes every tile's wait run out */
   const float *s1_prev;       /* k_vp_step(_tma): the previous step's eroded sediment */
-  /* Volume top-up: the step before's water per tile, which every CTA of
-   * this step sums for itself while its boxes are in flight, and this
-   * step's; null: sc->add and the last-CTA finish (grid_sum_commit). */
+  /* Volume top-up: sum_in the step before's water per tile, which every CTA
+   * of this step sums for itself while its boxes are in flight (null: the
+   * top-up is in sc->add); sum_out this step's (null: the last-CTA finish,
+   * grid_sum_commit, of steps that are not launches of their own). */
   const double *sum_in;
   double       *sum_out;
 };
 
-/* Most tiles of a grid whose steps sum the tiles' water themselves.  The
- * last-CTA finish costs a fence and an atomic round trip at the end of
- * every CTA (2300 of 9200 cycles at 256^2); the sum costs a load per 256
- * tiles and thread, hidden behind the staging wait, but its traffic grows
- * with the square of the tiles (33 MB of L2 reads per step at 2048). */
+/* Most tiles of a grid whose steps sum the tiles' water themselves; above,
+ * one CTA sums it between two steps (k_vp_top_up).  Either way a tile only
+ * stores its sum: the last-CTA finish costs a fence and an atomic round
+ * trip at the end of every CTA (2300 of 9200 cycles at 256^2; 100 steps with the defaults at 4096 x
+ * 4096 32.3 -> 28.1 ms, at 2048 x 2048 8.75 -> 7.75 ms).
+ * Summing in the step costs a load per 256 tiles and thread, hidden behind
+ * the staging wait, but its traffic grows with the square of the tiles (33
+ * MB of L2 reads per step at 2048). */
 constexpr unsigned SUM_TILES_MAX = 2048;
 
 /* The top-up of this step from the water per tile: the sum of
@@ -165,7 +169,16 @@ __device__ __forceinline__ float tiles_top_up(const double *tiles, unsigned n, c
   __shared__ double sm[FT_NT / 32];
   __shared__ float  s_add;
   double            acc = 0.0;
-  for (unsigned k = threadIdx.x; k < n; k += FT_NT) acc += tiles[k];
+  /* eight loads at a time in flight (a missing one adds +0, the identity):
+   * 100 steps at 1023 x 767 2.10 -> 2.00 ms against one at a time */
+  for (unsigned k = threadIdx.x; k < n; k += 8 * FT_NT)
+  {
+    double v[8];
+#pragma unroll
+    for (unsigned j = 0; j < 8; j++) v[j] = k + j * FT_NT < n ? tiles[k + j * FT_NT] : 0.0;
+#pragma unroll
+    for (unsigned j = 0; j < 8; j++) acc += v[j];
+  }
   const double total = block_sum<FT_NT>(acc, sm);
   if (threadIdx.x == 0) s_add = fsub(sc->v0, (float)total);
   __syncthreads();
