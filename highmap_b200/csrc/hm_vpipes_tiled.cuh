@@ -631,9 +631,47 @@ struct NoMid
   __device__ bool operator()() const { return true; }
 };
 
+/* The rain map on region 2, staged beside the wait for the boxes: read where
+ * the depth pass needs it, its latency stood in the way of every tile
+ * (100 steps with a rain map at 4096 x 4096 36.3 -> 30.8 ms, at 2048 x 2048
+ * 9.66 -> 8.15 ms, at 1023 x 767 2.16 -> 2.09 ms).  A thread reads back the
+ * pairs it has stored. */
+template <bool MAINTAIN, int F>
+struct RainStage
+{
+  static constexpr bool USED = MAINTAIN && (F & (FWE_GENERIC | FWE_RTOPTS)) == 0 && (F & FWE_RAINMAP) != 0;
+  static constexpr int  N = 18 * FT_H2, PER = (N + FT_NT - 1) / FT_NT;
+  float2                pair[USED ? N : 1];
+  /* between() runs with the loads in flight */
+  template <class Between>
+  __device__ __forceinline__ void load(const FweIo &io, const VpConst &c, int x0, int y0, Between between)
+  {
+    float2 r[PER];
+    if (USED)
+    {
+#pragma unroll
+      for (int k = 0; k < PER; k++)
+      {
+        const int    e = min((int)threadIdx.x + k * FT_NT, N - 1), q = e / 18, x = x0 - 2 + 2 * (e - q * 18);
+        const size_t row = (size_t)clampi(y0 - 2 + q, 0, c.ny - 1) * c.nx;
+        r[k].x = __ldg(io.rain + row + clampi(x, 0, c.nx - 1));
+        r[k].y = __ldg(io.rain + row + clampi(x + 1, 0, c.nx - 1));
+      }
+    }
+    between();
+    if (USED)
+    {
+#pragma unroll
+      for (int k = 0; k < PER; k++)
+        if ((int)threadIdx.x + k * FT_NT < N) pair[threadIdx.x + k * FT_NT] = r[k];
+    }
+  }
+};
+
 template <bool MAINTAIN, int F, bool INNER = false, class Mid = NoMid>
 __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, VpScalars *sc, double *partials,
-                                            float add, int bx, int by, int nbx, int nby, FweSmem &sm, Mid mid = Mid())
+                                            float add, int bx, int by, int nbx, int nby, FweSmem &sm, Mid mid = Mid(),
+                                            const RainStage<MAINTAIN, F> *rain = nullptr)
 {
   static_assert(FT_TX == 32 && FT_TY == 16 && FT_NT == 256, "one cell pair per thread in the water pass");
   constexpr bool GEN = (F & FWE_GENERIC) != 0;
@@ -656,7 +694,12 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
     const int q = e / 18, cc = 2 + 2 * (e - q * 18);
     float2    dd = lds2(&sm.d[q][cc]);
     float     r0 = 1.f, r1 = 1.f;
-    if (rain_map)
+    if (RainStage<MAINTAIN, F>::USED)
+    {
+      r0 = rain->pair[e].x;
+      r1 = rain->pair[e].y;
+    }
+    else if (rain_map)
     {
       const size_t row = (size_t)clampi(y0 - 2 + q, 0, ny - 1) * nx;
       r0 = __ldg(io.rain + row + clampi(x0 - 4 + cc, 0, nx - 1));
@@ -875,15 +918,19 @@ __device__ __forceinline__ bool fwe_inner_tile(const FweIo &io, int nx, int ny, 
 template <bool MAINTAIN, int F>
 __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F)) k_vp_fwe(FweIo io, VpConst c, VpScalars *sc, double *partials)
 {
-  __shared__ FweSmem sm;
+  __shared__ FweSmem                sm;
+  __shared__ RainStage<MAINTAIN, F> rain;
+  rain.load(io, c, blockIdx.x * FT_TX, blockIdx.y * FT_TY, [] {});
   chain_wait();
   fwe_stage_cp_async(io, c.nx, c.ny, c.ld, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm);
   __syncthreads();
   const float add = MAINTAIN ? sc->add[io.parity] : 0.f;
   if (fwe_inner_tile(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY))
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, NoMid(), &rain);
   else
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, NoMid(), &rain);
 }
 
 /* The same step with the input tiles fetched by TMA.  A tile whose loads
@@ -894,7 +941,9 @@ template <bool MAINTAIN, int F>
 __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
     k_vp_fwe_tma(FweIo io, const __grid_constant__ FweMaps maps, VpConst c, VpScalars *sc, double *partials)
 {
-  __shared__ FweSmem sm;
+  __shared__ FweSmem                sm;
+  __shared__ RainStage<MAINTAIN, F> rain;
+  rain.load(io, c, blockIdx.x * FT_TX, blockIdx.y * FT_TY, [] {});
   if (!fwe_stage_tma<(F & FWE_FLOWONLY) == 0>(maps, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY, sm, io.tma_extra_tx))
   {
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
@@ -904,9 +953,11 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   }
   const float add = MAINTAIN ? sc->add[io.parity] : 0.f;
   if (fwe_inner_tile(io, c.nx, c.ny, blockIdx.x * FT_TX, blockIdx.y * FT_TY))
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, NoMid(), &rain);
   else
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, NoMid(), &rain);
 }
 
 /* A step after the first with cp.async staging (grids the TMA rules
@@ -918,7 +969,9 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
     k_vp_step(FweIo io, const float *u_prev, const float *v_prev, VpConst c,
               VpScalars *sc, double *partials)
 {
-  __shared__ FweSmem sm;
+  __shared__ FweSmem                sm;
+  __shared__ RainStage<MAINTAIN, F> rain;
+  rain.load(io, c, blockIdx.x * FT_TX, blockIdx.y * FT_TY, [] {});
   chain_wait();
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
   float     add = 0.f;
@@ -932,12 +985,14 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   if (fwe_inner_tile(io, c.nx, c.ny, x0, y0))
   {
     advect_region1<true>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, NoMid(), &rain);
   }
   else
   {
     advect_region1<false>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, NoMid(), &rain);
   }
 }
 
@@ -949,11 +1004,14 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
     k_vp_step_tma(FweIo io, const __grid_constant__ FweMaps maps, const __grid_constant__ AdvMaps am, VpConst c,
                   VpScalars *sc, double *partials)
 {
-  __shared__ FweSmem sm;
+  __shared__ FweSmem                sm;
+  __shared__ RainStage<MAINTAIN, F> rain;
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
   float     add = 0.f;
   auto      top_up = [&]() {
-    if (MAINTAIN) add = io.sum_in ? tiles_top_up(io.sum_in, gridDim.x * gridDim.y, sc) : sc->add[io.parity];
+    rain.load(io, c, x0, y0, [&] {
+      if (MAINTAIN) add = io.sum_in ? tiles_top_up(io.sum_in, gridDim.x * gridDim.y, sc) : sc->add[io.parity];
+    });
   };
   if (!fwe_stage_tma_step<MAINTAIN>(maps, am, x0, y0, sm, io.tma_extra_tx, top_up))
   {
@@ -971,12 +1029,14 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
   if (fwe_inner_tile(io, c.nx, c.ny, x0, y0))
   {
     advect_region1<true>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm, group_b);
+    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, group_b, &rain);
   }
   else
   {
     advect_region1<false>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, sm, group_b);
+    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+                                  gridDim.x, gridDim.y, sm, group_b, &rain);
   }
 }
 
