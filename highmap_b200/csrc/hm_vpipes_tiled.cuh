@@ -687,6 +687,11 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
   const bool     pl_one = GEN ? io.pl_one != 0 : true;
   const bool     kexp_one = GEN ? io.kexp_one != 0 : true;
 
+  /* the reciprocal of the rain's sum, for the top-up by a rain map */
+  F2         nrvol;
+  const bool rvol_ok = rvol >= 0x1p-40f && rvol <= 0x1p60f;
+  const float y_rvol = MAINTAIN && !GEN ? lo(rcp2(pk1(rvol), nrvol)) : 0.f;
+
   /* with the top-up: stored depth -> depth at the start of the step, region
    * 2 (columns x0-2 .. x0+33 = smem 2 .. 37), 18 pairs per row */
   for (int e = MAINTAIN ? tid : 18 * FT_H2; e < 18 * FT_H2; e += FT_NT)
@@ -705,7 +710,13 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
       r0 = __ldg(io.rain + row + clampi(x0 - 4 + cc, 0, nx - 1));
       r1 = __ldg(io.rain + row + clampi(x0 - 3 + cc, 0, nx - 1));
     }
-    if (rain_step)
+    if (!GEN && rain_map)
+    {
+      F2 d2 = add2(pk(dd), top_up_pair(pk(r0, r1), add, rvol, y_rvol, rvol_ok));
+      if (rain_step) d2 = add2(d2, mul2r(pk1(c.rps), pk(r0, r1), pk1(c.nz)));
+      dd = up(d2);
+    }
+    else if (rain_step)
     {
       dd.x = depth_d1<MAINTAIN, true>(dd.x, r0, add, rvol, c.rps);
       dd.y = depth_d1<MAINTAIN, true>(dd.y, r1, add, rvol, c.rps);
@@ -811,11 +822,12 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
       const float  frw0 = sm.fn[1][l][cw0], fle0 = sm.fn[0][l][ce0], fle1 = sm.fn[0][l][ce1];
       const float2 d1 = lds2(&sm.d[q][cc]);
       float        d2a, ua, va, d2b, ub, vb;
+      F2           depth;
       if (!GEN)
       {
         F2 d2, u, v;
         water_pair(c, pk(d1), pk(flc), pk(frc), pk(ftc), pk(fbc), pk(frw0, frc.x), pk(fle0, fle1), pk(ftn), pk(fbs), d2,
-                   u, v);
+                   u, v, depth);
         d2a = lo(d2), d2b = hi(d2), ua = lo(u), ub = hi(u), va = lo(v), vb = hi(v);
       }
       else if (pl_one)
@@ -884,7 +896,7 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
         {
           F2 zo, so;
           erosion_pair(c, pk(zc), pk(s0), pk(zw, zc.x), pk(zc.y, ze), pk(zn), pk(zs), pk(sw, s0.x), pk(s0.y, se), pk(sn),
-                       pk(ss), pk(d2a, d2b), pk(ua, ub), pk(va, vb), zo, so);
+                       pk(ss), depth, pk(ua, ub), pk(va, vb), zo, so);
           zoa = lo(zo), zob = hi(zo), soa = lo(so), sob = hi(so);
         }
         else if (kexp_one)
