@@ -296,7 +296,7 @@ VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p)
   c.nz = -0.f;
   c.rwh = 1.f / c.water_height;
   const auto in = [](float x, float l, float h) { return x >= l && x <= h; };
-  c.quot_ok = in(c.dt, 0x1p-20f, 0x1p20f) && in(c.water_height, 0x1p-40f, 0x1p60f) && in(c.vel_floor, 0x1p-40f, 0x1p60f);
+  c.quot_ok = in(c.water_height, 0x1p-40f, 0x1p60f) && in(c.vel_floor, 0x1p-40f, 0x1p60f);
   return c;
 }
 

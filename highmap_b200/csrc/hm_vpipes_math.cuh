@@ -128,7 +128,7 @@ struct VpConst
   float fnx;         /* (float)nx, the slope scale of :156              */
   float nz;          /* -0, unknown to the compiler (mul2r)              */
   float rwh;         /* 1 / water_height                                 */
-  int   quot_ok;     /* dt, water_height and vel_floor in quot2's range  */
+  int   quot_ok;     /* water_height and vel_floor in quot2's range      */
 };
 
 /* Depth at the start of a step: the stored evaporated depth, plus the
@@ -341,17 +341,12 @@ __device__ __forceinline__ void flow_pair(const VpConst &c, F2 zc, F2 d1c, F2 zw
     nb = add2(mul2r(c1, nb, nz), f_diff);
   }
   const F2     sum2 = add2(add2(add2(nl, nr), nt), nb);
-  const float2 sum = up(sum2), d = up(d1c);
-  float2       den = up(mul2(sum2, pk1(c.dt)));
+  const float2 sum = up(sum2), den = up(mul2(sum2, pk1(c.dt))), d = up(d1c);
   const bool   wx = sum.x > 1e-5f, wy = sum.y > 1e-5f;
-  den.x = wx ? den.x : 1.f;
-  den.y = wy ? den.y : 1.f;
-  F2       nden;
-  const F2 y = rcp2(pk(den), nden);
-  float2   q = up(quot2(d1c, nden, y));
-  if (!(c.quot_ok && quot_min(quot_min(~0u, d.x), d.y) >= QUOT_MIN && fadd(fadd(d.x, d.y), fadd(den.x, den.y)) < QUOT_MAX))
-    q = make_float2(fdiv(d.x, den.x), fdiv(d.y, den.y));
-  const F2 k = pk(wx ? __saturatef(q.x) : 0.f, wy ? __saturatef(q.y) : 0.f);
+  /* (quot2 gains nothing here, one divisor for one quotient: 100 steps with
+   * the defaults at 1024 x 1056 2.54 ms, divided 2.46) */
+  const float qx = __saturatef(fdiv(d.x, wx ? den.x : 1.f)), qy = __saturatef(fdiv(d.y, wy ? den.y : 1.f));
+  const F2    k = pk(wx ? qx : 0.f, wy ? qy : 0.f);
   fl = mul2(nl, k);
   fr = mul2(nr, k);
   ft = mul2(nt, k);
