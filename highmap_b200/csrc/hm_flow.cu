@@ -9,7 +9,8 @@
  * are the tiled vpipes kernels in their flow-only form (FWE_FLOWONLY:
  * flow, water, no erosion or advection, depth and fluxes written), the
  * state stays in HBM, and the dry-out is a max reduction plus one
- * elementwise pass.
+ * elementwise pass.  Where a tile's boxes fit the grid the steps go in
+ * pairs (hm_flow_steps.cuh).
  *
  * State: depth and the four fluxes in two copies (A, B); the terrain is
  * read in place, or from a copy where its rows miss the TMA rules (the
@@ -20,6 +21,7 @@
 
 #include <cstdint>
 
+#include "hm_flow_steps.cuh"
 #include "hm_internal.h"
 #include "hm_vpipes.h"
 #include "hm_vpipes_tiled.cuh"
@@ -85,6 +87,18 @@ __global__ void k_flow_dry_out(const float *__restrict__ d, const unsigned *__re
 }
 
 } // namespace
+
+/* maps of one state copy for k_flow_steps<T>; false if a box is larger than
+ * the grid (the caller has checked the TMA rules with fwe_maps) */
+template <int T>
+static bool flow_maps(const VpFields &f, int nx, int ny, int ld, FlowMaps *m)
+{
+  using L = FlowTile<T>;
+  if (nx < L::W || ny < L::ZH) return false;
+  auto map = [&](CUtensorMap *q, const float *p, int rows) { return encode_grid_map(q, p, nx, ny, ld, rows, L::W); };
+  return map(&m->z, f.z, L::ZH) && map(&m->d, f.d, L::ZH) && map(&m->fl, f.fl, L::FH) && map(&m->fr, f.fr, L::FH) &&
+         map(&m->ft, f.ft, L::FH) && map(&m->fb, f.fb, L::FH);
+}
 
 static size_t flow_state_floats(int nx, int ny, bool padded)
 {
@@ -163,7 +177,23 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
   const bool tma = fwe_maps(A, nx, ny, ld, &maps[0]) && fwe_maps(B, nx, ny, ld, &maps[1]);
   const dim3 g1((nx + FT_TX - 1) / FT_TX, (ny + FT_TY - 1) / FT_TY);
   VpFields  *cur = &A, *nxt = &B;
-  for (int it = 0; it < iterations; it++)
+  /* FLOW_T steps per launch; the remainder, and grids smaller than their
+   * boxes, a step at a time */
+  FlowMaps   fm[2];
+  const bool blocked = tma && iterations >= FLOW_T && flow_maps<FLOW_T>(A, nx, ny, ld, &fm[0]) &&
+                       flow_maps<FLOW_T>(B, nx, ny, ld, &fm[1]);
+  int        it = 0;
+  for (; blocked && it + FLOW_T <= iterations; it += FLOW_T)
+  {
+    const VpStateOut o{nxt->z, nxt->d, nxt->s, nxt->fl, nxt->fr, nxt->ft, nxt->fb, nullptr, nullptr};
+    chain_launch(it > 0, io.diffusion ? k_flow_steps<FLOW_T, true> : k_flow_steps<FLOW_T, false>, g1, FT_NT, s, o, io.vec,
+                 fm[cur == &A ? 0 : 1], c, sc);
+    HM_LAUNCH_CHECK("k_flow_steps");
+    VpFields *t = cur;
+    cur = nxt;
+    nxt = t;
+  }
+  for (; it < iterations; it++)
   {
     io.in = VpState{cur->z, cur->d, cur->s, cur->fl, cur->fr, cur->ft, cur->fb};
     io.out = VpStateOut{nxt->z, nxt->d, nxt->s, nxt->fl, nxt->fr, nxt->ft, nxt->fb, nullptr, nullptr};

@@ -354,15 +354,15 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
   return fn;
 }
 
-/* map of an nx x ny fp32 grid in rows of ld floats read in boxes of 40 x
- * box_rows, zeros outside */
-static bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, int ld, int box_rows)
+/* map of an nx x ny fp32 grid in rows of ld floats read in boxes of
+ * box_cols x box_rows, zeros outside */
+bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, int ld, int box_rows, int box_cols)
 {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
   cuuint64_t dims[2] = {(cuuint64_t)nx, (cuuint64_t)ny};
   cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(float)};
-  cuuint32_t box[2] = {40u, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1u, 1u};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,

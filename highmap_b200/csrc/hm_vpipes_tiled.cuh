@@ -1088,6 +1088,7 @@ int launch_vp_tb2(const TbIo &io, const VpConst &c, cudaStream_t s);
  * 16-byte aligned, boxes no larger than the grid).  f.s may be null (the
  * flow-only step). */
 bool fwe_maps(const VpFields &f, int nx, int ny, int ld, FweMaps *m);
+bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, int ld, int box_rows, int box_cols = FW);
 /* tensor maps of one copy of s1, u, v for k_vp_step_tma; false as above */
 bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, int ld, AdvMaps *m);
 
