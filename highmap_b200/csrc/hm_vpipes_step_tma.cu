@@ -19,16 +19,25 @@ template <bool M, int F> struct StepKernel
 {
   static auto fn() { return &k_vp_step_tma<M, F>; }
 };
+/* the wide form has fixed options only */
+template <bool M, int F> struct WideKernel
+{
+  static auto fn() { return &k_vp_step_tma<M, F, (F & FWE_GENERIC) ? FT_NT : FT_WIDE>; }
+};
 } // namespace
 
 int launch_step_tma(const FweIo &io, const FweMaps &maps, const AdvMaps &am, const VpConst &c, VpScalars *sc,
                     double *partials, dim3 grid, cudaStream_t s)
 {
-  return step_dispatch<StepKernel>(io.maintain != 0, fwe_flags(io, c), [&](auto kernel) -> int {
-    chain_launch(true, kernel, grid, dim3(FT_NT), s, io, maps, am, c, sc, partials);
+  const int  flags = fwe_flags(io, c);
+  const bool wide = grid.x * grid.y <= FT_WIDE_TILES && !(flags & FWE_GENERIC);
+  auto       launch = [&](auto kernel) -> int {
+    chain_launch(true, kernel, grid, dim3(wide ? FT_WIDE : FT_NT), s, io, maps, am, c, sc, partials);
     HM_LAUNCH_CHECK("k_vp_step_tma");
     return HM_OK;
-  });
+  };
+  return wide ? step_dispatch<WideKernel>(io.maintain != 0, flags, launch)
+              : step_dispatch<StepKernel>(io.maintain != 0, flags, launch);
 }
 
 } // namespace hm

@@ -53,6 +53,7 @@ namespace hm
 
 constexpr int FT_TX = 32, FT_TY = 16;          /* output tile                 */
 constexpr int FT_NT = 256;                     /* threads per CTA             */
+constexpr int FT_WIDE = 512;                   /* threads per CTA, a cell each (FT_WIDE_TILES) */
 constexpr int FT_W2 = FT_TX + 4, FT_H2 = FT_TY + 4; /* z, depth region (halo 2) */
 constexpr int FT_W1 = FT_TX + 2, FT_H1 = FT_TY + 2; /* s, fluxes region (halo 1) */
 
@@ -164,14 +165,15 @@ constexpr unsigned SUM_TILES_MAX = 2048;
 
 /* The top-up of this step from the water per tile: the sum of
  * grid_sum_commit in the same order.  For every thread of the CTA. */
+template <int NT = FT_NT>
 __device__ __forceinline__ float tiles_top_up(const double *tiles, unsigned n, const VpScalars *sc)
 {
-  __shared__ double sm[FT_NT / 32];
+  __shared__ double sm[NT / 32];
   __shared__ float  s_add;
   double            acc = 0.0;
   /* eight loads at a time in flight (a missing one adds +0, the identity):
    * 100 steps at 1023 x 767 2.10 -> 2.00 ms against one at a time */
-  for (unsigned k = threadIdx.x; k < n; k += 8 * FT_NT)
+  for (unsigned k = threadIdx.x; k < n && threadIdx.x < FT_NT; k += 8 * FT_NT)
   {
     double v[8];
 #pragma unroll
@@ -179,16 +181,29 @@ __device__ __forceinline__ float tiles_top_up(const double *tiles, unsigned n, c
 #pragma unroll
     for (unsigned j = 0; j < 8; j++) acc += v[j];
   }
-  const double total = block_sum<FT_NT>(acc, sm);
+  const double total = block_sum<NT>(acc, sm);
   if (threadIdx.x == 0) s_add = fsub(sc->v0, (float)total);
   __syncthreads();
   return s_add;
 }
 
 /* this tile's water, at the end of the step; every thread of the CTA */
+template <int NT = FT_NT>
 __device__ __forceinline__ void tile_water_commit(const FweIo &io, VpScalars *sc, double *partials, double part,
                                                   unsigned ntiles, unsigned tile)
 {
+  if (NT == FT_WIDE)
+  {
+    /* a cell per thread: pairs of columns first, then as FT_NT threads with
+     * a pair each, so the sum's order is the same */
+    __shared__ double pairs[FT_NT], smw[NT / 32];
+    part += __shfl_xor_sync(0xffffffffu, part, 1);
+    if ((threadIdx.x & 1) == 0) pairs[threadIdx.x >> 1] = part;
+    __syncthreads();
+    const double b = block_sum<NT>(threadIdx.x < FT_NT ? pairs[threadIdx.x] : 0.0, smw);
+    if (threadIdx.x == 0) io.sum_out[tile] = b;
+    return;
+  }
   if (io.sum_out)
   {
     __shared__ double sm[FT_NT / 32];
@@ -352,14 +367,14 @@ __device__ __forceinline__ void fwe_stage_cp_async16_step(const FweIo &io, const
  * the old fluxes and, WITH_S, the sediment on region 1.  The clamped cell
  * is always inside the box; the edge test depends only on the tile, so the
  * barrier inside it is uniform. */
-template <bool WITH_S>
+template <bool WITH_S, int NT = FT_NT>
 __device__ __forceinline__ void fwe_fix_edges(int nx, int ny, int x0, int y0, FweSmem &sm)
 {
   const int tid = threadIdx.x;
   if (x0 - 2 < 0 || x0 + FT_TX + 2 > nx || y0 - 2 < 0 || y0 + FT_TY + 2 > ny)
   {
     /* region 2: columns x0-2 .. x0+33 at smem 2 .. 37, rows y0-2 .. y0+17 */
-    for (int e = tid; e < FT_W2 * FT_H2; e += FT_NT)
+    for (int e = tid; e < FT_W2 * FT_H2; e += NT)
     {
       const int ly = e / FT_W2, lx = e - ly * FT_W2;
       const int gx = x0 - 2 + lx, gy = y0 - 2 + ly;
@@ -369,7 +384,7 @@ __device__ __forceinline__ void fwe_fix_edges(int nx, int ny, int x0, int y0, Fw
       sm.d[ly][lx + 2] = sm.d[cy][cx];
     }
     /* region 1: columns x0-1 .. x0+32 at smem 3 .. 36, rows y0-1 .. y0+16 */
-    for (int e = tid; e < FT_W1 * FT_H1; e += FT_NT)
+    for (int e = tid; e < FT_W1 * FT_H1; e += NT)
     {
       const int ly = e / FT_W1, lx = e - ly * FT_W1;
       const int gx = x0 - 1 + lx, gy = y0 - 1 + ly;
@@ -489,12 +504,13 @@ __device__ __forceinline__ bool fwe_stage_tma_step(const FweMaps &maps, const Ad
  * needs no rebuild: it is advected at clamped cells, and u, v and s1 are
  * only read at in-grid cells.  false, uniformly across the CTA, if the
  * group did not complete in time. */
+template <int NT>
 __device__ __forceinline__ bool fwe_wait_tma_step_b(int nx, int ny, int x0, int y0, FweSmem &sm)
 {
   bool ok = mbar_wait_bounded(&sm.bar2, 0);
   if (!ok) ok = mbar_wait_bounded(&sm.bar2, 0);
   if (!__syncthreads_and(ok)) return false;
-  fwe_fix_edges<false>(nx, ny, x0, y0, sm);
+  fwe_fix_edges<false, NT>(nx, ny, x0, y0, sm);
   return true;
 }
 
@@ -525,17 +541,16 @@ __device__ __forceinline__ AdvBox adv_box(int nx, int ny, int x0, int y0)
   return b;
 }
 
-/* rows of region 1 one thread advects */
-constexpr int ADV_ROWS = 3;
-
-/* Thread t < 204 takes column 3 + t % 34 of region 1 and its rows
+/* ADV_ROWS, 3 (2 for FT_WIDE threads): rows of region 1 one thread advects.
+ * Thread t < 204 (306) takes column 3 + t % 34 of region 1 and its rows
  * ADV_ROWS (t / 34) .. + ADV_ROWS - 1, as one straight chain where the taps
  * of all three lie in the staged box (nearly always), so that their loads
  * and blends overlap; else cell by cell. */
-template <bool INNER>
+template <bool INNER, int NT = FT_NT>
 __device__ __forceinline__ void advect_region1(const VpConst &c, const float *s1g, int x0, int y0,
                                                FweSmem &sm)
 {
+  constexpr int ADV_ROWS = NT == FT_WIDE ? 2 : 3;
   static_assert(FT_H1 % ADV_ROWS == 0, "region 1 splits into whole row groups");
   const int t = threadIdx.x;
   if (t >= FT_W1 * (FT_H1 / ADV_ROWS)) return;
@@ -636,11 +651,11 @@ struct NoMid
  * (100 steps with a rain map at 4096 x 4096 36.3 -> 30.8 ms, at 2048 x 2048
  * 9.66 -> 8.15 ms, at 1023 x 767 2.16 -> 2.09 ms).  A thread reads back the
  * pairs it has stored. */
-template <bool MAINTAIN, int F>
+template <bool MAINTAIN, int F, int NT = FT_NT>
 struct RainStage
 {
   static constexpr bool USED = MAINTAIN && (F & (FWE_GENERIC | FWE_RTOPTS)) == 0 && (F & FWE_RAINMAP) != 0;
-  static constexpr int  N = 18 * FT_H2, PER = (N + FT_NT - 1) / FT_NT;
+  static constexpr int  N = 18 * FT_H2, PER = (N + NT - 1) / NT;
   float2                pair[USED ? N : 1];
   /* between() runs with the loads in flight */
   template <class Between>
@@ -652,7 +667,7 @@ struct RainStage
 #pragma unroll
       for (int k = 0; k < PER; k++)
       {
-        const int    e = min((int)threadIdx.x + k * FT_NT, N - 1), q = e / 18, x = x0 - 2 + 2 * (e - q * 18);
+        const int    e = min((int)threadIdx.x + k * NT, N - 1), q = e / 18, x = x0 - 2 + 2 * (e - q * 18);
         const size_t row = (size_t)clampi(y0 - 2 + q, 0, c.ny - 1) * c.nx;
         r[k].x = __ldg(io.rain + row + clampi(x, 0, c.nx - 1));
         r[k].y = __ldg(io.rain + row + clampi(x + 1, 0, c.nx - 1));
@@ -663,17 +678,19 @@ struct RainStage
     {
 #pragma unroll
       for (int k = 0; k < PER; k++)
-        if ((int)threadIdx.x + k * FT_NT < N) pair[threadIdx.x + k * FT_NT] = r[k];
+        if ((int)threadIdx.x + k * NT < N) pair[threadIdx.x + k * NT] = r[k];
     }
   }
 };
 
-template <bool MAINTAIN, int F, bool INNER = false, class Mid = NoMid>
+template <bool MAINTAIN, int F, bool INNER = false, class Mid = NoMid, int NT = FT_NT>
 __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, VpScalars *sc, double *partials,
                                             float add, int bx, int by, int nbx, int nby, FweSmem &sm, Mid mid = Mid(),
-                                            const RainStage<MAINTAIN, F> *rain = nullptr)
+                                            const RainStage<MAINTAIN, F, NT> *rain = nullptr)
 {
-  static_assert(FT_TX == 32 && FT_TY == 16 && FT_NT == 256, "one cell pair per thread in the water pass");
+  static_assert(FT_TX == 32 && FT_TY == 16 && FT_NT == 256 && FT_WIDE == 512,
+                "one cell pair per thread in the water pass, or one cell");
+  static_assert(NT == FT_NT || (F & (FWE_GENERIC | FWE_FLOWONLY)) == 0, "FT_WIDE: erosion steps of fixed options");
   constexpr bool GEN = (F & FWE_GENERIC) != 0;
   constexpr bool RT = GEN || (F & FWE_RTOPTS) != 0;
   constexpr bool FLOW_ONLY = (F & FWE_FLOWONLY) != 0;
@@ -694,12 +711,12 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
 
   /* with the top-up: stored depth -> depth at the start of the step, region
    * 2 (columns x0-2 .. x0+33 = smem 2 .. 37), 18 pairs per row */
-  for (int e = MAINTAIN ? tid : 18 * FT_H2; e < 18 * FT_H2; e += FT_NT)
+  for (int e = MAINTAIN ? tid : 18 * FT_H2; e < 18 * FT_H2; e += NT)
   {
     const int q = e / 18, cc = 2 + 2 * (e - q * 18);
     float2    dd = lds2(&sm.d[q][cc]);
     float     r0 = 1.f, r1 = 1.f;
-    if (RainStage<MAINTAIN, F>::USED)
+    if (RainStage<MAINTAIN, F, NT>::USED)
     {
       r0 = rain->pair[e].x;
       r1 = rain->pair[e].y;
@@ -751,7 +768,7 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
         else flow_cell<false, false>(c, zc, dc, zw, dw, ze, de, zs, ds, zn, dn, fl, fr, ft, fb);
       }
     };
-    for (int e = tid; e < 16 * FT_H1 + 2 * FT_H1; e += FT_NT)
+    for (int e = tid; e < 16 * FT_H1 + 2 * FT_H1; e += NT)
     {
       if (e < 16 * FT_H1)
       {
@@ -802,122 +819,163 @@ __device__ __forceinline__ void fwe_compute(const FweIo &io, const VpConst &c, V
 
     /* water and erosion on the tile: thread t takes row t / 16 and the pair
      * of tile columns 2 (t % 16), 2 (t % 16) + 1 */
-    const int ty = tid >> 4, pr = tid & 15;
-    const int gy = y0 + ty, gx = x0 + 2 * pr;
-    const int cc = 4 + 2 * pr; /* smem column of the first cell */
-    if (INNER || (gx < nx && gy < ny))
+    if constexpr (NT == FT_WIDE)
     {
-      const bool second = INNER || gx + 1 < nx;
-      const int  l = ty + 1, q = ty + 2;
-      /* flux neighbours: rows and columns clamped to the grid (new fluxes are
-       * derived: outside the grid they are the edge cell's own values) */
-      const int  ln = INNER ? ty : clampi(gy - 1, 0, ny - 1) - (y0 - 1);
-      const int  ls = INNER ? ty + 2 : clampi(gy + 1, 0, ny - 1) - (y0 - 1);
-      const int  cw0 = INNER || gx > 0 ? cc - 1 : cc;          /* west of the first cell  */
-      const int  ce0 = second ? cc + 1 : cc;                   /* east of the first cell  */
-      const int  ce1 = INNER || gx + 2 < nx ? cc + 2 : cc + 1; /* east of the second cell */
-      const float2 flc = lds2(&sm.fn[0][l][cc]), frc = lds2(&sm.fn[1][l][cc]), ftc = lds2(&sm.fn[2][l][cc]),
-                   fbc = lds2(&sm.fn[3][l][cc]);
-      const float2 ftn = lds2(&sm.fn[2][ln][cc]), fbs = lds2(&sm.fn[3][ls][cc]);
-      const float  frw0 = sm.fn[1][l][cw0], fle0 = sm.fn[0][l][ce0], fle1 = sm.fn[0][l][ce1];
-      const float2 d1 = lds2(&sm.d[q][cc]);
-      float        d2a, ua, va, d2b, ub, vb;
-      F2           depth;
-      if (!GEN)
+      /* the pair form's operations, a cell per thread */
+      const int ty = tid >> 5, gx = x0 + (tid & 31), gy = y0 + ty, cc = 4 + (tid & 31);
+      if (INNER || (gx < nx && gy < ny))
       {
-        F2 d2, u, v;
-        water_pair(c, pk(d1), pk(flc), pk(frc), pk(ftc), pk(fbc), pk(frw0, frc.x), pk(fle0, fle1), pk(ftn), pk(fbs), d2,
-                   u, v, depth);
-        d2a = lo(d2), d2b = hi(d2), ua = lo(u), ub = hi(u), va = lo(v), vb = hi(v);
-      }
-      else if (pl_one)
-      {
-        water_cell<true>(c, d1.x, flc.x, frc.x, ftc.x, fbc.x, frw0, fle0, ftn.x, fbs.x, d2a, ua, va);
-        water_cell<true>(c, d1.y, flc.y, frc.y, ftc.y, fbc.y, frc.x, fle1, ftn.y, fbs.y, d2b, ub, vb);
-      }
-      else
-      {
-        water_cell<false>(c, d1.x, flc.x, frc.x, ftc.x, fbc.x, frw0, fle0, ftn.x, fbs.x, d2a, ua, va);
-        water_cell<false>(c, d1.y, flc.y, frc.y, ftc.y, fbc.y, frc.x, fle1, ftn.y, fbs.y, d2b, ub, vb);
-      }
-      const size_t k = (size_t)gy * c.ld + gx;
-      const bool   vec = INNER || io.vec != 0;
-      if (FLOW_ONLY)
-      {
-        /* flow_simulation: the depth after the water pass is the next step's
-         * depth as it is (no evaporation, no erosion; the terrain is fixed) */
-        st_pair(io.out.fl, k, flc.x, flc.y, second, vec);
-        st_pair(io.out.fr, k, frc.x, frc.y, second, vec);
-        st_pair(io.out.ft, k, ftc.x, ftc.y, second, vec);
-        st_pair(io.out.fb, k, fbc.x, fbc.y, second, vec);
-        st_pair(io.out.d, k, d2a, d2b, second, vec);
-        (void)ua, (void)ub, (void)va, (void)vb;
-      }
-      else
-      {
-        float dea = fmul(d2a, c.keep), deb = fmul(d2b, c.keep);
+        const int l = ty + 1, q = ty + 2;
+        const int ln = INNER ? ty : clampi(gy - 1, 0, ny - 1) - (y0 - 1);
+        const int ls = INNER ? ty + 2 : clampi(gy + 1, 0, ny - 1) - (y0 - 1);
+        const int cw = INNER || gx > 0 ? cc - 1 : cc, ce = INNER || gx + 1 < nx ? cc + 1 : cc;
+        const float fl = sm.fn[0][l][cc], fr = sm.fn[1][l][cc], ft = sm.fn[2][l][cc], fb = sm.fn[3][l][cc];
+        float       d2, u, v;
+        water_cell<true>(c, sm.d[q][cc], fl, fr, ft, fb, sm.fn[1][l][cw], sm.fn[0][l][ce], sm.fn[2][ln][cc],
+                         sm.fn[3][ls][cc], d2, u, v);
+        const size_t k = (size_t)gy * c.ld + gx;
+        float        de = fmul(d2, c.keep);
         if (!MAINTAIN && rain_step && !io.last)
-        {
-          /* the next step's rain */
-          float r0 = 1.f, r1 = 1.f;
-          if (rain_map)
-          {
-            const float *r = io.rain + (size_t)gy * nx + gx;
-            r0 = __ldg(r);
-            if (second) r1 = __ldg(r + 1);
-          }
-          dea = fadd(dea, fmul(c.rps, r0));
-          deb = fadd(deb, fmul(c.rps, r1));
-        }
-        /* what the water pass produced, stored before the erosion arithmetic
-         * so its registers are free there (the stores go through generic
-         * pointers, so the compiler keeps them after the shared-memory loads
-         * that follow them in the source: their order decides what stays
-         * live; 48 registers without spills, 2.5 % faster than storing after
-         * erosion) */
-        st_pair(io.out.fl, k, flc.x, flc.y, second, vec);
-        st_pair(io.out.fr, k, frc.x, frc.y, second, vec);
-        st_pair(io.out.ft, k, ftc.x, ftc.y, second, vec);
-        st_pair(io.out.fb, k, fbc.x, fbc.y, second, vec);
-        st_pair(io.out.d, k, dea, deb, second, vec);
-        st_pair(io.u, k, ua, ub, second, vec);
-        st_pair(io.v, k, va, vb, second, vec);
+          de = fadd(de, fmul(c.rps, rain_map ? __ldg(io.rain + (size_t)gy * nx + gx) : 1.f)); /* the next step's rain */
+        io.out.fl[k] = fl;
+        io.out.fr[k] = fr;
+        io.out.ft[k] = ft;
+        io.out.fb[k] = fb;
+        io.out.d[k] = de;
+        io.u[k] = u;
+        io.v[k] = v;
         if (io.u_out)
         {
-          st_pair(io.u_out, k, ua, ub, second, vec);
-          st_pair(io.v_out, k, va, vb, second, vec);
+          io.u_out[k] = u;
+          io.v_out[k] = v;
         }
-        const float2 zc = lds2(&sm.z[q][cc]), zn = lds2(&sm.z[q - 1][cc]), zs = lds2(&sm.z[q + 1][cc]);
-        const float  zw = sm.z[q][cc - 1], ze = sm.z[q][cc + 2];
-        const float2 s0 = lds2(&sm.s[l][cc]), sn = lds2(&sm.s[l - 1][cc]), ss = lds2(&sm.s[l + 1][cc]);
-        const float  sw = sm.s[l][cc - 1], se = sm.s[l][cc + 2];
-        float        zoa, soa, zob, sob;
+        float zo, so;
+        erosion_cell<true>(c, sm.z[q][cc], sm.s[l][cc], sm.z[q][cc - 1], sm.z[q][cc + 1], sm.z[q - 1][cc], sm.z[q + 1][cc],
+                           sm.s[l][cc - 1], sm.s[l][cc + 1], sm.s[l - 1][cc], sm.s[l + 1][cc], d2, u, v, zo, so);
+        io.out.z[k] = zo;
+        io.s1[k] = so;
+        part = (double)de;
+      }
+    }
+    else
+    {
+      const int ty = tid >> 4, pr = tid & 15;
+      const int gy = y0 + ty, gx = x0 + 2 * pr;
+      const int cc = 4 + 2 * pr; /* smem column of the first cell */
+      if (INNER || (gx < nx && gy < ny))
+      {
+        const bool second = INNER || gx + 1 < nx;
+        const int  l = ty + 1, q = ty + 2;
+        /* flux neighbours: rows and columns clamped to the grid (new fluxes are
+         * derived: outside the grid they are the edge cell's own values) */
+        const int  ln = INNER ? ty : clampi(gy - 1, 0, ny - 1) - (y0 - 1);
+        const int  ls = INNER ? ty + 2 : clampi(gy + 1, 0, ny - 1) - (y0 - 1);
+        const int  cw0 = INNER || gx > 0 ? cc - 1 : cc;          /* west of the first cell  */
+        const int  ce0 = second ? cc + 1 : cc;                   /* east of the first cell  */
+        const int  ce1 = INNER || gx + 2 < nx ? cc + 2 : cc + 1; /* east of the second cell */
+        const float2 flc = lds2(&sm.fn[0][l][cc]), frc = lds2(&sm.fn[1][l][cc]), ftc = lds2(&sm.fn[2][l][cc]),
+                     fbc = lds2(&sm.fn[3][l][cc]);
+        const float2 ftn = lds2(&sm.fn[2][ln][cc]), fbs = lds2(&sm.fn[3][ls][cc]);
+        const float  frw0 = sm.fn[1][l][cw0], fle0 = sm.fn[0][l][ce0], fle1 = sm.fn[0][l][ce1];
+        const float2 d1 = lds2(&sm.d[q][cc]);
+        float        d2a, ua, va, d2b, ub, vb;
+        F2           depth;
         if (!GEN)
         {
-          F2 zo, so;
-          erosion_pair(c, pk(zc), pk(s0), pk(zw, zc.x), pk(zc.y, ze), pk(zn), pk(zs), pk(sw, s0.x), pk(s0.y, se), pk(sn),
-                       pk(ss), depth, pk(ua, ub), pk(va, vb), zo, so);
-          zoa = lo(zo), zob = hi(zo), soa = lo(so), sob = hi(so);
+          F2 d2, u, v;
+          water_pair(c, pk(d1), pk(flc), pk(frc), pk(ftc), pk(fbc), pk(frw0, frc.x), pk(fle0, fle1), pk(ftn), pk(fbs), d2,
+                     u, v, depth);
+          d2a = lo(d2), d2b = hi(d2), ua = lo(u), ub = hi(u), va = lo(v), vb = hi(v);
         }
-        else if (kexp_one)
+        else if (pl_one)
         {
-          erosion_cell<true>(c, zc.x, s0.x, zw, zc.y, zn.x, zs.x, sw, s0.y, sn.x, ss.x, d2a, ua, va, zoa, soa);
-          erosion_cell<true>(c, zc.y, s0.y, zc.x, ze, zn.y, zs.y, s0.x, se, sn.y, ss.y, d2b, ub, vb, zob, sob);
+          water_cell<true>(c, d1.x, flc.x, frc.x, ftc.x, fbc.x, frw0, fle0, ftn.x, fbs.x, d2a, ua, va);
+          water_cell<true>(c, d1.y, flc.y, frc.y, ftc.y, fbc.y, frc.x, fle1, ftn.y, fbs.y, d2b, ub, vb);
         }
         else
         {
-          erosion_cell<false>(c, zc.x, s0.x, zw, zc.y, zn.x, zs.x, sw, s0.y, sn.x, ss.x, d2a, ua, va, zoa, soa);
-          erosion_cell<false>(c, zc.y, s0.y, zc.x, ze, zn.y, zs.y, s0.x, se, sn.y, ss.y, d2b, ub, vb, zob, sob);
+          water_cell<false>(c, d1.x, flc.x, frc.x, ftc.x, fbc.x, frw0, fle0, ftn.x, fbs.x, d2a, ua, va);
+          water_cell<false>(c, d1.y, flc.y, frc.y, ftc.y, fbc.y, frc.x, fle1, ftn.y, fbs.y, d2b, ub, vb);
         }
-        st_pair(io.out.z, k, zoa, zob, second, vec);
-        st_pair(io.s1, k, soa, sob, second, vec);
-        part = (double)dea;
-        if (second) part += (double)deb;
+        const size_t k = (size_t)gy * c.ld + gx;
+        const bool   vec = INNER || io.vec != 0;
+        if (FLOW_ONLY)
+        {
+          /* flow_simulation: the depth after the water pass is the next step's
+           * depth as it is (no evaporation, no erosion; the terrain is fixed) */
+          st_pair(io.out.fl, k, flc.x, flc.y, second, vec);
+          st_pair(io.out.fr, k, frc.x, frc.y, second, vec);
+          st_pair(io.out.ft, k, ftc.x, ftc.y, second, vec);
+          st_pair(io.out.fb, k, fbc.x, fbc.y, second, vec);
+          st_pair(io.out.d, k, d2a, d2b, second, vec);
+          (void)ua, (void)ub, (void)va, (void)vb;
+        }
+        else
+        {
+          float dea = fmul(d2a, c.keep), deb = fmul(d2b, c.keep);
+          if (!MAINTAIN && rain_step && !io.last)
+          {
+            /* the next step's rain */
+            float r0 = 1.f, r1 = 1.f;
+            if (rain_map)
+            {
+              const float *r = io.rain + (size_t)gy * nx + gx;
+              r0 = __ldg(r);
+              if (second) r1 = __ldg(r + 1);
+            }
+            dea = fadd(dea, fmul(c.rps, r0));
+            deb = fadd(deb, fmul(c.rps, r1));
+          }
+          /* what the water pass produced, stored before the erosion arithmetic
+           * so its registers are free there (the stores go through generic
+           * pointers, so the compiler keeps them after the shared-memory loads
+           * that follow them in the source: their order decides what stays
+           * live; 48 registers without spills, 2.5 % faster than storing after
+           * erosion) */
+          st_pair(io.out.fl, k, flc.x, flc.y, second, vec);
+          st_pair(io.out.fr, k, frc.x, frc.y, second, vec);
+          st_pair(io.out.ft, k, ftc.x, ftc.y, second, vec);
+          st_pair(io.out.fb, k, fbc.x, fbc.y, second, vec);
+          st_pair(io.out.d, k, dea, deb, second, vec);
+          st_pair(io.u, k, ua, ub, second, vec);
+          st_pair(io.v, k, va, vb, second, vec);
+          if (io.u_out)
+          {
+            st_pair(io.u_out, k, ua, ub, second, vec);
+            st_pair(io.v_out, k, va, vb, second, vec);
+          }
+          const float2 zc = lds2(&sm.z[q][cc]), zn = lds2(&sm.z[q - 1][cc]), zs = lds2(&sm.z[q + 1][cc]);
+          const float  zw = sm.z[q][cc - 1], ze = sm.z[q][cc + 2];
+          const float2 s0 = lds2(&sm.s[l][cc]), sn = lds2(&sm.s[l - 1][cc]), ss = lds2(&sm.s[l + 1][cc]);
+          const float  sw = sm.s[l][cc - 1], se = sm.s[l][cc + 2];
+          float        zoa, soa, zob, sob;
+          if (!GEN)
+          {
+            F2 zo, so;
+            erosion_pair(c, pk(zc), pk(s0), pk(zw, zc.x), pk(zc.y, ze), pk(zn), pk(zs), pk(sw, s0.x), pk(s0.y, se), pk(sn),
+                         pk(ss), depth, pk(ua, ub), pk(va, vb), zo, so);
+            zoa = lo(zo), zob = hi(zo), soa = lo(so), sob = hi(so);
+          }
+          else if (kexp_one)
+          {
+            erosion_cell<true>(c, zc.x, s0.x, zw, zc.y, zn.x, zs.x, sw, s0.y, sn.x, ss.x, d2a, ua, va, zoa, soa);
+            erosion_cell<true>(c, zc.y, s0.y, zc.x, ze, zn.y, zs.y, s0.x, se, sn.y, ss.y, d2b, ub, vb, zob, sob);
+          }
+          else
+          {
+            erosion_cell<false>(c, zc.x, s0.x, zw, zc.y, zn.x, zs.x, sw, s0.y, sn.x, ss.x, d2a, ua, va, zoa, soa);
+            erosion_cell<false>(c, zc.y, s0.y, zc.x, ze, zn.y, zs.y, s0.x, se, sn.y, ss.y, d2b, ub, vb, zob, sob);
+          }
+          st_pair(io.out.z, k, zoa, zob, second, vec);
+          st_pair(io.s1, k, soa, sob, second, vec);
+          part = (double)dea;
+          if (second) part += (double)deb;
+        }
       }
     }
   }
 
-  if (MAINTAIN) tile_water_commit(io, sc, partials, part, (unsigned)(nbx * nby), (unsigned)(by * nbx + bx));
+  if (MAINTAIN) tile_water_commit<NT>(io, sc, partials, part, (unsigned)(nbx * nby), (unsigned)(by * nbx + bx));
 }
 
 /* the tile at (x0, y0) and its 2-cell halo lie inside the grid, and the
@@ -1011,43 +1069,43 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
 /* The same with the nine input boxes fetched by TMA in two groups (am
  * holds the maps of the previous step's u, v and s1).  Timeouts as
  * k_vp_fwe_tma. */
-template <bool MAINTAIN, int F>
-__global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
+template <bool MAINTAIN, int F, int NT = FT_NT>
+__global__ void __launch_bounds__(NT, NT == FT_WIDE ? 2 : fwe_min_blocks(F))
     k_vp_step_tma(FweIo io, const __grid_constant__ FweMaps maps, const __grid_constant__ AdvMaps am, VpConst c,
                   VpScalars *sc, double *partials)
 {
-  __shared__ FweSmem                sm;
-  __shared__ RainStage<MAINTAIN, F> rain;
+  __shared__ FweSmem                    sm;
+  __shared__ RainStage<MAINTAIN, F, NT> rain;
   const int x0 = blockIdx.x * FT_TX, y0 = blockIdx.y * FT_TY;
   float     add = 0.f;
   auto      top_up = [&]() {
     rain.load(io, c, x0, y0, [&] {
-      if (MAINTAIN) add = io.sum_in ? tiles_top_up(io.sum_in, gridDim.x * gridDim.y, sc) : sc->add[io.parity];
+      if (MAINTAIN) add = io.sum_in ? tiles_top_up<NT>(io.sum_in, gridDim.x * gridDim.y, sc) : sc->add[io.parity];
     });
   };
   if (!fwe_stage_tma_step<MAINTAIN>(maps, am, x0, y0, sm, io.tma_extra_tx, top_up))
   {
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
     if (MAINTAIN)
-      tile_water_commit(io, sc, partials, 0.0, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x);
+      tile_water_commit<NT>(io, sc, partials, 0.0, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x);
     return;
   }
   /* group B (z, fluxes) arrives during the advection and the depth pass */
   auto group_b = [&]() {
-    if (fwe_wait_tma_step_b(c.nx, c.ny, x0, y0, sm)) return true;
+    if (fwe_wait_tma_step_b<NT>(c.nx, c.ny, x0, y0, sm)) return true;
     if (threadIdx.x == 0) atomicOr(&sc->error, 1u);
     return false;
   };
   if (fwe_inner_tile(io, c.nx, c.ny, x0, y0))
   {
-    advect_region1<true>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F, true>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+    advect_region1<true, NT>(c, io.s1_prev, x0, y0, sm);
+    fwe_compute<MAINTAIN, F, true, decltype(group_b), NT>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
                                   gridDim.x, gridDim.y, sm, group_b, &rain);
   }
   else
   {
-    advect_region1<false>(c, io.s1_prev, x0, y0, sm);
-    fwe_compute<MAINTAIN, F>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
+    advect_region1<false, NT>(c, io.s1_prev, x0, y0, sm);
+    fwe_compute<MAINTAIN, F, false, decltype(group_b), NT>(io, c, sc, partials, add, blockIdx.x, blockIdx.y,
                                   gridDim.x, gridDim.y, sm, group_b, &rain);
   }
 }
@@ -1091,6 +1149,14 @@ bool fwe_maps(const VpFields &f, int nx, int ny, int ld, FweMaps *m);
 bool encode_grid_map(CUtensorMap *m, const float *base, int nx, int ny, int ld, int box_rows, int box_cols = FW);
 /* tensor maps of one copy of s1, u, v for k_vp_step_tma; false as above */
 bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, int ld, AdvMaps *m);
+
+/* Most tiles of a grid whose steps take FT_WIDE threads per CTA: two per SM
+ * run at once (48 registers), and with no more tiles than that a step's
+ * time is a CTA's chain of passes, which twice the warps shorten.  100
+ * steps, FT_NT -> FT_WIDE threads: 64 x 64 0.68 -> 0.63 ms, 256 x 256 0.714
+ * -> 0.628 ms with the defaults and 0.588 -> 0.505 ms with rain, 384 x 384
+ * (288 tiles) 0.79 -> 0.76 and 0.69 -> 0.62 ms. */
+constexpr unsigned FT_WIDE_TILES = 296;
 
 /* template flags of a step's options */
 inline int fwe_flags(const FweIo &io, const VpConst &c)

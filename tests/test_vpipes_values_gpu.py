@@ -29,9 +29,11 @@ CASES = {
 
 
 @pytest.mark.parametrize("diffusion", [0, 1])
-@pytest.mark.parametrize("nx", [128, 131])
+@pytest.mark.parametrize("nx", [128, 131, 2084])
 @pytest.mark.parametrize("case", list(CASES))
 def test_magnitudes(gpu, case, nx, diffusion):
+    """(Grids of up to 296 tiles of 32 x 16 run a cell per thread, larger
+    ones a pair.)"""
     scale, extra = CASES[case]
     z0 = (fbm(nx, 70, seed=51) * np.float32(scale)).astype(np.float32)
     z0[20:30, 40:60] = z0.min()  # a dry, then filling, flat basin
