@@ -13,12 +13,16 @@
  * and fl, fr, ft, fb (outflow fluxes); copy A's z is the caller's z.  The
  * volume top-up (V0 - sum d) * rain / R is applied lazily: the step that
  * follows reads the stored depth plus the top-up, and the grid-wide sum is
- * a deterministic fp64 reduction finished by the last block of the step.
+ * a deterministic fp64 reduction over the tiles' sums (FweIo::sum_in).  Rows
+ * are padded to a multiple of 4 floats where nx or z misses the TMA rules;
+ * z is then copied too.
  *
  * Kernels
  *   k_vp_init          initial depth, zero sediment and fluxes, V0 and R.
- *   k_vp_fwe(_tma), k_vp_advect   one step as two kernels over 2-D tiles
+ *   k_vp_fwe(_tma), k_vp_step(_tma), k_vp_advect   the first step, the later
+ *                      steps and the last advection over 2-D tiles
  *                      (hm_vpipes_tiled.cuh), the default.
+ *   k_vp_top_up        the volume top-up between the steps of large grids.
  *   k_vp_fused         one whole step streaming down column strips
  *                      (hm_vpipes_fused.cuh).
  *   k_vp_final_depth   water-depth output with the last top-up applied.

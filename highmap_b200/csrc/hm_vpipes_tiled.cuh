@@ -626,8 +626,9 @@ __device__ __forceinline__ void st_pair(float *p, size_t k, float a, float b, bo
   }
 }
 
-/* One tile of the step on staged fields, two adjacent cells per thread:
- * depth at the start of the step, flow on the tile plus a 1-cell ring into
+/* One tile of the step on staged fields, two adjacent cells per thread (one
+ * with FT_WIDE threads): with the top-up the depth at the start of the step,
+ * flow on the tile plus a 1-cell ring into
  * shared memory, then water and erosion on the tile, which also store the
  * tile's new fluxes.  A pair reads its centre values as 8-byte words and
  * shares its inner neighbours, so a cell costs about half the shared-memory
