@@ -19,10 +19,14 @@ template <bool M, int F> struct StepKernel
 {
   static auto fn() { return &k_vp_step_tma<M, F>; }
 };
-/* the wide form has fixed options only */
+/* the wide form and the one of six CTAs per SM have fixed options only */
 template <bool M, int F> struct WideKernel
 {
-  static auto fn() { return &k_vp_step_tma<M, F, (F & FWE_GENERIC) ? FT_NT : FT_WIDE>; }
+  static auto fn() { return &k_vp_step_tma<M, F, (F & FWE_GENERIC) ? FT_NT : FT_WIDE, (F & FWE_GENERIC) ? 5 : 2>; }
+};
+template <bool M, int F> struct SixKernel
+{
+  static auto fn() { return &k_vp_step_tma<M, F, FT_NT, (F & FWE_GENERIC) ? 5 : 6>; }
 };
 } // namespace
 
@@ -36,8 +40,9 @@ int launch_step_tma(const FweIo &io, const FweMaps &maps, const AdvMaps &am, con
     HM_LAUNCH_CHECK("k_vp_step_tma");
     return HM_OK;
   };
-  return wide ? step_dispatch<WideKernel>(io.maintain != 0, flags, launch)
-              : step_dispatch<StepKernel>(io.maintain != 0, flags, launch);
+  if (wide) return step_dispatch<WideKernel>(io.maintain != 0, flags, launch);
+  if (grid.x * grid.y > FT_FIVE_TILES) return step_dispatch<SixKernel>(io.maintain != 0, flags, launch);
+  return step_dispatch<StepKernel>(io.maintain != 0, flags, launch);
 }
 
 } // namespace hm

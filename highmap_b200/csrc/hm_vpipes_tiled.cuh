@@ -74,7 +74,8 @@ constexpr int FWE_FLOWONLY = 16; /* flow and water passes only (flow_simulation)
 /* Resident CTAs per SM the step kernels are compiled for.  The erosion
  * forms take five (at most 48 registers, 5 x 34 KB of shared memory): 40
  * warps per SM issuing outrun four CTAs of the unconstrained 52-register
- * code although a few words then spill.  The flow-only form
+ * code (only the generic form spills a few words), six on large grids
+ * (FT_FIVE_TILES).  The flow-only form
  * (flow_simulation) fits 40 registers, six CTAs per SM; a looser bound
  * lets the compiler take 46 and costs the sixth CTA (5 % slower). */
 constexpr int fwe_min_blocks(int flags) { return (flags & FWE_FLOWONLY) ? 6 : 5; }
@@ -1070,8 +1071,8 @@ __global__ void __launch_bounds__(FT_NT, fwe_min_blocks(F))
 /* The same with the nine input boxes fetched by TMA in two groups (am
  * holds the maps of the previous step's u, v and s1).  Timeouts as
  * k_vp_fwe_tma. */
-template <bool MAINTAIN, int F, int NT = FT_NT>
-__global__ void __launch_bounds__(NT, NT == FT_WIDE ? 2 : fwe_min_blocks(F))
+template <bool MAINTAIN, int F, int NT = FT_NT, int CTAS = fwe_min_blocks(F)>
+__global__ void __launch_bounds__(NT, CTAS)
     k_vp_step_tma(FweIo io, const __grid_constant__ FweMaps maps, const __grid_constant__ AdvMaps am, VpConst c,
                   VpScalars *sc, double *partials)
 {
@@ -1158,6 +1159,12 @@ bool adv_maps(const float *u, const float *v, const float *s1, int nx, int ny, i
  * -> 0.628 ms with the defaults and 0.588 -> 0.505 ms with rain, 384 x 384
  * (288 tiles) 0.79 -> 0.76 and 0.69 -> 0.62 ms. */
 constexpr unsigned FT_WIDE_TILES = 296;
+/* Most tiles of a grid whose steps run at five CTAs per SM: three waves.
+ * Above, six (40 registers, no spills) cover more of the waits: 100 steps
+ * with rain at 1130 x 1184 2.47 -> 2.39 ms, at 4096 x 4096 22.7 -> 21.9 ms,
+ * with the defaults 3.03 -> 2.93 and 27.8 -> 27.2 ms.  With few waves the
+ * 48-register code's shorter passes win: 512 x 512 0.93 against 1.05 ms. */
+constexpr unsigned FT_FIVE_TILES = 2220;
 
 /* template flags of a step's options */
 inline int fwe_flags(const FweIo &io, const VpConst &c)

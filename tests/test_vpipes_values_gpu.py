@@ -44,3 +44,17 @@ def test_magnitudes(gpu, case, nx, diffusion):
     gpu.hydraulic_vpipes(z, water_depth=out[0], sediment=out[1], vel_u=out[2], vel_v=out[3], **kw)
     for name, got, w in zip(("z", "water", "sediment", "u", "v"), [z] + out, want):
         assert np.array_equal(got, w), name
+
+
+@pytest.mark.parametrize("diffusion", [0, 1])
+@pytest.mark.parametrize("nx", [1028, 1031])
+def test_many_tiles(gpu, nx, diffusion):
+    """More than 2220 tiles: six CTAs per SM."""
+    z0 = fbm(nx, 1090, seed=52)
+    kw = {**BASE, "flux_diffusion": diffusion, "iterations": 4}
+    want = po.vpipes(z0, po.VpipesParams.make(**kw))
+    z = z0.copy()
+    out = [np.empty_like(z) for _ in range(4)]
+    gpu.hydraulic_vpipes(z, water_depth=out[0], sediment=out[1], vel_u=out[2], vel_v=out[3], **kw)
+    for name, got, w in zip(("z", "water", "sediment", "u", "v"), [z] + out, want):
+        assert np.array_equal(got, w), name
