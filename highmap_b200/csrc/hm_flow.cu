@@ -182,12 +182,14 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
   FlowMaps   fm[2];
   const bool blocked = tma && iterations >= FLOW_T && flow_maps<FLOW_T>(A, nx, ny, ld, &fm[0]) &&
                        flow_maps<FLOW_T>(B, nx, ny, ld, &fm[1]);
+  const bool wide = flow_steps_wide(g1.x * g1.y);
+  const auto kernel = wide ? (io.diffusion ? k_flow_steps<FLOW_T, true, FT_WIDE> : k_flow_steps<FLOW_T, false, FT_WIDE>)
+                           : (io.diffusion ? k_flow_steps<FLOW_T, true, FT_NT> : k_flow_steps<FLOW_T, false, FT_NT>);
   int        it = 0;
   for (; blocked && it + FLOW_T <= iterations; it += FLOW_T)
   {
     const VpStateOut o{nxt->z, nxt->d, nxt->s, nxt->fl, nxt->fr, nxt->ft, nxt->fb, nullptr, nullptr};
-    chain_launch(it > 0, io.diffusion ? k_flow_steps<FLOW_T, true> : k_flow_steps<FLOW_T, false>, g1, FT_NT, s, o, io.vec,
-                 fm[cur == &A ? 0 : 1], c, sc);
+    chain_launch(it > 0, kernel, g1, wide ? FT_WIDE : FT_NT, s, o, io.vec, fm[cur == &A ? 0 : 1], c, sc);
     HM_LAUNCH_CHECK("k_flow_steps");
     VpFields *t = cur;
     cur = nxt;

@@ -32,6 +32,17 @@ namespace hm
 /* steps per launch */
 constexpr int FLOW_T = 2;
 
+/* 512 threads per tile instead of 256 by the number of tiles.  Up to two
+ * tiles per SM a launch's time is one CTA's chain of passes, which twice the
+ * warps shorten (100 steps at 256 x 256 0.243 -> 0.217 ms).  Up to four
+ * (592), the CTAs of two launches fit side by side at 256 threads and the
+ * next launch's start is hidden (420 x 480 0.344 against 0.376 ms); above
+ * that they no longer do, and the 512-thread form fills the SMs with half
+ * the CTAs (540 x 560 0.594 -> 0.426 ms, 660 x 700 0.615 -> 0.542 ms, 800 x
+ * 760 0.677 -> 0.666 ms) until the waves are many (2048 x 2048 3.13 against
+ * 3.32 ms). */
+constexpr bool flow_steps_wide(unsigned tiles) { return tiles <= 296 || (tiles > 592 && tiles <= 1480); }
+
 /* tensor maps of one state copy: boxes of W x ZH (z, d) and W x FH (fluxes) */
 struct FlowMaps
 {
@@ -56,7 +67,7 @@ struct FlowTile
   static constexpr unsigned BYTES = 4u * W * (2u * ZH + 4u * FH);
 };
 
-template <int T, bool DIFF, bool INNER>
+template <int T, bool DIFF, bool INNER, int NT>
 __device__ __forceinline__ void flow_steps_tile(const VpStateOut &out, const VpConst &c, bool vec_, int x0, int y0,
                                                 FlowTile<T> &sm)
 {
@@ -68,7 +79,7 @@ __device__ __forceinline__ void flow_steps_tile(const VpStateOut &out, const VpC
   {
     {
       const int h = 2 * (T - t) + 1, np = FT_TX / 2 + h + 1, nr = FT_TY + 2 * h;
-      for (int e = threadIdx.x; e < np * nr; e += FT_NT)
+      for (int e = threadIdx.x; e < np * nr; e += NT)
       {
         const int r = e / np, p = e - r * np;
         const int gy = y0 - h + r, gx = x0 - (h + 1) + 2 * p;
@@ -95,7 +106,7 @@ __device__ __forceinline__ void flow_steps_tile(const VpStateOut &out, const VpC
     __syncthreads();
     {
       const int g = 2 * (T - t), np = FT_TX / 2 + g, nr = FT_TY + 2 * g;
-      for (int e = threadIdx.x; e < np * nr; e += FT_NT)
+      for (int e = threadIdx.x; e < np * nr; e += NT)
       {
         const int r = e / np, p = e - r * np;
         const int gy = y0 - g + r, gx = x0 - g + 2 * p;
@@ -129,10 +140,10 @@ __device__ __forceinline__ void flow_steps_tile(const VpStateOut &out, const VpC
 }
 
 /* A tile whose loads time out sets bit 0 of sc->error and writes nothing.
- * 32 registers: eight CTAs per SM instead of six cover more of the waits
+ * 32 registers: eight CTAs (of 256 threads) per SM instead of six cover more of the waits
  * (513 x 511 0.50 -> 0.40 ms, 4096 x 4096 11.65 -> 11.50 ms). */
-template <int T, bool DIFF>
-__global__ void __launch_bounds__(FT_NT, 8)
+template <int T, bool DIFF, int NT>
+__global__ void __launch_bounds__(NT, 2048 / NT)
     k_flow_steps(VpStateOut out, int vec, const __grid_constant__ FlowMaps maps, VpConst c, VpScalars *sc)
 {
   using L = FlowTile<T>;
@@ -169,9 +180,9 @@ __global__ void __launch_bounds__(FT_NT, 8)
     return;
   }
   if (vec && x0 >= 2 * T && x0 + FT_TX + 2 * T <= c.nx && y0 >= 2 * T && y0 + FT_TY + 2 * T <= c.ny)
-    flow_steps_tile<T, DIFF, true>(out, c, true, x0, y0, sm);
+    flow_steps_tile<T, DIFF, true, NT>(out, c, true, x0, y0, sm);
   else
-    flow_steps_tile<T, DIFF, false>(out, c, vec != 0, x0, y0, sm);
+    flow_steps_tile<T, DIFF, false, NT>(out, c, vec != 0, x0, y0, sm);
 }
 
 } // namespace hm
