@@ -312,11 +312,10 @@ constexpr float QUOT_MAX = 1152921504606846976.f; /* 2^60 */
 __device__ __forceinline__ F2 top_up_pair(F2 rain, float add, float rvol, float y, bool ok)
 {
   const float2 n = up(mul2(pk1(add), rain));
-  float2       q = up(quot2(pk(n), pk1(-rvol), pk1(y)));
-  if (!(ok && quot_min(quot_min(~0u, n.x), n.y) >= QUOT_MIN && fadd(fabsf(q.x), fabsf(q.y)) < QUOT_MAX))
-    q = make_float2(fdiv(n.x, rvol), fdiv(n.y, rvol));
-  /* (a zero keeps its sign) */
-  return pk(copysignf(q.x, n.x), copysignf(q.y, n.y));
+  const float2 q = up(quot2(pk(n), pk1(-rvol), pk1(y)));
+  if (ok && quot_min(quot_min(~0u, n.x), n.y) >= QUOT_MIN && fadd(fabsf(q.x), fabsf(q.y)) < QUOT_MAX)
+    return pk(copysignf(q.x, n.x), copysignf(q.y, n.y)); /* rvol > 0: the sign of n, of a zero too */
+  return pk(fdiv(n.x, rvol), fdiv(n.y, rvol));
 }
 
 /* flow_cell for a pair; w and e are the pairs one column to the west and
