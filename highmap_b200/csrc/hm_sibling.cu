@@ -127,7 +127,6 @@ struct SiblingRule
     return pk(cell(lo(c), lo(w), lo(s), lo(n), lo(e), lo(nw), lo(sw), lo(ne), lo(se), lo(t), lo(x), first, p),
               cell(hi(c), hi(w), hi(s), hi(n), hi(e), hi(nw), hi(sw), hi(ne), hi(se), hi(t), hi(x), first, p));
   }
-  __device__ static __forceinline__ F2 talus_pair(F2 t) { return t; }
 };
 
 constexpr int SS_NT = 256, SS2_NT = 128, SS_H = 16; /* as the thermal sweeps */

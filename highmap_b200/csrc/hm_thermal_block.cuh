@@ -100,7 +100,7 @@ __device__ __forceinline__ void thermal_block(const float *a,
   for (int q = 0; q < ROWS; q++)
   {
     const size_t o = (size_t)min(max(j0 + q, 0), ny - 1) * nx;
-    tl[q] = R::talus_pair(TMAP ? pair_ldg<VEC>(talus + o, x0, x1) : pk1(talus_value));
+    tl[q] = TMAP ? pair_ldg<VEC>(talus + o, x0, x1) : pk1(talus_value);
     ex[q] = R::EXTRA ? pair_ldg<VEC>(extra + o, x0, x1) : pk1(0.f);
   }
   chain_wait();

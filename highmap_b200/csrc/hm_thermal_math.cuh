@@ -139,12 +139,13 @@ __device__ __forceinline__ float thermal_cell(float c,
 }
 
 /* The same for two adjacent cells at once, in packed arithmetic
- * (hm_pack.cuh): 42 instead of 62 issue slots per cell, the same bits.
- * Each exchange is the scalar one, operation by operation: the
- * subtractions, the products and the sums are packed; the max and the sign
- * go per half (packed instructions take no absolute value).
- * No product feeds a packed add directly (a copysign or the last fma of
- * the division lies between), so nothing is contracted. */
+ * (hm_pack.cuh): fewer issue slots per cell, the same bits.
+ * Each exchange is the scalar one, operation by operation: the difference
+ * of the heights, the products and the sums are packed; the absolute value
+ * (packed instructions take none), the max and the sign go per half.
+ * No packed product feeds a packed add or subtract directly: diag_talus2
+ * forms none, and a copysign or the last fma of the division lies between
+ * the others and the sum. */
 __device__ __forceinline__ F2 copysign2(F2 mag, F2 sgn)
 {
   /* mag is not negative */
@@ -156,21 +157,14 @@ __device__ __forceinline__ F2 copysign2(F2 mag, F2 sgn)
   return r;
 }
 
-/* 0.2 * max(|n| - t, 0) for both halves as 0.2 * (max(|n|, t) - t), which
- * leaves only the max per half: the same value for every n (NaN gives 0 in
- * both) and every t that talus2 lets through */
+/* 0.2 * max(|n| - t, 0) for both halves.  (max(|n|, t) - t would leave one
+ * scalar instruction per half, but is NaN for an infinite or NaN t, and
+ * bounding t first is wrong where |n| is beyond the bound.) */
 __device__ __forceinline__ F2 exch2(F2 n, F2 t)
 {
-  const float2 a = up(n), b = up(t);
-  return mul2(sub2(pk(fmaxf(fabsf(a.x), b.x), fmaxf(fabsf(a.y), b.y)), t), pk1(0.2f));
-}
-
-/* A talus pair for the packed exchanges: NaN and +inf, which stop every
- * exchange, become the largest talus whose product with 1.414 is finite */
-__device__ __forceinline__ F2 talus2(F2 t)
-{
-  const float2 v = up(t);
-  return pk(fminf(v.x, 2.4e38f), fminf(v.y, 2.4e38f));
+  const float2 a = up(n);
+  const float2 x = up(sub2(pk(fabsf(a.x), fabsf(a.y)), t));
+  return mul2(pk(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)), pk1(0.2f));
 }
 
 __device__ __forceinline__ F2 exch_axial2(F2 self, F2 other, F2 t)
@@ -189,10 +183,19 @@ __device__ __forceinline__ F2 exch_diag2(F2 self, F2 other, F2 md)
   return copysign2(fma2(r, y, q), n);
 }
 
-__device__ __forceinline__ F2 thermal_amount2(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw, F2 sw, F2 ne, F2 se, F2 t)
+/* 1.414 t, which exch2 subtracts: two scalar products, or, PACKED, one fma
+ * that cannot be contracted (mul2r; blocks are flat, so threadIdx.z is a
+ * zero the compiler does not know) */
+template <bool PACKED>
+__device__ __forceinline__ F2 diag_talus2(F2 t)
 {
-  const F2 md = mul2(pk1(1.414f), t);
-  F2       a = exch_axial2(c, w, t);
+  if (PACKED) return mul2r(pk1(1.414f), t, pk1(__uint_as_float(0x80000000u | threadIdx.z)));
+  return pk(__fmul_rn(1.414f, lo(t)), __fmul_rn(1.414f, hi(t)));
+}
+
+__device__ __forceinline__ F2 thermal_amount2(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw, F2 sw, F2 ne, F2 se, F2 t, F2 md)
+{
+  F2 a = exch_axial2(c, w, t);
   a = add2(a, exch_axial2(c, s, t));
   a = add2(a, exch_axial2(c, n, t));
   a = add2(a, exch_axial2(c, e, t));
@@ -210,7 +213,11 @@ __device__ __forceinline__ F2 thermal_cell2(F2 c, F2 w, F2 s, F2 n, F2 e, F2 nw,
 {
   const float2 v = up(c), b = up(bed);
   if (BED == BED_LITERAL) return pk(v.x > b.x ? v.x : b.x, v.y > b.y ? v.y : b.y);
-  const F2     x2 = add2(c, thermal_amount2(c, w, s, n, e, nw, sw, ne, se, t));
+  /* (auto-bedrock's sweep has two registers too many for seven CTAs per SM
+   * with the scalar products: 96 steps at 2048 x 2048 1.53 against 1.40 ms;
+   * the block kernel of the other modes is 3 to 5 % faster with them) */
+  const F2     md = diag_talus2<BED == BED_AUTO>(t);
+  const F2     x2 = add2(c, thermal_amount2(c, w, s, n, e, nw, sw, ne, se, t, md));
   if (BED == BED_NONE) return x2;
   const float2 x = up(x2);
   /* val < bedrock leaves the bedrock, so both tests of thermal_cell end in

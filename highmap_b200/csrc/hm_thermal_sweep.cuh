@@ -47,8 +47,6 @@ struct TalusExchange
   {
     return thermal_cell2<BED>(c, w, s, n, e, nw, sw, ne, se, t, x, first);
   }
-  /* the talus of a pair as R::pair takes it */
-  __device__ static __forceinline__ F2 talus_pair(F2 t) { return talus2(t); }
 };
 
 /* Columns wx .. wx+31 (lane = column; columns past nx only feed the
@@ -215,7 +213,7 @@ __device__ __forceinline__ void thermal_sweep2_warp(const float *a,
     {
       load(min(j0 + 1 + q, ny - 1), q + 2);
       const size_t o = (size_t)min(j0 + q, ny - 1) * nx + gxc;
-      tl[q] = R::talus_pair(TMAP ? ldg2(talus + o) : pk1(talus_value));
+      tl[q] = TMAP ? ldg2(talus + o) : pk1(talus_value);
       bd[q] = R::EXTRA ? ldg2(bedrock + o) : pk1(0.f);
     }
 #pragma unroll
