@@ -937,6 +937,9 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
   const int        nlanes = spread ? LANES : HM_BATCH_LANES;
   std::vector<int> large;
   std::vector<Lane *> lane_of; /* of large[q] */
+  /* of large[q]: asked once, since the answer sizes the lane's scratch and
+   * another thread may change the process's choice of kernels meanwhile */
+  std::vector<bool> padded;
   int              maxit = 0;
   for (int k = 0; k < njobs && !st; k++)
   {
@@ -964,11 +967,11 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
     const hm_job &j = jobs[k];
     l->jobs++;
     lane_of.push_back(l);
+    padded.push_back(j.kind == HM_JOB_VPIPES && hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations));
     l->work += work(k);
     l->bytes = std::max(l->bytes, j.kind == HM_JOB_THERMAL
                                       ? hm::thermal_scratch_floats(j.nx, j.ny, j.deposition_map != nullptr) * sizeof(float)
-                                      : hm::vpipes_scratch_bytes(
-                                            j.nx, j.ny, hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations)));
+                                      : hm::vpipes_scratch_bytes(j.nx, j.ny, padded.back()));
   }
   cudaEvent_t fork = nullptr;
   if (!st && !large.empty())
@@ -1014,7 +1017,7 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
         hm_vpipes_params p = j.vpipes;
         p.iterations = j.iterations;
         rc = hm::vpipes_core(j.z, j.nx, j.ny, p, j.rain_map, j.water_depth, j.sediment, j.vel_u, j.vel_v, l.mem, l.s,
-                             hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations));
+                             padded[q]);
       }
       if (rc) return rc;
     }
