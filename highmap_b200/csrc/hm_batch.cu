@@ -973,10 +973,16 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
                                       ? hm::thermal_scratch_floats(j.nx, j.ny, j.deposition_map != nullptr) * sizeof(float)
                                       : hm::vpipes_scratch_bytes(j.nx, j.ny, padded.back()));
   }
+  /* a word per job: the error word its solve left (a tile whose loads timed
+   * out wrote nothing), copied before the lane's next job reuses the scratch */
+  unsigned   *errors = nullptr;
   cudaEvent_t fork = nullptr;
   if (!st && !large.empty())
   {
     cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+      e = cudaMallocFromPoolAsync((void **)&errors, large.size() * sizeof(unsigned), b->pool, b->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(errors, 0, large.size() * sizeof(unsigned), b->stream);
     for (Lane &l : lanes)
     {
       if (l.jobs == 0 || e != cudaSuccess) continue;
@@ -1018,6 +1024,9 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
         p.iterations = j.iterations;
         rc = hm::vpipes_core(j.z, j.nx, j.ny, p, j.rain_map, j.water_depth, j.sediment, j.vel_u, j.vel_v, l.mem, l.s,
                              padded[q]);
+        if (!rc)
+          HM_CUDA_TRY(cudaMemcpyAsync(errors + q, hm::vpipes_error_word(l.mem, j.nx, j.ny, padded[q]),
+                                      sizeof(unsigned), cudaMemcpyDeviceToDevice, l.s));
       }
       if (rc) return rc;
     }
@@ -1077,12 +1086,21 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
     if (!st) st = join_large();
     if (!st) st = hm_batch_synchronize(b);
   }
+  if (!st && !large.empty())
+  {
+    std::vector<unsigned> word(large.size());
+    const cudaError_t     e = cudaMemcpy(word.data(), errors, word.size() * sizeof(unsigned), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) st = hm::cuda_fail(e, "hm_batch_run: error words");
+    for (size_t q = 0; q < word.size() && !st; q++)
+      if (word[q]) st = hm::fail(HM_ERR_TIMEOUT, "hm_batch_run: tile loads timed out on the device");
+  }
   /* the lanes are done (joined, or synchronised here on an error path)
    * before their memory goes back to the pool */
   for (Lane &l : lanes)
     if (l.s) cudaStreamSynchronize(l.s);
   for (Lane &l : lanes)
     if (l.mem) cudaFreeAsync(l.mem, b->stream);
+  if (errors) cudaFreeAsync(errors, b->stream);
   cudaStreamSynchronize(b->stream);
   for (Lane &l : lanes)
   {

@@ -720,7 +720,9 @@ long long hm_batch_round(const hm_batch *batch);
  * by cell-updates) beside the rounds of the smaller jobs, launched while the
  * rounds' graph is built.  In batches of more than a few milliseconds of
  * work, thermal jobs and virtual-pipes jobs of at least 2^17 cells go there
- * too, on four side streams.  Results are the same either way. */
+ * too, on four side streams.  Results are the same either way.
+ * HM_ERR_TIMEOUT if a job's tile loads timed out there: the jobs' grids then
+ * hold no complete results. */
 #define HM_BATCH_LARGE_CELLS (1 << 20)
 #define HM_BATCH_LANES 1
 int       hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph);

@@ -1,9 +1,11 @@
 """Batches of more than a few milliseconds of work, whose thermal jobs and
 larger virtual-pipes jobs run on four side streams: every job gives the bits
-of its plain call."""
+of its plain call, and a virtual-pipes job whose tile loads time out there
+makes the run report it."""
 import numpy as np
 import pytest
 
+from highmap_b200 import _lib as L
 from highmap_b200.inputs import fbm
 
 pytestmark = pytest.mark.gpu
@@ -123,3 +125,34 @@ def test_kernel_choice_changes_meanwhile(gpu):
         stop.set()
         t.join()
         gpu.vpipes_set_algorithm(gpu.VPIPES_AUTO)
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("first", [0, 1])
+def test_lane_timeout_is_reported(gpu, use_graph, first):
+    """The test hook makes every TMA tile's bounded wait run out; a later job
+    on the same lane starts with a clean error word and may be shorter or a
+    thermal one."""
+    import torch
+    from highmap_b200 import batch as B
+    specs = [("thermal", 1024, 1024, 1200, dict(), 0), ("vpipes", 512, 256, 1, RAIN, 0), ("vpipes", 64, 48, 2, RAIN, 0)]
+    if first:
+        specs = specs[1:]
+        specs[0] = ("vpipes", 1024, 1024, 1, RAIN, 0)  # above 2^20 cells: the one lane of smaller batches
+    jobs = [_job(*c) for c in _make(specs)]
+    try:
+        gpu.vpipes_set_algorithm(gpu.VPIPES_TILED)
+        gpu.debug_tma_expect_extra(16)
+        with pytest.raises(L.HMError) as e:
+            B.run(jobs, use_graph=use_graph)
+        assert e.value.status == L.HM_ERR_TIMEOUT and "timed out" in str(e.value)
+    finally:
+        gpu.debug_tma_expect_extra(0)
+        gpu.vpipes_set_algorithm(gpu.VPIPES_AUTO)
+    got, want = _make(specs), _make(specs)
+    B.run([_job(*c) for c in got], use_graph=use_graph)
+    for c in want:
+        _plain(gpu, *c)
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        assert torch.equal(g[1], w[1])
