@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(TBK_NT)
                     const float *__restrict__ zmax, float intensity, int T)
 {
   thermal_block<RULE != HM_RIB, SiblingRule<RULE>, ROWS, VEC>(a, b, nx, ny, talus, 0.f, zmax, T, blockIdx.x,
-                                                              blockIdx.y, false, intensity);
+                                                              false, intensity);
 }
 
 template <int RULE>

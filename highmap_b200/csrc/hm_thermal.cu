@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(TBK_NT)
                     int first)
 {
   thermal_block<TMAP, TalusExchange<BED>, ROWS, VEC>(a, b, nx, ny, talus, talus_value, bedrock, T, blockIdx.x,
-                                                     blockIdx.y, first != 0);
+                                                     first != 0);
 }
 
 /* ------------------------------------------------------------------ */
@@ -461,7 +461,7 @@ int thermal_core(int device,
     if (rows == 0) rows = e.rows;
   }
   if (tb == 0) plan = block_pick(nx, ny, iterations, !keep_z);
-  else if (tb == 1 || iterations < 2) plan = BlockPlan{1, 0, iterations};
+  else if (tb == 1 || iterations == 0) plan = BlockPlan{1, 0, iterations};
   else plan = block_fixed(tb > TBK_TMAX ? TBK_TMAX : tb, rows, iterations, !keep_z);
   /* auto-bedrock reads the input heights as its bedrock */
   const int    mode = kernel_bed_mode(bedrock, o.bedrock_mode, auto_bed);
@@ -470,7 +470,8 @@ int thermal_core(int device,
   for (int l = 0; l < plan.launches; l++)
   {
     float *dst = buf[l & 1];
-    if (plan.T == 1)
+    /* (a plan asked for goes on past the rows a launch of the sweep takes) */
+    if (plan.T == 1 && (plan.rows == 0 || ny <= 65535 * SW_H))
     {
       step_dispatch(src, dst, nx, ny, talus, talus_value, bed, mode, l == 0, s, chained || l > 0);
       HM_LAUNCH_CHECK("k_thermal_sweep");

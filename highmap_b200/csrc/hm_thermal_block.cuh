@@ -66,7 +66,7 @@ __device__ __forceinline__ F2 pair_ldg(const float *row, int x0, int x1)
   return VEC ? ldg2(row + x0) : pk(__ldg(row + x0), __ldg(row + x1));
 }
 
-/* Tile (bx, by): T steps from a into b.  talus and extra are loaded before
+/* Tile bx of the block's row of tiles: T steps from a into b.  talus and extra are loaded before
  * the wait for the launch before (hm_chain.cuh).  Loads are clamped to the grid;
  * what lies outside only feeds halo cells, since border cells copy their
  * inward neighbour. */
@@ -80,7 +80,6 @@ __device__ __forceinline__ void thermal_block(const float *a,
                                               const float *__restrict__ extra,
                                               int T,
                                               int bx,
-                                              int by,
                                               bool first,
                                               float param = 0.f)
 {
@@ -89,7 +88,10 @@ __device__ __forceinline__ void thermal_block(const float *a,
   const int  HL = (T + 1) >> 1, W = 64 - 4 * HL;
   const int  lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int  c0 = bx * W - 2 * HL, gx = c0 + 2 * lane;
-  const int  r0 = by * (TY - 2 * T) - T; /* first row of the tile */
+  /* first row of the tile's output; tbk_grid folds a grid's y into z */
+  const unsigned y0 = (blockIdx.y + blockIdx.z * gridDim.y) * (unsigned)(TY - 2 * T);
+  if (y0 >= (unsigned)ny) return;        /* the whole CTA: a block that the fold adds */
+  const int  r0 = (int)y0 - T;           /* first row of the tile */
   const int  j0 = r0 + wp * ROWS;        /* first row of the warp */
   const int  x0 = min(max(gx, 0), VEC ? nx - 2 : nx - 1), x1 = min(max(gx + 1, 0), nx - 1);
   const bool edge = c0 <= 0 || c0 + 64 >= nx || r0 <= 0 || r0 + TY >= ny;
@@ -162,10 +164,12 @@ struct BlockPlan
   int T, rows, launches;
 };
 
+/* (a grid has at most 65535 blocks in y) */
 inline dim3 tbk_grid(int nx, int ny, const BlockPlan &p)
 {
   const int w = tbk_cols(p.T), h = tbk_rows(p.rows, p.T);
-  return dim3((nx + w - 1) / w, (ny + h - 1) / h);
+  const int gy = (ny + h - 1) / h;
+  return dim3((nx + w - 1) / w, gy < 65535 ? gy : 65535, (gy + 65534) / 65535);
 }
 
 /* `iterations` steps in launches of at most T, the count rounded up so that
@@ -195,7 +199,7 @@ inline BlockPlan block_pick(int nx, int ny, int iterations, bool even)
       const BlockPlan p = block_split(iterations, T, rows, even);
       if (p.T < 2) continue;
       const dim3   g = tbk_grid(nx, ny, p);
-      const int    k = (int)((g.x * g.y + 147) / 148);
+      const int    k = (int)((g.x * g.y * g.z + 147) / 148);
       const double s = rows == 1 ? 0.20 : 0.30, c = rows == 1 ? 0.45 : 0.80;
       const double us = 2.0 + p.T * (s + k * c);
       const double total = p.launches * (us > 4.1 ? us : 4.1);
