@@ -31,6 +31,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -288,6 +289,9 @@ VpConst vpipes_consts(int nx, int ny, const hm_vpipes_params &p)
   c.c0 = p.flux_diffusion_strength;
   c.c1 = 1.f - 4.f * p.flux_diffusion_strength;
   c.vel_floor = 0.001f * p.water_height / p.dt;
+  /* the kernels' max returns NaN where the reference's max(floor, depth)
+   * with a NaN floor is the depth */
+  if (c.vel_floor != c.vel_floor) c.vel_floor = -HUGE_VALF;
   c.water_height = p.water_height;
   c.ratio = p.downcutting_max_depth_ratio;
   c.k_capacity = p.k_capacity;
