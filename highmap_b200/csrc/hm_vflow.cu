@@ -166,8 +166,11 @@ __global__ void __launch_bounds__(VF_NT) k_vflow_init(float *__restrict__ h, con
   unsigned m = 0u;
   for (size_t k = blockIdx.x * (size_t)VF_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * VF_NT)
   {
-    const float    v = __fmul_rn(water_height, depth_map[k]);
-    const unsigned key = fkey(v);
+    const float v = __fmul_rn(water_height, depth_map[k]);
+    /* the reference's maximum starts at the first cell and takes what is
+     * greater: a NaN counts there and is passed over elsewhere (steps leave
+     * no NaN) */
+    const unsigned key = v == v ? fkey(v) : (k == 0 ? ~0u : 0u);
     h[k] = v;
     m = key > m ? key : m;
   }
