@@ -173,6 +173,7 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
     for (const void *q : outs) ok = ok && al8(q);
     io.vec = ok ? 1 : 0;
   }
+  io.tma_extra_tx = tma_extra_tx();
   FweMaps    maps[2];
   const bool tma = fwe_maps(A, nx, ny, ld, &maps[0]) && fwe_maps(B, nx, ny, ld, &maps[1]);
   const dim3 g1((nx + FT_TX - 1) / FT_TX, (ny + FT_TY - 1) / FT_TY);
@@ -183,8 +184,11 @@ int flow_simulation_core(const float *z, int nx, int ny, float water_height, con
   const bool blocked = tma && iterations >= FLOW_T && flow_maps<FLOW_T>(A, nx, ny, ld, &fm[0]) &&
                        flow_maps<FLOW_T>(B, nx, ny, ld, &fm[1]);
   const bool wide = flow_steps_wide(g1.x * g1.y);
-  const auto kernel = wide ? (io.diffusion ? k_flow_steps<FLOW_T, true, FT_WIDE> : k_flow_steps<FLOW_T, false, FT_WIDE>)
+  auto       kernel = wide ? (io.diffusion ? k_flow_steps<FLOW_T, true, FT_WIDE> : k_flow_steps<FLOW_T, false, FT_WIDE>)
                            : (io.diffusion ? k_flow_steps<FLOW_T, true, FT_NT> : k_flow_steps<FLOW_T, false, FT_NT>);
+  if (io.tma_extra_tx)
+    kernel = wide ? (io.diffusion ? k_flow_steps<FLOW_T, true, FT_WIDE, true> : k_flow_steps<FLOW_T, false, FT_WIDE, true>)
+                  : (io.diffusion ? k_flow_steps<FLOW_T, true, FT_NT, true> : k_flow_steps<FLOW_T, false, FT_NT, true>);
   int        it = 0;
   for (; blocked && it + FLOW_T <= iterations; it += FLOW_T)
   {

@@ -190,6 +190,7 @@ static FusedCfg g_cfg_override = {0, 0, 0};
 static int g_algo_override = -1;
 /* bytes a TMA tile's barrier expects beyond its boxes (hm_debug_tma_expect_extra) */
 static unsigned g_tma_extra_tx = 0;
+unsigned        tma_extra_tx() { return g_tma_extra_tx; }
 
 FusedCfg vpipes_pick_config(int nx, int ny)
 {

@@ -32,6 +32,8 @@ int     vpipes_init(const VpFields &A, const float *rain, int nx, int ny, float 
 /* device address of the solve's error word (bit 0: a tile's TMA loads
  * timed out and the tile was skipped) inside the scratch of vpipes_core */
 const unsigned *vpipes_error_word(const void *scratch_buf, int nx, int ny, bool padded);
+/* what hm_debug_tma_expect_extra has set */
+unsigned        tma_extra_tx();
 /* flow_simulation (hm_flow.cu): device pointers, ordered on s; scratch of
  * flow_scratch_bytes; water_depth receives the final depth */
 int             flow_check_args(const float *z, const float *depth_map, const float *out, int nx, int ny,

@@ -521,7 +521,7 @@ def vpipes_set_algorithm(algo: int = VPIPES_AUTO) -> None:
 
 
 def debug_tma_expect_extra(nbytes: int = 0) -> None:
-    """Test hook: every TMA-staged vpipes tile expects ``nbytes`` more than
+    """Test hook: every TMA-staged vpipes or flow tile expects ``nbytes`` more than
     its boxes deliver, so its bounded wait runs out and the call reports
     HM_ERR_TIMEOUT (0 turns it off)."""
     L.check(L.lib().hm_debug_tma_expect_extra(int(nbytes)))
