@@ -187,7 +187,16 @@ inline BlockPlan block_split(int iterations, int T, int rows, bool even)
  * launches x max(4.1, 2 + T (s + k c)) us with k CTAs on the fullest SM,
  * s + c = 0.65, c = 0.45 for ROWS 1 and s + c = 1.1, c = 0.8 for ROWS 2, a
  * fit within 10 % of the times measured at 64^2, 256^2, 513 x 257, 512^2,
- * 1025 x 769 and 1024^2 for T = 2 .. 8. */
+ * 1025 x 769 and 1024^2 for T = 2 .. 8.
+ *
+ * Two shapes fill the tiles badly.  Grids of up to 32 rows are compared
+ * with one step per launch (5 us and 2 per million cells; odd widths, whose
+ * warps take 32 columns and load 8 rows at a time, 6 per million cells of at
+ * least 8 rows): 10 steps, blocked and not, 350000 x 4 187 and 68 us,
+ * 466666 x 3 412 and 240, 87500 x 16 109 and 86, 43750 x 32 117 and 90, but
+ * 3000 x 20 24 and 69 and 19781 x 63 78 and 127.  Grids of 3 or 4 columns
+ * take one step per launch from 150000 rows on: 3 x 466666 1.30 and 0.99 ms,
+ * 3 x 30000 116 and 142 us. */
 inline BlockPlan block_pick(int nx, int ny, int iterations, bool even)
 {
   if (iterations < 2 || (long long)nx * ny > 1500000) return BlockPlan{1, 0, iterations};
@@ -209,6 +218,8 @@ inline BlockPlan block_pick(int nx, int ny, int iterations, bool even)
         best = p;
       }
     }
+  const double sweep_us = nx % 2 == 0 ? 5.0 + 2e-6 * nx * ny : 5.0 + 6e-6 * nx * (ny < 8 ? 8 : ny);
+  if (ny <= 32 ? iterations * sweep_us < best_us : nx <= 4 && ny >= 150000) return BlockPlan{1, 0, iterations};
   return best;
 }
 
