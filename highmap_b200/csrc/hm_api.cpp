@@ -598,7 +598,7 @@ int hm_vpipes(hm_context *ctx, float *z, int nx, int ny, const hm_vpipes_params 
   const size_t nbytes = n * sizeof(float);
   size_t       fields = 1 + (rain_map ? 1 : 0) + (water_depth ? 1 : 0) + (sediment ? 1 : 0) + (vel_u ? 1 : 0) +
                   (vel_v ? 1 : 0);
-  const bool   padded = hm::vpipes_wants_padding(nullptr, nx, ny, p.iterations); /* z goes to an aligned grid */
+  const bool   padded = hm::vpipes_wants_padding(nullptr, nx, ny, p.iterations, !!sediment + !!vel_u + !!vel_v); /* z goes to an aligned grid */
   const size_t scratch = hm::vpipes_scratch_bytes(nx, ny, padded);
   size_t       total = fields * align_up(nbytes, 256) + align_up(scratch, 256);
   void        *ws = nullptr;
@@ -646,7 +646,7 @@ int hm_vpipes_device(hm_context *ctx, float *z, int nx, int ny, const hm_vpipes_
   int st = hm::vpipes_check_args(z, nx, ny, &p);
   if (st) return st;
   if ((st = hm::use_device(ctx->device))) return st;
-  const bool padded = hm::vpipes_wants_padding(z, nx, ny, p.iterations);
+  const bool padded = hm::vpipes_wants_padding(z, nx, ny, p.iterations, !!sediment + !!vel_u + !!vel_v);
   void      *ws = nullptr;
   if ((st = hm::workspace(ctx, hm::vpipes_scratch_bytes(nx, ny, padded), &ws))) return st;
   return hm::vpipes_core(z, nx, ny, p, rain_map, water_depth, sediment, vel_u, vel_v, ws, (cudaStream_t)stream,

@@ -967,7 +967,8 @@ int hm_batch_run(hm_context *ctx, const hm_job *jobs, int njobs, int use_graph)
     const hm_job &j = jobs[k];
     l->jobs++;
     lane_of.push_back(l);
-    padded.push_back(j.kind == HM_JOB_VPIPES && hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations));
+    padded.push_back(j.kind == HM_JOB_VPIPES && hm::vpipes_wants_padding(j.z, j.nx, j.ny, j.iterations,
+                                                                            !!j.sediment + !!j.vel_u + !!j.vel_v));
     l->work += work(k);
     l->bytes = std::max(l->bytes, j.kind == HM_JOB_THERMAL
                                       ? hm::thermal_scratch_floats(j.nx, j.ny, j.deposition_map != nullptr) * sizeof(float)

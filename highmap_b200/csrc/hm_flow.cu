@@ -107,7 +107,9 @@ static size_t flow_state_floats(int nx, int ny, bool padded)
 
 bool flow_wants_padding(const float *z, int nx, int ny, int iterations)
 {
-  return iterations > 0 && nx >= 40 && ny >= FT_H2 && (long long)nx * ny <= (1ll << 28) &&
+  /* one step: the terrain's copy costs more than it wins on small grids
+   * (255 x 257 26.7 -> 28.2 us; 601 x 599 6 % faster) */
+  return (iterations > 1 || (iterations == 1 && (long long)nx * ny >= 100000)) && nx >= 40 && ny >= FT_H2 && (long long)nx * ny <= (1ll << 28) &&
          (nx % 4 != 0 || ((uintptr_t)z & 15u) != 0);
 }
 

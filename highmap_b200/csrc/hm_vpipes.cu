@@ -31,6 +31,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -262,9 +263,12 @@ static size_t state_floats(int nx, int ny, bool padded)
   return align_up((padded ? align_up((size_t)nx, 4) : (size_t)nx) * ny, 64);
 }
 
-bool vpipes_wants_padding(const float *z, int nx, int ny, int iterations)
+bool vpipes_wants_padding(const float *z, int nx, int ny, int iterations, int copied_outputs)
 {
-  return iterations > 0 && nx >= 40 && ny >= FS_H && (long long)nx * ny <= (1ll << 28) &&
+  /* the steps that repay the copies, with all three outputs and with none */
+  const double cells = (double)nx * ny, none = 3.0;
+  const double all = std::min(std::max(1.2e6 / cells, cells < 1e6 ? 5.0 : 4.0), 20.0);
+  return iterations >= none + (all - none) * copied_outputs / 3.0 && nx >= 40 && ny >= FS_H && (long long)nx * ny <= (1ll << 28) &&
          vpipes_pick_algo(nx, ny) == 0 && (nx % 4 != 0 || !aligned16(z));
 }
 

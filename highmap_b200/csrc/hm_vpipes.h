@@ -10,12 +10,20 @@ namespace hm
 {
 int    vpipes_check_args(const float *z, int nx, int ny, const hm_vpipes_params *p);
 /* Whether a solve should keep its state in rows padded to a multiple of 4
- * floats, with a copy of z: where nx or z miss the TMA rules, the copy
- * (8 B per cell in, 8 out) buys the TMA-staged kernels for every step:
+ * floats, with copies of z and of the copied_outputs among sediment, vel_u
+ * and vel_v: where nx or z miss the TMA rules, the copies (8 B per cell in
+ * and out each) buy the TMA-staged kernels for every step:
  * 1023 x 767, rain map and top-up, 50 steps, 1575 us with clamped 4-byte
- * copies, 1394 us padded.  Not above 2^28 cells, so that memory limits stay where
- * they are, nor where another kernel is asked for or tuned. */
-bool   vpipes_wants_padding(const float *z, int nx, int ny, int iterations);
+ * copies, 1394 us padded.  The copies take the time of a few launches or of
+ * a few steps: with all outputs, cp.async tiles and padded, 255 x 257 8 steps
+ * 93 and 104 us, 50 steps 1.09x; 601 x 599 2 steps 0.89x, 4 steps 0.97x, 8
+ * steps 1.03x; 2047 x 2049 2 steps 0.86x, 4 steps 1.01x, 8 steps 1.15x.  So
+ * from 1.2 M cell-steps on, and between 5 (4 from a million cells on) and 20
+ * steps; with z alone, 3
+ * steps (1.01x and 1.13x at the two smaller and the largest).  Not above 2^28
+ * cells, so that memory limits stay where they are, nor where another kernel
+ * is asked for or tuned. */
+bool   vpipes_wants_padding(const float *z, int nx, int ny, int iterations, int copied_outputs);
 size_t vpipes_scratch_bytes(int nx, int ny, bool padded);
 /* Device pointers; ordered on s.  rain and the outputs are nullable. */
 int    vpipes_core(float *z, int nx, int ny, const hm_vpipes_params &p, const float *rain, float *water_depth,

@@ -101,7 +101,7 @@ def test_kernel_choice_changes_meanwhile(gpu):
     import threading
     import torch
     from highmap_b200 import batch as B
-    specs = [("vpipes", 517, 259 + k, 3, RAIN, k % 2) for k in range(12)] + [("thermal", 1024, 1024, 1300, dict(), 0)]
+    specs = [("vpipes", 517, 259 + k, 12, RAIN, k % 2) for k in range(12)] + [("thermal", 1024, 1024, 1300, dict(), 0)]
     want = _make(specs)
     for c in want:
         _plain(gpu, *c)
