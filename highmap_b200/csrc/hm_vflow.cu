@@ -182,13 +182,17 @@ __global__ void __launch_bounds__(VF_NT) k_vflow_init(float *__restrict__ h, con
  * south edges), into shared memory; a face is the same value for the two
  * cells it separates (fadd is commutative), so this equals evaluating it
  * from both sides, at about half the pow calls.  Faces on the grid's edge
- * pair a cell with itself, as the clamped reads do. */
+ * pair a cell with itself, as the clamped reads do.  GENERAL: a power that
+ * needs pow, without the code of the half-integer ones beside it (power 2.2,
+ * 20 steps at 2048 x 2048 2.48 -> 2.35 ms). */
 constexpr int VT_X = 32, VT_Y = 8;
 
+template <bool GENERAL>
 __global__ void __launch_bounds__(VT_X *VT_Y) k_vflow_step(const float *__restrict__ z, const float *hin,
                                                           float *__restrict__ hout, int nx, int ny, VfScalars *sc,
                                                           VfConst c, int want_max)
 {
+  if (GENERAL) c.half = 0;
   __shared__ float me[VT_Y][VT_X + 1]; /* me[ty][tx + 1]: east face of (tx, ty); [ty][0]: west edge  */
   __shared__ float mn[VT_Y + 1][VT_X]; /* mn[ty + 1][tx]: north face of (tx, ty); [0][tx]: south edge */
   chain_wait();
@@ -411,7 +415,7 @@ int vflow_core(const float *z, int nx, int ny, float water_height, const float *
     if (per == 1)
     {
       const dim3 tiles((nx + VT_X - 1) / VT_X, (ny + VT_Y - 1) / VT_Y);
-      chain_launch(it > 0, k_vflow_step, tiles, dim3(VT_X, VT_Y), s, z, cur, nxt, nx, ny, sc, c, want_max);
+      chain_launch(it > 0, c.half ? k_vflow_step<false> : k_vflow_step<true>, tiles, dim3(VT_X, VT_Y), s, z, cur, nxt, nx, ny, sc, c, want_max);
       HM_LAUNCH_CHECK("k_vflow_step");
     }
     else
