@@ -37,14 +37,19 @@ struct Slab
  * into pinned memory takes 7 us and the transfer runs on its own beside the
  * launches (up), or all outputs come down with one wait.  Above, the second
  * pass over host memory costs more than the synchronisations (4 MB: 269 us
- * against 84 + 248). */
+ * against 84 + 248).  Calls whose result is an array of its own, which a
+ * program allocates for the call, stage up to 256 KB: the copy into memory
+ * not yet touched takes the time of its page faults, which the driver's copy
+ * hides (flow_simulation, 2 steps, staged and not: 256 x 256 96 and 107 us,
+ * 360 x 360 170 and 147, 512 x 512 291 and 263). */
 class HostCopies
 {
 public:
   static constexpr int MAX_GRIDS = 8; /* most copies of a call: 8 MB of staging */
-  HostCopies(hm_context *ctx, size_t nbytes) : s_(ctx->stream), nbytes_(nbytes)
+  static constexpr size_t FRESH_RESULT = (size_t)1 << 18; /* most bytes a grid of such a call may have */
+  HostCopies(hm_context *ctx, size_t nbytes, size_t most = (size_t)1 << 20) : s_(ctx->stream), nbytes_(nbytes)
   {
-    if (nbytes <= ((size_t)1 << 20)) pin_ = (char *)hm::pinned(ctx, MAX_GRIDS * align_up(nbytes, 256) + 256);
+    if (nbytes <= most) pin_ = (char *)hm::pinned(ctx, MAX_GRIDS * align_up(nbytes, 256) + 256);
   }
   int up(float *dev, const float *host)
   {
@@ -501,7 +506,7 @@ int hm_flow_simulation(hm_context *ctx, const float *z, int nx, int ny, float wa
   float       *dd = sl.take(n);
   void        *scr = sl.take_bytes(hm::flow_scratch_bytes(nx, ny, padded));
   cudaStream_t s = ctx->stream;
-  HostCopies   io(ctx, nbytes);
+  HostCopies   io(ctx, nbytes, HostCopies::FRESH_RESULT);
   if ((st = io.up(dz, z))) return st;
   if ((st = io.up(dm, depth_map))) return st;
   st = hm::flow_simulation_core(dz, nx, ny, water_height, dm, iterations, dt, flux_diffusion, flux_diffusion_strength,
@@ -555,7 +560,7 @@ int hm_flow_simulation_viscous(hm_context *ctx, const float *z, int nx, int ny, 
   float       *dout = sl.take(n);
   void        *scr = sl.take_bytes(hm::vflow_scratch_bytes(nx, ny));
   cudaStream_t s = ctx->stream;
-  HostCopies   io(ctx, nbytes);
+  HostCopies   io(ctx, nbytes, HostCopies::FRESH_RESULT);
   if ((st = io.up(dz, z))) return st;
   if ((st = io.up(ddm, depth_map))) return st;
   st = hm::vflow_core(dz, nx, ny, water_height, ddm, iterations, dt, dry_out_ratio, viscosity, power, dout, scr, s);
