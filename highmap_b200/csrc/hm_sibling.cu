@@ -422,7 +422,7 @@ int sibling_core(int device, int rule, float *z, int nx, int ny, const float *ta
     case HM_SCHOTT: HM_SIB_SWEEP(HM_SCHOTT) break;
     case HM_INFLATE: HM_SIB_SWEEP(HM_INFLATE) break;
     case HM_RIB: HM_SIB_SWEEP(HM_RIB) break;
-    case HM_FLATTEN: 
+    case HM_FLATTEN:
       chain_launch(l > 0, k_sibling_step<HM_FLATTEN>, grid, block, s, src, dst, nx, ny, talus, zmax, intensity, p1);
       break;
     default: chain_launch(l > 0, k_sibling_step<HM_OLSEN>, grid, block, s, src, dst, nx, ny, talus, zmax, intensity, p1);

@@ -92,10 +92,13 @@ __device__ __forceinline__ float hyp_try(float x, float y, bool &ok, float &rinv
   return lo;
 }
 
-/* x / h for h from hyp_try, h >= 1 and 1e-3 <= x <= h: Markstein's division
- * (IBM J. Res. Dev. 34(1), 1990) from the reciprocal r of relative error
- * under 2^-21: one Newton step, the quotient and one residual correction.
- * No operand can leave the normal range. */
+/* x / h for h = hyp(1, x) from hyp_try, x >= 1e-3, r its approximate
+ * reciprocal: one Newton step, the quotient and one residual correction, the
+ * steps of Markstein's division (IBM J. Res. Dev. 34(1), 1990).  The Newton
+ * step need not give the correctly rounded reciprocal, so the theorem does
+ * not apply; the quotient was compared with the division instead, for every
+ * float x from 1e-3 to 7e4 and r off by up to 3 ulp either way, and for 1.6
+ * 10^8 larger x, where it is 1.  No operand can leave the normal range. */
 __device__ __forceinline__ float div_hyp(float x, float h, float r)
 {
   r = __fmaf_rn(r, __fmaf_rn(-h, r, 1.f), r);
