@@ -2,7 +2,7 @@
 out is reported with the caller's output untouched: the test hook arms every
 tile's barrier with bytes that never come.  One step runs the one-step
 kernel, two the two-step one, three both; with rows of a multiple of 4
-floats and padded."""
+floats and padded (which one step is from 100000 cells on)."""
 import numpy as np
 import pytest
 
@@ -14,10 +14,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("iters", [1, 2, 3])
-@pytest.mark.parametrize("nx", [64, 67])
-def test_wait_runs_out_and_is_reported(gpu, nx, iters):
+@pytest.mark.parametrize("nx, ny", [(64, 40), (67, 1500)])
+def test_wait_runs_out_and_is_reported(gpu, nx, ny, iters):
     import ctypes as C
-    z, dm = fbm(nx, 40, seed=13), fbm(nx, 40, seed=14)
+    z, dm = fbm(nx, ny, seed=13), fbm(nx, ny, seed=14)
     out = np.full_like(z, -7.0)
     ctx = gpu.Context(0)
 
@@ -25,7 +25,7 @@ def test_wait_runs_out_and_is_reported(gpu, nx, iters):
         return C.c_void_p(a.ctypes.data)
 
     def call():
-        return L.lib().hm_flow_simulation(ctx.handle, p(z), nx, 40, C.c_float(0.05), p(dm), iters, C.c_float(0.5), 1,
+        return L.lib().hm_flow_simulation(ctx.handle, p(z), nx, ny, C.c_float(0.05), p(dm), iters, C.c_float(0.5), 1,
                                           C.c_float(0.01), C.c_float(0.0), p(out))
     try:
         gpu.debug_tma_expect_extra(16)
