@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) k_border(float *z, int nx, int ny)
 {
   const long long n = 2ll * nx + 2ll * (ny - 2);
   chain_wait();
-  for (long long k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256)
+  for (long long k = blockIdx.x * 256ll + threadIdx.x; k < n; k += gridDim.x * 256ll)
   {
     int i, j;
     if (k < 2ll * nx)
