@@ -16,9 +16,10 @@
  * warp's walk down its rows: 6.3 us per step from 64^2 to 512^2, 8.3 us at
  * 1024^2.  Here a step inside the launch takes 0.65 us (ROWS 1) or 1.1 us
  * (ROWS 2) on one CTA per SM.  Measured, 48 steps, talus map and bedrock:
- * 1.1 us per step at 64^2, 1.34 at 256^2, 2.13 at 512^2, 5.7 at 1024^2.
- * Above, the recomputed halo costs more than the launch: 17.5 against
- * 16.5 us at 2048^2, 65 against 55 us at 4096^2.
+ * 1.1 us per step at 64^2, 1.3 at 256^2, 2.0 at 512^2, 5.3 at 1024^2, 6.2
+ * at 1200^2 (one step per launch, chained: 4.8, 5.9, 6.0, 6.6, 7.9).  Above,
+ * the recomputed halo costs more than the launch: 15.5 against 13.9 us at
+ * 2048^2, 62 against 52 us at 4096^2.
  *
  * Every cell follows the one-step rule (border copies of
  * _common_index.cl:106-132, then the cell rule), so T steps here are T
